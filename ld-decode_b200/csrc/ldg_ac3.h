@@ -9,6 +9,8 @@ namespace ldg {
 
 // Filter taps of the front end, device pointers; only non-zero taps are
 // stored (value + index), in ascending index order like the reference.
+constexpr int kMaxAc3Rrc = 95;  // matched-filter taps the register-blocked kernel holds
+
 struct Ac3Taps {
     const float* hb19_val;
     const int* hb19_off;
@@ -23,6 +25,11 @@ struct Ac3Taps {
     const float* sin_lut;
     int lut_bits;
     int phase_step;
+    // the register-blocked kernel's taps (host values: they go in its
+    // parameters) and mixer table, when the filters have its shapes
+    bool fast;
+    float h_hb19[11], h_hb23[13], h_rrc[kMaxAc3Rrc];
+    const float2* mix;
 };
 
 cudaError_t launch_ac3_frontend(const void* in, int in_kind, long long in_first, long long nsamples,

@@ -166,6 +166,29 @@ def test_gpu_frontend_int16_and_device_buffers(cuda_ok, signals):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("fs", [29e6, 40e6, 45e6])
+@pytest.mark.parametrize("kind", ["int16", "float32"])
+def test_gpu_frontend_tile_edges(cuda_ok, fs, kind):
+    """Output counts and first outputs around the kernel's tile (1006 - taps
+    + 1 outputs), odd input starts (no paired loads) and the matched filters
+    of other rates, against the oracle over the whole input."""
+    from ldgpu.ac3 import Ac3Frontend
+    fe = Ac3Frontend(fs)
+    tile = 1006 - len(fe.design.rrc) + 1
+    rng = np.random.default_rng(int(fs) // 1000)
+    x = rng.integers(-2000, 2001, 16 * (3 * tile + 5) + 3).astype(kind)
+    oi, oq = oac3.frontend(x.astype(np.float64), fs)
+    scale = np.abs(oi).max()
+    total = (len(x) + 15) // 16
+    for first, count, cut in [(0, 1, 0), (0, tile - 1, 0), (0, tile, 0), (0, tile + 1, 0), (0, total, 0),
+                              (total - 1, 1, 0), (500, 2 * tile + 3, 16 * 500 - 2047), (tile, tile, 16 * tile - 1700)]:
+        i, q = fe.run(np.ascontiguousarray(x[cut:]), cut, first, count)
+        assert np.abs(i - oi[first:first + count]).max() / scale < 2e-5, (first, count)
+        assert np.abs(q - oq[first:first + count]).max() / scale < 2e-5, (first, count)
+    fe.close()
+
+
+@pytest.mark.gpu
 def test_gpu_streaming_demodulator_loopback(cuda_ok, g, signals):
     from ldgpu.ac3 import Ac3RfDemodulator
     clean, noisy = signals
