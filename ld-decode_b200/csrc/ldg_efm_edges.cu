@@ -9,10 +9,14 @@
 // (one every ~25 samples of band-limited EFM) instead of 2 bytes per
 // sample.
 //
-// Three launches, as the sync-run scan: crossings counted per tile of 8192
-// samples, an exclusive scan of the tile counts (which also writes the
-// total where the caller asked, device or host-mapped memory), crossings
-// written in order.
+// Two streaming launches over the same contiguous chunks, one per resident
+// CTA: the first counts each chunk's crossings, the second adds up the counts
+// before its chunk and writes its crossings, from the chunk's end to its
+// start, whose samples the first left in L2 last.  Bound: HBM, 2 bytes read
+// per sample and 8 written per crossing.  80 M samples, B200: 197 us as
+// counts, a scan and a second pass with 2-byte loads; 68 us so (2.7 TB/s
+// of the 182 MB it has to move).  One pass with decoupled look-back took 80
+// us at best: the CTAs of a wave all wait for the wave's slowest load.
 #include <stdint.h>
 
 #include <string>
@@ -26,119 +30,208 @@ int api_fail(int code, const std::string& msg);
 
 namespace {
 
-constexpr int kTile = 8192;
-constexpr int kThreads = 256;
-constexpr int kSteps = kTile / (4 * kThreads);
+// 128 threads and 16 CTAs per SM: 68 us; 256 and 8: 72, 512 and 4: 77, 1024 and
+// 2: 84 (the more CTAs, the less a barrier holds up).
+constexpr int kThreads = 128;
+constexpr int kTile = 32 * kThreads;    // samples: one 32-bit word of sign flags per thread
+constexpr int kMaxChunks = 148 * 16;    // the resident CTAs
 
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
-// crossing bits of samples base .. base+3 (bit k: sample base+k)
-__device__ __forceinline__ unsigned crossings4(const int16_t* __restrict__ x, long long n, long long base,
-                                               int has_before) {
-    int prev = base > 0 ? (int)x[base - 1] : (has_before ? (int)x[-1] : 0);
-    unsigned bits = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-        if (base + k >= n) break;
-        const int cur = x[base + k];
-        if ((prev ^ cur) < 0) bits |= 1u << k;
-        prev = cur;
-    }
-    return bits;
+// Sample i sits at position i + mis of the tiles, mis the samples x lies past
+// a 16-byte boundary, so that any x takes 16-byte loads.
+
+// Eight samples from i on (0 outside [0, n), where In is false), two per word.
+template <bool In>
+__device__ __forceinline__ uint4 load8(const int16_t* __restrict__ x, long long n, long long i) {
+    if (In || (i >= 0 && i + 8 <= n)) return __ldg(reinterpret_cast<const uint4*>(x + i));
+    unsigned w[4] = {0, 0, 0, 0};
+    for (int k = 0; k < 8; ++k)
+        if (i + k >= 0 && i + k < n) w[k >> 1] |= (unsigned)(uint16_t)x[i + k] << (16 * (k & 1));
+    return make_uint4(w[0], w[1], w[2], w[3]);
 }
 
-__global__ void __launch_bounds__(kThreads) efm_count_kernel(const int16_t* __restrict__ x, long long n,
-                                                             int has_before, int* __restrict__ counts) {
-    const long long t0 = (long long)blockIdx.x * kTile;
-    int c = 0;
-    for (int j = 0; j < kSteps; ++j) {
-        const long long base = t0 + (long long)j * 4 * kThreads + 4 * threadIdx.x;
-        if (base < n) c += __popc(crossings4(x, n, base, has_before));
+constexpr unsigned kSigns = 0x80008000u;
+
+// Sign changes among eight samples, given the word that ends with the sample
+// before them.
+__device__ __forceinline__ int changes8(uint4 v, unsigned before) {
+    const unsigned a = (v.x ^ __funnelshift_l(before, v.x, 16)) & kSigns;
+    const unsigned b = (v.y ^ __funnelshift_l(v.x, v.y, 16)) & kSigns;
+    const unsigned c = (v.z ^ __funnelshift_l(v.y, v.z, 16)) & kSigns;
+    const unsigned d = (v.w ^ __funnelshift_l(v.z, v.w, 16)) & kSigns;
+    return __popc(a | (b >> 1) | (c >> 2) | (d >> 3));
+}
+
+// Their sign bits, the first sample's in bit 7.
+__device__ __forceinline__ unsigned signs8(uint4 v) {
+    const unsigned s = (v.x & kSigns) | ((v.y & kSigns) >> 2) | ((v.z & kSigns) >> 4) | ((v.w & kSigns) >> 6);
+    return ((s & 0xffffu) | (s >> 17)) >> 8;
+}
+
+// Crossings among the tile samples c .. c + 31 (c the tile's, i = t0 + c the
+// array's index) from their signs and the sign of the sample before: none
+// outside [0, n), and sample 0 against x[-1] (has_before) or against 0.
+template <bool In>
+__device__ __forceinline__ unsigned crossings32(unsigned f, unsigned before, const int16_t* __restrict__ x, long long n,
+                                                long long i, int has_before) {
+    unsigned prev = (f << 1) | before;
+    if (In) return f ^ prev;
+    if (i <= 0 && i + 32 > 0) {
+        const unsigned first = 1u << (int)(-i);
+        prev = (prev & ~first) | (has_before && x[-1] < 0 ? first : 0u);
     }
+    unsigned e = f ^ prev;
+    if (i < 0) e &= i <= -32 ? 0u : 0xffffffffu << (int)(-i);
+    if (i + 32 > n) e &= i >= n ? 0u : 0xffffffffu >> (int)(i + 32 - n);
+    return e;
+}
+
+// A chunk's crossings.  A tile whose samples, and the one before, all exist
+// compares neighbouring words; the array's first and last tiles go sample by
+// sample.
+__global__ void __launch_bounds__(kThreads) efm_count_kernel(const int16_t* __restrict__ x, long long n, int mis,
+                                                             int has_before, long long ntiles,
+                                                             long long* __restrict__ counts) {
     __shared__ int warp_sum[kThreads / 32];
-    for (int o = 16; o; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-    if ((threadIdx.x & 31) == 0) warp_sum[threadIdx.x >> 5] = c;
+    const int t = threadIdx.x, lane = t & 31;
+    const long long g0 = ntiles * blockIdx.x / gridDim.x, g1 = ntiles * (blockIdx.x + 1) / gridDim.x;
+    int c = 0;
+#pragma unroll 1
+    for (long long tile = g0; tile < g1; ++tile) {
+        const long long t0 = tile * kTile - mis;
+        if (t0 > 0 && t0 + kTile <= n) {
+            const int16_t* xt = x + t0 + 8 * t;
+            uint4 v[4];
+            unsigned ahead[4];  // the word that ends with the sample before the warp's 256
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[j] = __ldg(reinterpret_cast<const uint4*>(xt + 8 * j * kThreads));
+            if (lane == 0) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) ahead[j] = (unsigned)(uint16_t)__ldg(xt + 8 * j * kThreads - 1) << 16;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const unsigned up = __shfl_up_sync(0xffffffffu, v[j].w, 1);
+                c += changes8(v[j], lane ? up : ahead[j]);
+            }
+        } else {
+            for (int k = t; k < kTile; k += kThreads) {
+                const long long i = t0 + k;
+                if (i < 0 || i >= n) continue;
+                const int prev = i > 0 || has_before ? x[i - 1] : 0;
+                c += (prev ^ x[i]) < 0;
+            }
+        }
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) c += __shfl_xor_sync(0xffffffffu, c, o);
+    if (lane == 0) warp_sum[t >> 5] = c;
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (t == 0) {
         int s = 0;
         for (int w = 0; w < kThreads / 32; ++w) s += warp_sum[w];
         counts[blockIdx.x] = s;
     }
 }
 
-// exclusive scan of the tile counts (one CTA); the total to *total and, if
-// given, to *count_out
-__global__ void __launch_bounds__(1024) efm_scan_kernel(const int* __restrict__ counts, long long ntiles,
-                                                        long long* __restrict__ offsets, long long* total,
-                                                        long long* count_out) {
-    __shared__ long long part[1024];
-    __shared__ long long carry;
-    if (threadIdx.x == 0) carry = 0;
+// Writes one tile's crossings, the last of them at edges[end - 1]; returns
+// their number.  The signs make a shared bitmap; thread t owns the 32 samples
+// of word t.  All threads; ends with every read of the shared arrays done
+// but warp_tot's.
+template <bool In>
+__device__ __forceinline__ int write_tile(const int16_t* __restrict__ x, long long n, long long t0, int has_before,
+                                          unsigned* bm, int* warp_tot, ldg_efm_edge* __restrict__ edges,
+                                          long long cap, long long pos_offset, long long end) {
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    uint8_t* bytes = reinterpret_cast<uint8_t*>(bm);
+    uint4 v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) v[j] = load8<In>(x, n, t0 + 8 * (j * kThreads + t));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) bytes[j * kThreads + t] = (uint8_t)signs8(v[j]);
+    unsigned before = 0;
+    if (t == 0) before = In || (t0 > 0 && t0 <= n) ? (unsigned)(x[t0 - 1] < 0) : 0u;
     __syncthreads();
-    for (long long base = 0; base < ntiles; base += 1024) {
-        const long long i = base + threadIdx.x;
-        const long long v = i < ntiles ? counts[i] : 0;
-        part[threadIdx.x] = v;
-        __syncthreads();
-        for (int o = 1; o < 1024; o <<= 1) {
-            const long long add = threadIdx.x >= o ? part[threadIdx.x - o] : 0;
-            __syncthreads();
-            part[threadIdx.x] += add;
-            __syncthreads();
+    if (t > 0) before = (bm[t - 1] >> 24) & 1u;
+    // byte order to sample order: the word's first sample in bit 0
+    const unsigned f = __brev(__byte_perm(bm[t], 0, 0x0123));
+    unsigned e = crossings32<In>(f, before, x, n, t0 + 32 * t, has_before);
+    const int cnt = __popc(e);
+    int inc = cnt;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+    }
+    if (lane == 31) warp_tot[warp] = inc;
+    __syncthreads();
+    int total = 0, ahead = 0;  // crossings of the tile, of the warps before this one
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) {
+        const int q = warp_tot[w];
+        ahead += w < warp ? q : 0;
+        total += q;
+    }
+    long long k = end - total + ahead + inc - cnt;
+    const int16_t* xt = x + t0 + 32 * t;
+    const unsigned pos = (unsigned)(pos_offset + t0 + 32 * t);
+    if (In && end <= cap && (reinterpret_cast<uintptr_t>(edges) & 7) == 0) {
+        uint2* out = reinterpret_cast<uint2*>(edges + k);
+        while (e) {
+            const int c = __ffs(e) - 1;
+            e &= e - 1;
+            *out++ = make_uint2(pos + c, (unsigned)(uint16_t)xt[c - 1] | ((unsigned)(uint16_t)xt[c] << 16));
         }
-        if (i < ntiles) offsets[i] = carry + part[threadIdx.x] - v;
-        __syncthreads();
-        if (threadIdx.x == 1023) carry += part[1023];
-        __syncthreads();
+        return total;
     }
-    if (threadIdx.x == 0) {
-        *total = carry;
-        if (count_out) *count_out = carry;
+    while (e) {
+        const int c = __ffs(e) - 1;
+        e &= e - 1;
+        if (k < cap) {
+            ldg_efm_edge r;
+            r.pos = (int32_t)(pos + c);
+            r.prev = t0 + 32 * t + c > 0 || has_before ? xt[c - 1] : (int16_t)0;
+            r.cur = xt[c];
+            edges[k] = r;
+        }
+        ++k;
     }
+    return total;
 }
 
-__global__ void __launch_bounds__(kThreads) efm_write_kernel(const int16_t* __restrict__ x, long long n,
-                                                             int has_before, const long long* __restrict__ offsets,
+__global__ void __launch_bounds__(kThreads) efm_write_kernel(const int16_t* __restrict__ x, long long n, int mis,
+                                                             int has_before, long long ntiles,
+                                                             const long long* __restrict__ counts,
                                                              ldg_efm_edge* __restrict__ edges, long long cap,
-                                                             long long pos_offset) {
-    __shared__ int warp_cnt[kThreads / 32];
-    const long long t0 = (long long)blockIdx.x * kTile;
-    long long out = offsets[blockIdx.x];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int j = 0; j < kSteps; ++j) {
-        const long long base = t0 + (long long)j * 4 * kThreads + 4 * threadIdx.x;
-        const unsigned e = base < n ? crossings4(x, n, base, has_before) : 0u;
-        const int cnt = __popc(e);
-        int inc = cnt;
+                                                             long long pos_offset, long long* count_out) {
+    __shared__ unsigned bm[2][kThreads];
+    __shared__ int warp_tot[2][kThreads / 32];
+    __shared__ long long s_sum[kThreads / 32];
+    const int t = threadIdx.x;
+    const long long g0 = ntiles * blockIdx.x / gridDim.x, g1 = ntiles * (blockIdx.x + 1) / gridDim.x;
+    // the crossings up to this chunk's end
+    long long s = 0;
+    for (int g = t; g <= (int)blockIdx.x; g += kThreads) s += counts[g];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int y = __shfl_up_sync(0xffffffffu, inc, o);
-            if (lane >= o) inc += y;
+    for (int o = 16; o; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if ((t & 31) == 0) s_sum[t >> 5] = s;
+    __syncthreads();
+    long long end = 0;
+#pragma unroll
+    for (int w = 0; w < kThreads / 32; ++w) end += s_sum[w];
+    if (t == 0 && count_out && blockIdx.x == gridDim.x - 1) *count_out = end;
+    // the shared arrays alternate: a tile's barriers order the reads of the
+    // tile before it against the writes of the tile after
+#pragma unroll 1
+    for (long long tile = g1 - 1; tile >= g0; --tile) {
+        const long long t0 = tile * kTile - mis;
+        const int b = (int)(tile & 1);
+        if (t0 > 0 && t0 + kTile <= n) {
+            end -= write_tile<true>(x, n, t0, has_before, bm[b], warp_tot[b], edges, cap, pos_offset, end);
+        } else {
+            end -= write_tile<false>(x, n, t0, has_before, bm[b], warp_tot[b], edges, cap, pos_offset, end);
         }
-        if (lane == 31) warp_cnt[warp] = inc;
-        __syncthreads();
-        int before = 0, chunk = 0;
-#pragma unroll
-        for (int w = 0; w < kThreads / 32; ++w) {
-            before += w < warp ? warp_cnt[w] : 0;
-            chunk += warp_cnt[w];
-        }
-        long long k = out + before + inc - cnt;
-#pragma unroll
-        for (int q = 0; q < 4; ++q)
-            if (e & (1u << q)) {
-                if (k < cap) {
-                    const long long i = base + q;
-                    ldg_efm_edge r;
-                    r.pos = (int32_t)(pos_offset + i);
-                    r.prev = i > 0 ? x[i - 1] : (has_before ? x[-1] : (int16_t)0);
-                    r.cur = x[i];
-                    edges[k] = r;
-                }
-                ++k;
-            }
-        out += chunk;
-        __syncthreads();
     }
 }
 
@@ -148,8 +241,7 @@ extern "C" {
 
 int64_t ldg_efm_edges_scratch_bytes(int64_t n) {
     if (n < 0) return -1;
-    const long long ntiles = (n + kTile - 1) / kTile;
-    return (int64_t)(align256((size_t)ntiles * sizeof(int)) + align256((size_t)ntiles * sizeof(long long)) + 256);
+    return (int64_t)align256(kMaxChunks * sizeof(long long));  // a count per chunk
 }
 
 int ldg_efm_edges(const int16_t* efm, int64_t n, int32_t has_before, int64_t pos_offset, ldg_efm_edge* edges,
@@ -165,16 +257,14 @@ int ldg_efm_edges(const int16_t* efm, int64_t n, int32_t has_before, int64_t pos
             return ldg::api_fail(LDG_ERR_ARG, "ldg_efm_edges: count must be device memory or pinned host memory");
     }
     cudaStream_t st = (cudaStream_t)stream;
-    const long long ntiles = (n + kTile - 1) / kTile;
-    char* p = static_cast<char*>(scratch);
-    int* counts = reinterpret_cast<int*>(p);
-    long long* offsets = reinterpret_cast<long long*>(p + align256((size_t)ntiles * sizeof(int)));
-    long long* total = reinterpret_cast<long long*>(p + align256((size_t)ntiles * sizeof(int)) +
-                                                    align256((size_t)ntiles * sizeof(long long)));
-    if (ntiles > 0) {
-        efm_count_kernel<<<(unsigned)ntiles, kThreads, 0, st>>>(efm, n, has_before, counts);
-        efm_scan_kernel<<<1, 1024, 0, st>>>(counts, ntiles, offsets, total, dcount);
-        efm_write_kernel<<<(unsigned)ntiles, kThreads, 0, st>>>(efm, n, has_before, offsets, edges, cap, pos_offset);
+    if (n > 0) {
+        const int mis = (int)((reinterpret_cast<uintptr_t>(efm) & 15) / sizeof(int16_t));
+        const long long ntiles = (n + mis + kTile - 1) / kTile;
+        long long* counts = static_cast<long long*>(scratch);
+        const unsigned grid = (unsigned)(ntiles < kMaxChunks ? ntiles : kMaxChunks);
+        efm_count_kernel<<<grid, kThreads, 0, st>>>(efm, n, mis, has_before, ntiles, counts);
+        efm_write_kernel<<<grid, kThreads, 0, st>>>(efm, n, mis, has_before, ntiles, counts, edges, cap, pos_offset,
+                                                    dcount);
     } else if (dcount) {
         if (cudaMemsetAsync(dcount, 0, sizeof(long long), st) != cudaSuccess) cudaGetLastError();
     }

@@ -36,6 +36,26 @@ def test_edges_equal_numpy(cuda_ok, name):
     assert got2.tobytes() == want2.tobytes()
 
 
+@pytest.mark.parametrize("n", [1, 7, 8, 31, 32, 33, 4095, 4096, 4097, 4102, 5 * 4096 + 5, 2369 * 4096 - 3])
+@pytest.mark.parametrize("off", [0, 1, 3, 7])
+def test_edges_tile_edges(cuda_ok, n, off):
+    """Lengths around the kernel's words and tiles, starts off a 16-byte
+    boundary (their first tile begins before the samples), with and without
+    the sample before, and more tiles than chunks."""
+    import torch
+    from ldgpu.efm import efm_edges
+    rng = np.random.default_rng(n + off)
+    x = rng.integers(-3, 3, n + off + 1).astype(np.int16)
+    x[rng.random(len(x)) < 0.5] = 5
+    t = torch.from_numpy(x).cuda()
+    want = efm_crossings(x[off:off + n])
+    assert efm_edges(t[off:off + n]).tobytes() == want.tobytes()
+    if off:
+        got = efm_edges(t[off:off + n], has_before=True, pos_offset=off)
+        want = efm_crossings(x[:off + n])
+        assert got.tobytes() == want[want["pos"] >= off].tobytes()
+
+
 def test_edges_count_beyond_cap_and_empty(cuda_ok):
     import torch
     from ldgpu import lib as L
