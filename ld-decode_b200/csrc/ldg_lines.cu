@@ -11,14 +11,16 @@
 //
 // ldg_lines_refine: the per-line refinement of Field.process() for all
 // fields of a capture (pulse-level line locations from the host chain):
-//   lines_hsync_kernel   one CTA per field: refine_linelocs_hsync
-//                        (core.py:2483-2551), compute_deriv_error
-//                        (2553-2564); NTSC: the colour-burst zero crossings
-//                        of compute_line_bursts (2998-3047, clb_findbursts
-//                        utils.py:1339-1368) per line; PAL:
+//   lines_hsync_kernel   one warp per line: refine_linelocs_hsync
+//                        (core.py:2483-2551)
+//   lines_burst_kernel   NTSC, one warp per line: compute_deriv_error
+//                        (2553-2564), the colour-burst zero crossings of
+//                        compute_line_bursts (2998-3047, clb_findbursts
+//                        utils.py:1339-1368)
+//   lines_pal_kernel     PAL, one CTA per field: compute_deriv_error,
 //                        refine_linelocs_pilot twice (3054-3093) and
 //                        fix_badlines (2566-2589) -> final line locations;
-//                        PAL: the burst levels and line 7-19 burst crossings
+//                        the burst levels and line 7-19 burst crossings
 //                        of determine_field_number (3095-3203).
 //   pal_sequence_kernel  PAL, one warp walking the fields in order: the
 //                        8-field sequence (field phase IDs).
@@ -38,6 +40,7 @@
 #include <mutex>
 #include <string>
 
+#include "ldg_attr.cuh"
 #include "ldg_copy.cuh"
 #include "ldg_scan.cuh"
 #include "ldgpu.h"
@@ -57,7 +60,6 @@ namespace {
 constexpr int kMaxL = LDG_CHAIN_MAX_LINES;
 constexpr int kEdgeTile = 16384;  // samples per sync-run scan tile
 constexpr int kEdgeThreads = 256;
-constexpr int kLineThreads = 352;   // >= proclines (326 PAL)
 constexpr int kBurstLines = 266;    // compute_burst_offsets covers lines 0..265
 constexpr int kPilotLines = 323;    // refine_linelocs_pilot covers lines 0..322
 constexpr int kZc = 16;             // clb_findbursts' fixed zero-crossing slots
@@ -285,37 +287,6 @@ __global__ void run_pair_kernel(const long long* __restrict__ edges, const long 
 
 // --------------------------------------------------------- per-line helpers
 
-// calczc (utils.py:812-841) over x[0, n): first crossing of `target` within
-// count+1 samples from int(start); edge 0 decides rising/falling from
-// x[int(start)].  Comparisons and the interpolation in FP64.
-__device__ bool calczc(const float* x, long long n, double start_offset, double target, int edge, double count,
-                       double& out) {
-    const long long s = (long long)start_offset;
-    if (s < 0 || s >= n) return false;
-    const long long icount = (long long)(count + 1);
-    if (edge == 0) edge = (double)x[s] < target ? 1 : -1;
-    const long long end = min(s + icount, n);
-    long long loc = -1;
-    if (edge == 1) {
-        for (long long i = s + 1; i < end; ++i)
-            if ((double)x[i - 1] < target && (double)x[i] >= target) {
-                loc = i;
-                break;
-            }
-    } else {
-        for (long long i = s + 1; i < end; ++i)
-            if ((double)x[i - 1] > target && (double)x[i] <= target) {
-                loc = i;
-                break;
-            }
-    }
-    if (loc < 0) return false;
-    const double a = (double)x[loc - 1] - target, b = (double)x[loc] - target;
-    const double y = (b - a != 0) ? -a / (-a + b) : 0.0;
-    out = (double)(loc - 1) + y;
-    return true;
-}
-
 // A line's window of a sample array staged in shared memory: x[i] from the
 // window when i lies in [base, end), else from global memory.
 struct WinView {
@@ -348,7 +319,10 @@ __device__ double median_f32(const X& x, long long lo, long long hi, long long n
 
 // Warp-cooperative forms (every lane returns the same result).
 
-// calczc with 32 samples tested per step and the first crossing by ballot
+// calczc (utils.py:812-841) over x[0, n): first crossing of `target` within
+// count+1 samples from int(start); edge 0 decides rising/falling from
+// x[int(start)].  Comparisons and the interpolation in FP64; 32 samples
+// tested per step and the first crossing by ballot.
 template <class X>
 __device__ bool warp_calczc(const X& x, long long n, double start_offset, double target, int edge, double count,
                             double& out) {
@@ -527,63 +501,112 @@ struct BurstRec {
     int count, rising, valid, pad;
 };
 
+constexpr int kBurstWin = 128;  // samples of a line's colour burst
+
+// The first set bit at or after j of a 128-bit mask, 128 when none.
+__device__ __forceinline__ int next_bit(const unsigned (&m)[4], int j) {
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+        const int o = j - 32 * w;
+        const unsigned v = o <= 0 ? m[w] : o >= 32 ? 0u : m[w] & (0xffffffffu << o);
+        if (v) return 32 * w + __ffs(v) - 1;
+    }
+    return kBurstWin;
+}
+
 // compute_line_bursts up to the phase update: the zero crossings of the
-// line's colour burst (they do not depend on the phase seed)
-__device__ void burst_record(const LineParams& P, const double* ll, int line, int lc, const float* burst,
-                             const float* demod, long long n, BurstRec& r) {
-    r.valid = 0;
-    r.count = 0;
-    r.rising = 0;
-    const long long s = (long long)ll[line];
-    const double s_rem = ll[line] - (double)s;
+// line's colour burst (they do not depend on the phase seed).  One warp: the
+// burst's samples staged in shared memory (sb, sd: kBurstWin floats each),
+// the sums in the samples' order by every lane (the two means side by side),
+// and the search for crossings on bit masks of the samples.
+__device__ void warp_burst_record(const LineParams& P, const double* ll, int line, int lc, const float* burst,
+                                  const float* demod, long long n, float* sb, float* sd, BurstRec* r) {
+    const int lane = threadIdx.x & 31;
+    const double l0 = ll[line];
+    const long long s = (long long)l0;
+    const double s_rem = l0 - (double)s;
     const double lfreq = P.samplesperline * line_len(ll, line, lc, P.linelen);
     const double fsc_inv = 1 / P.fsc_mhz;
     const long long bstart = (long long)(21 * fsc_inv * lfreq);
     const long long bend = (long long)(28 * fsc_inv * lfreq);
-    long long lo = s + bstart, hi = min(s + bend, n);
+    const long long lo = s + bstart, hi = min(s + bend, n);
+    if (lane == 0) {
+        r->valid = 0;
+        r->count = 0;
+        r->rising = 0;
+    }
     if (lo < 0 || hi <= lo) return;
-    const int m = (int)min(hi - lo, 128LL);
-    float ba[128];
+    const int m = (int)min(hi - lo, (long long)kBurstWin);
+    __syncwarp();
+    for (int k = lane; k < m; k += 32) {
+        sb[k] = burst[lo + k];
+        sd[k] = demod[lo + k];
+    }
+    __syncwarp();
+    // odd lanes the demodulated video's sum, even lanes the burst's
+    const float* src = (lane & 1) ? sd : sb;
     double acc = 0;
-    for (int k = 0; k < m; ++k) acc += (double)burst[lo + k];
-    const float mean_f = (float)(acc / m);
-    for (int k = 0; k < m; ++k) ba[k] = burst[lo + k] - mean_f;
+#pragma unroll 8
+    for (int k = 0; k < m; ++k) acc += (double)src[k];
+    const float mean = (float)(acc / m);
+    const float mean_f = __shfl_sync(0xffffffffu, mean, 0), mean_d = __shfl_sync(0xffffffffu, mean, 1);
+    float mx = 0;
+    for (int k = lane; k < m; k += 32) {
+        mx = fmaxf(mx, fabsf(sd[k] - mean_d));
+        sb[k] = sb[k] - mean_f;
+    }
+#pragma unroll
+    for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    __syncwarp();
+    if ((double)mx > 30 * P.hz_ire) return;
     double m2 = 0;
-    for (int k = 0; k < m; ++k) m2 += (double)ba[k];
+#pragma unroll 8
+    for (int k = 0; k < m; ++k) m2 += (double)sb[k];
     m2 /= m;
     double ss = 0;
+#pragma unroll 8
     for (int k = 0; k < m; ++k) {
-        const double d = (double)ba[k] - m2;
+        const double d = (double)sb[k] - m2;
         ss += d * d;
     }
     const double threshold = sqrt(ss / m);
-    double accd = 0;
-    for (int k = 0; k < m; ++k) accd += (double)demod[lo + k];
-    const float mean_d = (float)(accd / m);
-    float mx = 0;
-    for (int k = 0; k < m; ++k) mx = fmaxf(mx, fabsf(demod[lo + k] - mean_d));
-    if ((double)mx > 30 * P.hz_ire) return;
-    r.valid = 1;
-    const double zcburstdiv = (lfreq * fsc_inv) / 2;
-    float zcs[kZc];
-    for (int k = 0; k < kZc; ++k) zcs[k] = 0.0f;
-    int c = 0;
-    long long j = 0;
-    const long long end = m - 1;
-    while (j < end && c < kZc) {
-        if ((double)fabsf(ba[j]) > threshold) {
-            double zc;
-            if (!calczc(ba, m, (double)j, 0.0, 0, 16, zc)) break;
-            if (ba[j] < 0) r.rising |= 1 << c;
-            zcs[c] = (float)zc;
-            ++c;
-            j = (long long)zc + 1;
-        } else {
-            ++j;
-        }
+    // per sample: above the threshold, negative, a rising / falling crossing
+    unsigned above[4], neg[4], up[4], down[4];
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+        const int k = 32 * w + lane;
+        const float v = k < m ? sb[k] : 0.0f, u = k > 0 && k < m ? sb[k - 1] : 0.0f;
+        above[w] = __ballot_sync(0xffffffffu, k < m && (double)fabsf(v) > threshold);
+        neg[w] = __ballot_sync(0xffffffffu, v < 0);
+        up[w] = __ballot_sync(0xffffffffu, k > 0 && k < m && u < 0 && v >= 0);
+        down[w] = __ballot_sync(0xffffffffu, k > 0 && k < m && u > 0 && v <= 0);
     }
-    r.count = c;
-    for (int k = 0; k < kZc; ++k) r.cyc[k] = ((double)bstart + (double)zcs[k] - s_rem) / zcburstdiv;
+    const double zcburstdiv = (lfreq * fsc_inv) / 2;
+    float mine = 0.0f;  // lane k: slot k's crossing
+    int c = 0, rising = 0, j = 0;
+    while (c < kZc) {
+        j = next_bit(above, j);
+        if (j >= m - 1) break;
+        const unsigned nw = j < 64 ? (j < 32 ? neg[0] : neg[1]) : (j < 96 ? neg[2] : neg[3]);
+        const bool is_neg = (nw >> (j & 31)) & 1u;
+        // calczc from j: the first crossing of its sign within 16 samples
+        const unsigned cross[4] = {is_neg ? up[0] : down[0], is_neg ? up[1] : down[1], is_neg ? up[2] : down[2],
+                                   is_neg ? up[3] : down[3]};
+        const int loc = next_bit(cross, j + 1);
+        if (loc >= min(j + 17, m)) break;
+        const double a = (double)sb[loc - 1], b = (double)sb[loc];
+        const double zc = (double)(loc - 1) + ((b - a != 0) ? -a / (-a + b) : 0.0);
+        if (is_neg) rising |= 1 << c;
+        if (lane == c) mine = (float)zc;
+        ++c;
+        j = (int)zc + 1;
+    }
+    if (lane < kZc) r->cyc[lane] = ((double)bstart + (double)mine - s_rem) / zcburstdiv;
+    if (lane == 0) {
+        r->valid = 1;
+        r->count = c;
+        r->rising = rising;
+    }
 }
 
 // FieldPAL.get_burstlevel (core.py:3095-3104, numpy slice semantics at
@@ -591,29 +614,39 @@ __device__ void burst_record(const LineParams& P, const double* ll, int line, in
 // l_adj, less its mean, times sqrt(2); NaN for the reference's None (a
 // sample above 30 IRE) or an empty slice.  lc = linecount + lineoffset of
 // the moment (get_linelen's last-line rule).
-__device__ double pal_burstlevel(const LineParams& P, const double* ll, int l_adj, int lc, const float* demod,
-                                 long long n, double hz_ire) {
+struct LevelWindow {
+    long long lo, hi;  // samples [lo, hi); empty when hi <= lo
+};
+
+__device__ __forceinline__ LevelWindow pal_level_window(const LineParams& P, const double* ll, int l_adj, int lc,
+                                                        long long n) {
     const double begin = ll[l_adj] + 5.5 * (P.samplesperline * line_len(ll, l_adj, lc, P.linelen));
     const double length = 2.4 * (P.samplesperline * P.linelen);
-    const long long lo = (long long)begin;
-    const long long hi = min((long long)(begin + length + 1.0), n);
-    if (lo < 0 || hi <= lo) return nan("");
-    const long long m = hi - lo;
+    LevelWindow w{(long long)begin, min((long long)(begin + length + 1.0), n)};
+    if (w.lo < 0) w.hi = w.lo;
+    return w;
+}
+
+__device__ double pal_burstlevel(const float* x, int m, double hz_ire) {
+    if (m <= 0) return nan("");
     double acc = 0;  // float32 samples near 7 MHz: this double sum is exact
-    for (long long k = 0; k < m; ++k) acc += (double)demod[lo + k];
+#pragma unroll 4
+    for (int k = 0; k < m; ++k) acc += (double)x[k];
     const float mean_f = (float)(acc / (double)m);
     float mx = -INFINITY;
     double s1 = 0;
-    for (long long k = 0; k < m; ++k) {
-        const float v = demod[lo + k] - mean_f;
+#pragma unroll 4
+    for (int k = 0; k < m; ++k) {
+        const float v = x[k] - mean_f;
         mx = fmaxf(mx, v);
         s1 += (double)v;
     }
     if ((double)mx > 30 * hz_ire) return nan("");
     const double mu = s1 / (double)m;
     double ss = 0;
-    for (long long k = 0; k < m; ++k) {
-        const double d = (double)(demod[lo + k] - mean_f) - mu;
+#pragma unroll 4
+    for (int k = 0; k < m; ++k) {
+        const double d = (double)(x[k] - mean_f) - mu;
         ss += d * d;
     }
     return sqrt(ss / (double)m) * 1.4142135623730951;
@@ -627,161 +660,216 @@ __device__ __forceinline__ double phase_distance(double x, double c) {
     return d;
 }
 
-// one refine_linelocs_pilot pass over ll (shared), in place
+constexpr int kRefineWarps = 8;      // lines per CTA of the per-line kernels
+constexpr int kPalThreads = 1024;    // one CTA per PAL field
+constexpr int kLevelLines = 303;     // lines 11 .. 312 and line 6 of the sequence
+constexpr int kLevelWin = 99;        // samples of a burst level (odd: lanes on different banks; 40 MSPS needs 98)
+static_assert(kMaxL <= kPalThreads && kLevelLines <= kPalThreads, "one thread per line");
+
+// For each of the first `count` threads the largest v of the threads up to and
+// including it.  All threads of the CTA; wsum: 32 ints.
+__device__ __forceinline__ int block_max_scan(int v, int* wsum) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, v, o);
+        if (lane >= o) v = max(v, y);
+    }
+    if (lane == 31) wsum[warp] = v;
+    __syncthreads();
+    for (int w = 0; w < warp; ++w) v = max(v, wsum[w]);
+    __syncthreads();
+    return v;
+}
+
+// one refine_linelocs_pilot pass over ll (shared), in place: a warp per line
+// finds the pilot's peak and the crossing after it, a thread per line the rest
 __device__ void pilot_pass(const LineParams& P, double* ll, const float* pilot, long long n, double* zcs,
-                           double* plen, unsigned char* ok, double* red) {
-    const int l = threadIdx.x;
-    double zc = 0;
-    bool good = false;
-    if (l < kPilotLines) {
+                           double* plen, unsigned char* ok, double* red, int* wsum) {
+    const int lane = threadIdx.x & 31;
+    for (int l = threadIdx.x >> 5; l < kPilotLines; l += kPalThreads / 32) {
         double adjfreq = P.freq;
         if (l > 1) adjfreq /= (ll[l] - ll[l - 1]) / P.linelen;
-        plen[l] = (adjfreq / P.pilot_mhz) / 2;
+        const double pl = (adjfreq / P.pilot_mhz) / 2;
         const double b0 = ll[l];
         const long long st = (long long)(b0 + 0.0);
         long long sp = (long long)(b0 + 6 * P.linefreq0 + 0.0 + 1);
         sp = min(sp, n);
         const double lsoffset = ll[l] - (double)st;
+        double zc = 0;
+        bool good = false;
         if (st >= 0 && sp > st) {
             const float* seg = pilot + st;
-            const long long m = sp - st;
-            long long peak = 0;
+            const int m = (int)(sp - st);
+            // the first of the largest magnitudes
+            int peak = 0x7fffffff;
             float best = -1.0f;
-            for (long long k = 0; k < m; ++k) {
+#pragma unroll 8
+            for (int k = lane; k < m; k += 32) {
                 const float v = fabsf(seg[k]);
                 if (v > best) {
                     best = v;
                     peak = k;
                 }
             }
+#pragma unroll
+            for (int o = 16; o; o >>= 1) {
+                const float bv = __shfl_xor_sync(0xffffffffu, best, o);
+                const int bp = __shfl_xor_sync(0xffffffffu, peak, o);
+                if (bv > best || (bv == best && bp < peak)) {
+                    best = bv;
+                    peak = bp;
+                }
+            }
+            if (peak == 0x7fffffff) peak = 0;
             double zb;
-            if (calczc(seg, m, (double)peak, 0.0, 0, 16, zb)) {
-                zc = (zb - lsoffset) / plen[l];
+            if (warp_calczc(seg, (long long)m, (double)peak, 0.0, 0, 16, zb)) {
+                zc = (zb - lsoffset) / pl;
                 good = true;
             }
         }
-        zcs[l] = zc;
-        ok[l] = good;
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        // a line without a crossing repeats the previous line's value
-        double last = 0;
-        for (int k = 0; k < kPilotLines; ++k) {
-            if (!ok[k]) zcs[k] = last;
-            last = zcs[k];
+        if (lane == 0) {
+            plen[l] = pl;
+            zcs[l] = zc;
+            ok[l] = good;
         }
     }
     __syncthreads();
+    // a line without a crossing repeats the previous line's value (0 before any)
+    const int l = threadIdx.x;
+    const int from = block_max_scan(l < kPilotLines && ok[l] ? l : -1, wsum);
+    const double z = l < kPilotLines && from >= 0 ? zcs[from] : 0.0;
     // mean phase of the fractional parts
-    double cs = 0, sn = 0;
     if (l < kPilotLines) {
-        const double x = zcs[l];
-        const double x2 = x - (double)(int)x;
+        const double x2 = z - (double)(int)z;
         const double th = x2 * 3.14159265358979323846 * 2;
-        cs = cos(th);
-        sn = sin(th);
-    }
-    red[2 * l] = cs;
-    red[2 * l + 1] = sn;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        double a = 0, b = 0;
-        for (int k = 0; k < kPilotLines; ++k) {
-            a += red[2 * k];
-            b += red[2 * k + 1];
-        }
-        double am = atan2(b / kPilotLines, a / kPilotLines) / (3.14159265358979323846 * 2);
-        if (am < 0) am = 1 + am;
-        red[0] = am;
+        red[l] = cos(th);
+        red[kMaxL + l] = sin(th);
     }
     __syncthreads();
-    const double am = red[0];
-    if (l < kPilotLines) ll[l] += phase_distance(zcs[l], am) * plen[l];
+    __shared__ double s_sum[2];
+    if (l == 0 || l == 32) {  // the two sums in line order, side by side
+        const double* v = red + (l ? kMaxL : 0);
+        double a = 0;
+#pragma unroll 8
+        for (int k = 0; k < kPilotLines; ++k) a += v[k];
+        s_sum[l >> 5] = a;
+    }
+    __syncthreads();
+    double am = atan2(s_sum[1] / kPilotLines, s_sum[0] / kPilotLines) / (3.14159265358979323846 * 2);
+    if (am < 0) am = 1 + am;
+    if (l < kPilotLines) ll[l] += phase_distance(z, am) * plen[l];
     __syncthreads();
 }
 
-__global__ void __launch_bounds__(kLineThreads) lines_hsync_kernel(const __grid_constant__ LineParams P) {
+// refine_linelocs_hsync, one warp per line: the line location into P.ll2, its
+// flag into linebad.  Each line's samples (from just before its search start
+// to past its porch) are staged in shared memory by one burst of independent
+// loads, so the searches below do not wait on one global load after another.
+// Bound: latency, one line's chain of searches.  Lines of a field are
+// independent, so they spread over the chip.  With one CTA walking a field's
+// lines, and one thread per line on the bursts or pilots after it, this stage
+// took 220 us for one NTSC field and 355 us for 15 PAL ones; with a warp per
+// line (ncu) 7 + 15 us and 14 + 107 us (this kernel and the next).
+__global__ void __launch_bounds__(32 * kRefineWarps) lines_hsync_kernel(const __grid_constant__ LineParams P) {
+    const int f = P.a.first_field + blockIdx.y;
+    const ldg_lines_args& a = P.a;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int li = blockIdx.x * kRefineWarps + warp;
+    if (li >= a.proclines) return;
+    const long long base = a.startloc[f];
+    const long long n = min((long long)a.wlen[f], (long long)(a.capture_len - base));
+    const float* d05 = a.d05 + base;
+    __shared__ float win[kRefineWarps][kHsWin];
+    const double start = a.linelocs1[(long long)f * kMaxL + li];
+    bool b = a.linebad1[(long long)f * kMaxL + li];
+    double v2 = start;
+    if ((li >= 3 && li <= 6) || (P.system == 1 && li >= 1 && li <= 2)) {
+        b = true;
+    } else {
+        const double l1 = start - P.freq;
+        const long long wb = max((long long)l1 - 64, 0LL);
+        const long long we = min(wb + kHsWin, n);
+        float* w = win[warp];
+        for (long long i = wb + lane; i < we; i += 32) w[i - wb] = d05[i];
+        __syncwarp();
+        const WinView x{d05, w, wb, we};
+        double zc;
+        if (warp_calczc(x, n, l1, P.half_sync, 0, P.freq * 2, zc) && !b) {
+            v2 = zc;
+            float mn, mx;
+            warp_minmax(x, (long long)(zc - (P.freq * 0.75)), (long long)(zc + (P.freq * 8)), n, mn, mx);
+            if ((double)mn < P.lo_ok || (double)mx > P.hi_ok) {
+                b = true;
+            } else {
+                const double porch =
+                    warp_median_f32(x, (long long)(zc + (P.freq * 8)), (long long)(zc + (P.freq * 9)), n);
+                const double sync =
+                    warp_median_f32(x, (long long)(zc + (P.freq * 1)), (long long)(zc + (P.freq * 2.5)), n);
+                double zc2;
+                if (warp_calczc(x, n, l1, (porch + sync) / 2, 0, 400, zc2) && fabs(zc2 - zc) < (P.freq / 2))
+                    v2 = zc2;
+                else
+                    b = true;
+            }
+        } else {
+            b = true;
+        }
+    }
+    if (lane == 0) {
+        P.ll2[(long long)f * kMaxL + li] = b ? start : v2;
+        a.linebad[(long long)f * kMaxL + li] = b;
+    }
+}
+
+// NTSC, one warp per line: the second differences' bad-line flags (a line's
+// flag depends on the two lines before it and the one after), linelocs2 out,
+// the line's burst zero crossings.
+__global__ void __launch_bounds__(32 * kRefineWarps) lines_burst_kernel(const __grid_constant__ LineParams P) {
+    const int f = P.a.first_field + blockIdx.y;
+    const ldg_lines_args& a = P.a;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int l = blockIdx.x * kRefineWarps + warp, nl = a.proclines;
+    if (l >= nl) return;
+    const double* ll = P.ll2 + (long long)f * kMaxL;
+    if (lane == 0) {
+        bool bad = false;
+        if (l >= 1 && l + 1 < nl) bad |= fabs((ll[l + 1] - ll[l]) - (ll[l] - ll[l - 1])) > 4;
+        if (l >= 2) bad |= fabs((ll[l] - ll[l - 1]) - (ll[l - 1] - ll[l - 2])) > 4;
+        if (bad) a.linebad[(long long)f * kMaxL + l] = 1;
+        if (a.linelocs2) a.linelocs2[(long long)f * kMaxL + l] = ll[l];
+    }
+    if (l >= kBurstLines) return;
+    const long long base = a.startloc[f];
+    const long long n = min((long long)a.wlen[f], (long long)(a.capture_len - base));
+    __shared__ float win[kRefineWarps][2 * kBurstWin + 1];
+    warp_burst_record(P, ll, l, a.linecount[f], a.burst + base, a.demod + base, n, win[warp], win[warp] + kBurstWin + 1,
+                      P.rec + (long long)f * kBurstLines + l);
+}
+
+// PAL, one CTA per field: second differences, two pilot passes, fix_badlines
+// (no backup, lines from 0), the inputs of the 8-field sequence.
+__global__ void __launch_bounds__(kPalThreads) lines_pal_kernel(const __grid_constant__ LineParams P) {
+    extern __shared__ float lev[];  // kLevelLines x kLevelWin
     const int f = P.a.first_field + blockIdx.x;
     const ldg_lines_args& a = P.a;
     const long long base = a.startloc[f];
     const long long n = min((long long)a.wlen[f], (long long)(a.capture_len - base));
-    const float* d05 = a.d05 + base;
     const int nl = a.proclines;
-    __shared__ double ll1[kMaxL], ll[kMaxL], tmp[kMaxL];
+    __shared__ double ll[kMaxL], tmp[kMaxL], plen[kMaxL], red[2 * kMaxL];
     __shared__ unsigned char bad[kMaxL], okf[kMaxL];
-    __shared__ double red[2 * kLineThreads];
-    const int i = threadIdx.x;
+    __shared__ int wsum[32];
+    __shared__ float win[4][2 * kBurstWin + 1];
+    static_assert(2 * kMaxL >= 512, "the level sort's keys");
+    const int i = threadIdx.x, lane = i & 31, warp = i >> 5;
     if (i < nl) {
-        ll1[i] = a.linelocs1[(long long)f * kMaxL + i];
-        bad[i] = a.linebad1[(long long)f * kMaxL + i];
-    }
-    __syncthreads();
-    // refine_linelocs_hsync: one warp per line; each line's samples (from just
-    // before its search start to past its porch) staged in shared memory by
-    // one burst of independent loads, so the searches below do not wait on
-    // one global load after another
-    {
-        const int lane = threadIdx.x & 31, nwarps = blockDim.x >> 5;
-        __shared__ float win[kLineThreads / 32][kHsWin];
-        for (int li = threadIdx.x >> 5; li < nl; li += nwarps) {
-            bool b = bad[li];
-            double v2 = ll1[li];
-            if ((li >= 3 && li <= 6) || (P.system == 1 && li >= 1 && li <= 2)) {
-                b = true;
-            } else {
-                const double l1 = ll1[li] - P.freq;
-                const long long wb = max((long long)l1 - 64, 0LL);
-                const long long we = min(wb + kHsWin, n);
-                float* w = win[threadIdx.x >> 5];
-                __syncwarp();
-                for (long long i = wb + lane; i < we; i += 32) w[i - wb] = d05[i];
-                __syncwarp();
-                const WinView x{d05, w, wb, we};
-                double zc;
-                if (warp_calczc(x, n, l1, P.half_sync, 0, P.freq * 2, zc) && !b) {
-                    v2 = zc;
-                    float mn, mx;
-                    warp_minmax(x, (long long)(zc - (P.freq * 0.75)), (long long)(zc + (P.freq * 8)), n, mn, mx);
-                    if ((double)mn < P.lo_ok || (double)mx > P.hi_ok) {
-                        b = true;
-                    } else {
-                        const double porch =
-                            warp_median_f32(x, (long long)(zc + (P.freq * 8)), (long long)(zc + (P.freq * 9)), n);
-                        const double sync =
-                            warp_median_f32(x, (long long)(zc + (P.freq * 1)), (long long)(zc + (P.freq * 2.5)), n);
-                        double zc2;
-                        if (warp_calczc(x, n, l1, (porch + sync) / 2, 0, 400, zc2) && fabs(zc2 - zc) < (P.freq / 2))
-                            v2 = zc2;
-                        else
-                            b = true;
-                    }
-                } else {
-                    b = true;
-                }
-            }
-            if (b) v2 = ll1[li];
-            if (lane == 0) {
-                ll[li] = v2;
-                bad[li] = b;
-            }
-        }
+        ll[i] = P.ll2[(long long)f * kMaxL + i];
+        bad[i] = a.linebad[(long long)f * kMaxL + i];
     }
     __syncthreads();
     deriv_error_block(ll, bad, nl);
-    if (P.system == 0) {
-        // NTSC: linelocs2 out, burst zero crossings per line
-        if (i < nl) P.ll2[(long long)f * kMaxL + i] = ll[i];
-        if (i < nl && a.linelocs2) a.linelocs2[(long long)f * kMaxL + i] = ll[i];
-        if (i < nl) a.linebad[(long long)f * kMaxL + i] = bad[i];
-        if (i < kBurstLines && i < nl)
-            burst_record(P, ll, i, a.linecount[f], a.burst + base, a.demod + base, n,
-                         P.rec[(long long)f * kBurstLines + i]);
-        return;
-    }
-    // PAL: two pilot passes, then fix_badlines (no backup, lines from 0)
-    pilot_pass(P, ll, a.pilot + base, n, tmp, ll1, okf, red);
-    pilot_pass(P, ll, a.pilot + base, n, tmp, ll1, okf, red);
+    pilot_pass(P, ll, a.pilot + base, n, tmp, plen, okf, red, wsum);
+    pilot_pass(P, ll, a.pilot + base, n, tmp, plen, okf, red, wsum);
     deriv_error_block(ll, bad, nl);
     fix_badlines_block(ll, bad, tmp, nl, 0);
     if (i < nl) {
@@ -793,29 +881,36 @@ __global__ void __launch_bounds__(kLineThreads) lines_hsync_kernel(const __grid_
     // calc_burstmedian runs while the field's line count and offset are still
     // compute_linelocs' (263 / 262 and 0), determine_field_number after they
     // become 312 / 313 and 2 / 3
-    {
-        const bool isf = a.isfirst[f] != 0;
-        const int lc_med = isf ? 263 : 262;
-        const int off = isf ? 2 : 3;
-        const int lc_seq = (isf ? 312 : 313) + off;
-        const float* demod = a.demod + base;
-        double lvl = INFINITY;
-        if (i >= 11 && i < 313) {
-            const double b = pal_burstlevel(P, tmp, i, lc_med, demod, n, P.hz_ire);
-            if (!isnan(b)) lvl = b;
-        }
-        for (int k = i; k < 512; k += blockDim.x) red[k] = k == i ? lvl : INFINITY;
-        const int cnt = __syncthreads_count(lvl != INFINITY);
-        bitonic512(red);
-        if (i == 0) {
-            double* out = P.adjs + (long long)f * kBurstLines;
-            out[0] = pal_burstlevel(P, tmp, 6 + off, lc_seq, demod, n, P.hz_ire);
-            out[1] = cnt ? sorted_median(red, cnt) / P.hz_ire : 0.0;
-        }
-        if (i < 4)
-            burst_record(P, tmp, 7 + 4 * i + off, lc_seq, a.burst + base, demod, n,
-                         P.rec[(long long)f * kBurstLines + i]);
+    const bool isf = a.isfirst[f] != 0;
+    const int lc_med = isf ? 263 : 262;
+    const int off = isf ? 2 : 3;
+    const int lc_seq = (isf ? 312 : 313) + off;
+    const float* demod = a.demod + base;
+    // the levels' samples staged a warp per line, then a thread per line sums
+    // them in order
+    for (int e = warp; e < kLevelLines; e += kPalThreads / 32) {
+        const LevelWindow w = e < kLevelLines - 1 ? pal_level_window(P, tmp, 11 + e, lc_med, n)
+                                                  : pal_level_window(P, tmp, 6 + off, lc_seq, n);
+        if (w.hi - w.lo <= kLevelWin)
+            for (long long k = w.lo + lane; k < w.hi; k += 32) lev[e * kLevelWin + (int)(k - w.lo)] = demod[k];
     }
+    __syncthreads();
+    double lvl = INFINITY;
+    if (i < kLevelLines) {
+        const LevelWindow w = i < kLevelLines - 1 ? pal_level_window(P, tmp, 11 + i, lc_med, n)
+                                                  : pal_level_window(P, tmp, 6 + off, lc_seq, n);
+        const int m = (int)max(w.hi - w.lo, 0LL);
+        const double b = pal_burstlevel(m <= kLevelWin ? lev + i * kLevelWin : demod + w.lo, m, P.hz_ire);
+        if (i == kLevelLines - 1) P.adjs[(long long)f * kBurstLines] = b;
+        else if (!isnan(b)) lvl = b;
+    }
+    if (i < 512) red[i] = lvl;
+    const int cnt = __syncthreads_count(lvl != INFINITY);
+    bitonic512(red);
+    if (i == 0) P.adjs[(long long)f * kBurstLines + 1] = cnt ? sorted_median(red, cnt) / P.hz_ire : 0.0;
+    if (warp < 4)
+        warp_burst_record(P, tmp, 7 + 4 * warp + off, lc_seq, a.burst + base, demod, n, win[warp],
+                          win[warp] + kBurstWin + 1, P.rec + (long long)f * kBurstLines + warp);
 }
 
 // np.median of 16 doubles (mean of the two middle ones): Batcher's
@@ -1233,8 +1328,8 @@ __global__ void __launch_bounds__(512) burst_apply_kernel(const __grid_constant_
     const int lc = a.linecount[f];
     __shared__ double ll2[kMaxL], adj_ll[kMaxL], out[kMaxL], adjs[kBurstLines];
     __shared__ unsigned char bad[kMaxL], has[kBurstLines];
-    __shared__ double keys[512];
-    __shared__ int nadj;
+    __shared__ double keys[512], mid[2];
+    __shared__ int nadj, wsum[32];
     const int l = threadIdx.x;
     if (l == 0) nadj = 0;
     if (l < nl) {
@@ -1260,25 +1355,31 @@ __global__ void __launch_bounds__(512) burst_apply_kernel(const __grid_constant_
     keys[l] = isnan(adj) ? INFINITY : adj;
     if (l < nl) adj_ll[l] = ll2[l];
     __syncthreads();
-    bitonic512(keys);
-    if (l == 0) {
-        const int cnt = nadj;
-        if (cnt) {
-            const double med = sorted_median(keys, cnt);
-            double lastvalid = med;
-            for (int k = 0; k < kBurstLines && k < nl; ++k) {
-                if (has[k] && adjs[k] - med >= -2 && adjs[k] - med <= 2) {
-                    adj_ll[k] += adjs[k];
-                    lastvalid = adjs[k];
-                } else {
-                    adj_ll[k] += lastvalid;
-                }
+    const int cnt = nadj;  // the same for all threads
+    if (cnt) {
+        // the adjustments' median: every line counts those below and equal to its own
+        if (l < kBurstLines && l < nl && has[l]) {
+            const double mine = keys[l];
+            int less = 0, same = 0;
+#pragma unroll 4
+            for (int k = 0; k < kBurstLines; ++k) {
+                less += keys[k] < mine;
+                same += keys[k] == mine;
             }
-            const bool first = a.isfirst[f] != 0, f14 = P.field14[f] != 0;
-            a.field_phase[f] = first ? (f14 ? 1 : 3) : (f14 ? 4 : 2);
-        } else {
-            a.field_phase[f] = 1;
+            const int r1 = cnt & 1 ? cnt / 2 : cnt / 2 - 1, r2 = cnt / 2;
+            if (less <= r1 && r1 < less + same) mid[0] = mine;
+            if (less <= r2 && r2 < less + same) mid[1] = mine;
         }
+        __syncthreads();
+        const double med = cnt & 1 ? mid[1] : (mid[0] + mid[1]) / 2.0;
+        // a line without a valid adjustment takes the last valid one before it (the median before any)
+        const bool valid = l < kBurstLines && l < nl && has[l] && adj - med >= -2 && adj - med <= 2;
+        const int from = block_max_scan(valid ? l : -1, wsum);
+        if (l < kBurstLines && l < nl) adj_ll[l] += from >= 0 ? adjs[from] : med;
+    }
+    if (l == 0) {
+        const bool first = a.isfirst[f] != 0, f14 = cnt && P.field14[f] != 0;
+        a.field_phase[f] = cnt ? (first ? (f14 ? 1 : 3) : (f14 ? 4 : 2)) : 1;
     }
     __syncthreads();
     // fix_badlines(linelocs3, linelocs2): deriv error, NaN from backup, interpolate (from line 1)
@@ -1446,7 +1547,27 @@ extern "C" int ldg_lines_refine(ldg_ctx* c, const ldg_lines_args* a) {
     cudaSetDevice(ldg::ctx_device(c));
     cudaStream_t st = (cudaStream_t)a->stream;
     const int stages = a->stages ? a->stages : 7;
-    if (stages & 1) lines_hsync_kernel<<<P.a.count, kLineThreads, 0, st>>>(P);
+    if (stages & 1) {
+        const unsigned per_field = (unsigned)((a->proclines + kRefineWarps - 1) / kRefineWarps);
+        if (P.system == 1) {
+            constexpr size_t bytes = (size_t)kLevelLines * kLevelWin * sizeof(float);
+            static ldg::SmemAttr attr;
+            if (attr.ensure(lines_pal_kernel, bytes) != cudaSuccess) {
+                if (prev >= 0) cudaSetDevice(prev);
+                return ldg::lines_fail(LDG_ERR_CUDA, std::string("ldg_lines_refine: ") +
+                                                         cudaGetErrorString(cudaGetLastError()));
+            }
+        }
+        for (int lo = 0; lo < P.a.count; lo += 65535) {  // grid.y limit
+            LineParams Q = P;
+            Q.a.first_field = P.a.first_field + lo;
+            const unsigned nfl = (unsigned)(P.a.count - lo < 65535 ? P.a.count - lo : 65535);
+            lines_hsync_kernel<<<dim3(per_field, nfl), 32 * kRefineWarps, 0, st>>>(Q);
+            if (P.system == 0) lines_burst_kernel<<<dim3(per_field, nfl), 32 * kRefineWarps, 0, st>>>(Q);
+        }
+        if (P.system == 1)
+            lines_pal_kernel<<<P.a.count, kPalThreads, (size_t)kLevelLines * kLevelWin * sizeof(float), st>>>(P);
+    }
     if (P.system == 1 && (stages & 2)) pal_sequence_kernel<<<1, 32, 0, st>>>(P);
     if (P.system == 0) {
         if (stages & 2) {
