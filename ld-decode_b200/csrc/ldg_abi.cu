@@ -115,12 +115,12 @@ struct ldg_ctx {
     } tws[4];
     int tws_next = 0;
     size_t lines_cap = 0;
-    // ldg_dropouts: device field descriptors and error lists; reused once the
+    // ldg_dropouts: device field descriptors and scratch; reused once the
     // launch that last used them has completed
     ldg::DropField* d_drop_fields = nullptr;
     size_t drop_fields_cap = 0;
-    int* d_drop_errs = nullptr;
-    size_t drop_errs_cap = 0;
+    char* d_drop_scratch = nullptr;
+    size_t drop_scratch_cap = 0;
     cudaEvent_t drop_done = nullptr;
     bool drop_used = false;
     int notch_lo = 0, notch_hi = 0;      // PAL_V4300D_NotchFilter search band (bins), 0 0: off
@@ -349,7 +349,7 @@ void ldg_ctx_destroy(ldg_ctx* c) {
     cudaFree(c->d_rftbc);
     if (c->rftbc_done) cudaEventDestroy(c->rftbc_done);
     cudaFree(c->d_drop_fields);
-    cudaFree(c->d_drop_errs);
+    cudaFree(c->d_drop_scratch);
     if (c->drop_done) cudaEventDestroy(c->drop_done);
     for (auto& w : c->tws) {
         if (w.used) cudaEventSynchronize(w.done);
@@ -980,7 +980,9 @@ int ldg_dropouts(ldg_ctx* c, const ldg_dropout_params* p, const ldg_dropout_fiel
     if (c->drop_used) LDG_CK(cudaEventSynchronize(c->drop_done));
     int rc = grow((void**)&c->d_drop_fields, &c->drop_fields_cap, (size_t)nfields * sizeof(ldg::DropField));
     if (rc) return rc;
-    rc = grow((void**)&c->d_drop_errs, &c->drop_errs_cap, (size_t)nfields * p->err_cap * sizeof(int));
+    long long max_len = 0;
+    for (int i = 0; i < nfields; ++i) max_len = std::max(max_len, (long long)fields[i].len);
+    rc = grow((void**)&c->d_drop_scratch, &c->drop_scratch_cap, ldg::dropout_scratch(nfields, max_len, nullptr, nullptr));
     if (rc) return rc;
     std::vector<ldg::DropField> h(nfields);
     for (int i = 0; i < nfields; ++i) {
@@ -1007,7 +1009,8 @@ int ldg_dropouts(ldg_ctx* c, const ldg_dropout_params* p, const ldg_dropout_fiel
     k.vmax05 = hz(115);
     k.smin = hz(pal ? p->vsync_ire - 60 : p->vsync_ire - 35);
     k.smin05 = hz(p->vsync_ire - 10);
-    cudaError_t e = ldg::launch_dropouts(c->d_drop_fields, nfields, k, c->d_drop_errs, drops, counts, rfstd, st);
+    cudaError_t e = ldg::launch_dropouts(c->d_drop_fields, nfields, max_len, k, c->d_drop_scratch, drops, counts,
+                                          rfstd, st);
     if (e != cudaSuccess) return fail(LDG_ERR_CUDA, std::string("dropout launch: ") + cudaGetErrorString(e));
     LDG_CK(cudaEventRecord(c->drop_done, st));
     c->drop_used = true;

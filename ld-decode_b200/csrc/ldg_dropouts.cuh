@@ -4,7 +4,8 @@
 
 namespace ldg {
 
-constexpr int kDropThreads = 512;
+constexpr int kDropStdTile = 4096;   // samples per CTA of the standard deviation
+constexpr int kDropMaskTile = 8192;  // samples per CTA of the error mask
 constexpr int kMaxDropRegions = 512;  // sync areas: lines 1 .. nlines-1, nlines <= 513
 
 struct DropField {
@@ -23,7 +24,24 @@ struct DropConsts {
     float vmin, vmax, vmin05, vmax05, smin, smin05;  // float32 limits (Hz)
 };
 
-cudaError_t launch_dropouts(const DropField* fields, int nfields, const DropConsts& k, int* errs, int* drops,
-                            int* counts, double* rfstd, cudaStream_t stream);
+// Device scratch of a call, per field: tiles' rfhpf sums and squared
+// deviations, sync areas (start, prefix maximum of the ends), a flag for areas
+// that cannot be built, the error mask.
+struct DropScratch {
+    double2* part;
+    int2* areas;
+    int* bad;
+    float* rf_hi;       // the error limit of rfhpf (3 standard deviations)
+    unsigned* words;
+    int tiles;          // entries of part per field
+    long long nwords;   // mask words per field
+    int place_words;    // mask words the placement's shared memory holds
+};
+
+// Bytes of scratch for fields of up to max_len samples; with sc, its layout at base.
+size_t dropout_scratch(int nfields, long long max_len, char* base, DropScratch* sc);
+
+cudaError_t launch_dropouts(const DropField* fields, int nfields, long long max_len, const DropConsts& k, char* scratch,
+                            int* drops, int* counts, double* rfstd, cudaStream_t stream);
 
 }  // namespace ldg

@@ -72,7 +72,8 @@ def run(rf, descs, stream=None, err_cap=ERR_CAP, out_cap=OUT_CAP, rfstd=False):
         if c[bad[0], 1] < 0:
             why = f"more than {err_cap} error samples"
         raise L.LdgError(L.LDG_ERR_RANGE, f"dropout detection, field {int(bad[0])}: {why}")
-    d = drops.cpu().numpy().reshape(n, out_cap, 3)
+    # only the rows that were written come back
+    d = drops.view(n, out_cap, 3)[:, :max(int(c[:, 0].max()), 1)].cpu().numpy()
     out = []
     for i in range(n):
         k = int(c[i, 0])

@@ -103,6 +103,46 @@ def test_caps_and_bad_fields_raise(capture):
     torch.cuda.synchronize()
 
 
+@pytest.mark.parametrize("rate,runs", [(0.0, 0), (0.0, 3), (3e-4, 10), (3e-3, 30), (0.05, 50), (0.3, 0), (0.95, 0)])
+@pytest.mark.parametrize("order", [True, False])
+def test_masks_equal_oracle(cuda_ok, rate, runs, order):
+    """Error masks from empty to nearly full (spans that merge over gaps, end
+    at their cap, start off the ends of the kernel's tiles and words), two
+    fields of different lengths, with line locations in order and not (within
+    a sample, as the reference takes them): the oracle's lists exactly."""
+    import torch
+    from ldgpu import RFDecode
+    from ldgpu.dropouts import _field, run
+    rf = RFDecode(system="NTSC")
+    rng = np.random.default_rng(int(rate * 1e4) + runs)
+    lim = odrop.limits(rf.system, rf.DecoderParams["ire0"], rf.DecoderParams["hz_ire"], rf.SysParams["vsync_ire"])
+    descs, keep, want = [], [], []
+    for n, nlines, lineoffset in ((8192 * 9 + 1, 26, 0), (33333, 12, 1)):
+        ll = 1500.3 + 2542.2 * np.arange(nlines) + rng.normal(size=nlines) * 0.3
+        if not order:
+            ll[6], ll[7] = np.floor(ll[7]) + 0.75, np.floor(ll[7]) + 0.25
+        demod = rng.normal(rf.iretohz(20), 1e5, n).astype(np.float32)
+        bad = rng.random(n) < rate
+        for s, k in zip(rng.integers(0, n, runs), rng.integers(1, 1600, runs)):
+            bad[s:s + k] = True
+        demod[bad] = 2e6
+        d05 = np.full(n, rf.iretohz(20), np.float32)
+        raw, hp = demod.copy(), rng.normal(0, 100, n).astype(np.float32)
+        iserr, sd = odrop.mask(demod, d05, raw, hp, ll, lineoffset, nlines - lineoffset - 3, True, 190, rf.system,
+                               int(rf.delays["video_rot"]), rf.freq_hz_half, lim)
+        want.append((odrop.detect(iserr, ll, lineoffset, nlines - lineoffset - 3, rf.freq,
+                                  rf.SysParams["outlinelen"]), sd))
+        t = [torch.from_numpy(v).cuda() for v in (demod, d05, raw, hp, ll)]
+        keep.append(t)
+        descs.append(_field(*(v.data_ptr() for v in t[:4]), n, t[4].data_ptr(), nlines, lineoffset,
+                            nlines - lineoffset - 3, True, 190))
+    got, sd = run(rf, descs, rfstd=True)
+    for i, ((lines, starts, ends), std) in enumerate(want):
+        assert got[i] == (list(lines), list(starts), list(ends)), i
+        assert sd[i] == pytest.approx(std, rel=1e-12)
+    rf.close()
+
+
 @pytest.mark.parametrize("system", ["NTSC", "PAL"])
 def test_reference_golden_fields(cuda_ok, system):
     """The reference's own fields (its line locations and hsync length) on
