@@ -16,6 +16,7 @@
 //                      optional float32 rounding (the reference's own cast),
 //                      16-tap windowed-sinc gather with linear interpolation
 //                      between LUT phases, level adjust, uint16 conversion.
+#include <algorithm>
 #include <climits>
 
 #include "ldg_tbc.cuh"
@@ -829,43 +830,123 @@ cudaError_t launch_tbc(const TbcField* dfields, int nfields, long long max_nout,
 // expression term by term with every product and sum rounded on its own
 // (no fused multiply-adds), so the output is bit-identical.  One CTA per
 // (line, field).
-__global__ void __launch_bounds__(256) rf_tbc_kernel(const RfTbcField* fields) {
+//
+// Bound: the FP64 pipe (about one warp instruction per clock and SM;
+// conversions between integers and FP64 half that).  The polynomial's
+// coefficients are sums of 16-bit samples, exact in integers, and numbers
+// cross between int and double by an addition to 2^52 (and 2^51 or 2^31),
+// whose low word then is the integer: 17 FP64 operations per sample instead of
+// 21 and 8 conversions.  Five samples per thread are in flight, and one CTA
+// takes up to four lines.  50 PAL fields (40 M samples), B200 (ncu): 128 us
+// before, 88 us so.
+constexpr int kRfThreads = 256, kRfPer = 5, kRfMaxLines = 4;
+constexpr double kIntMagic = 6755399441055744.0;  // 2^52 + 2^51
+
+__device__ __forceinline__ double int_to_double(int k) {  // exact, |k| < 2^31
+    return __dsub_rn(__hiloint2double(0x43300000, k ^ (int)0x80000000), 4503601774854144.0);  // 2^52 + 2^31
+}
+
+// One output line: begin and scale of its input, the samples' output.
+struct RfLine {
+    double begin, sf;
+    int16_t* out;
+    int inside;  // every tap of the line lies inside the read
+};
+
+__global__ void __launch_bounds__(kRfThreads) rf_tbc_kernel(const RfTbcField* fields, int lines_per_cta) {
+    __shared__ RfLine s_line[kRfMaxLines];
     const RfTbcField& f = fields[blockIdx.y];
-    const int line = blockIdx.x;
-    if (line >= f.nout) return;
-    const int l = f.startline + line;
-    const double begin = __dsub_rn(f.ll[l], f.delay);
-    const double end = __dsub_rn(f.ll[l + 1], f.delay);
-    const double sf = __ddiv_rn(__dsub_rn(end, begin), (double)f.linelen);
-    int16_t* out = f.out + (long long)line * f.linelen;
-    for (int i = threadIdx.x; i < f.linelen; i += blockDim.x) {
-        const double coord = __dadd_rn(__dmul_rn((double)i, sf), begin);
-        // taps int(coord) - 1 .. int(coord) + 2 inside the read: 1 <= coord < len - 2
-        if (!(coord >= 1.0 && coord < (double)(f.len - 2))) {
-            atomicOr(f.status, LDG_TBC_OUT_OF_RANGE);
-            out[i] = 0;
+    const int line0 = blockIdx.x * lines_per_cta;
+    const int nlines = min(lines_per_cta, f.nout - line0);
+    if (nlines <= 0) return;
+    const int n = f.linelen;
+    const int16_t* in = f.in;
+    const double limit = (double)(f.len - 2);
+    // one thread per line: what the whole line shares
+    if (threadIdx.x < nlines) {
+        const int line = line0 + threadIdx.x, l = f.startline + line;
+        RfLine q;
+        q.begin = __dsub_rn(f.ll[l], f.delay);
+        const double end = __dsub_rn(f.ll[l + 1], f.delay);
+        q.sf = __ddiv_rn(__dsub_rn(end, q.begin), (double)n);
+        q.out = f.out + (long long)line * n;
+        // taps int(coord) - 1 .. int(coord) + 2 inside the read: 1 <= coord < len - 2.
+        // The rounded coordinate never turns back along a line, so its ends tell for all of it
+        const double last = __dadd_rn(__dmul_rn((double)(n - 1), q.sf), q.begin);
+        q.inside = f.len < (1ll << 31) && q.begin >= 1.0 && q.begin < limit && last >= 1.0 && last < limit;
+        s_line[threadIdx.x] = q;
+    }
+    __syncthreads();
+    for (int k = 0; k < nlines; ++k) {
+        const double begin = s_line[k].begin, sf = s_line[k].sf;
+        int16_t* out = s_line[k].out;
+        if (s_line[k].inside) {
+            double xi = (double)threadIdx.x;
+            for (int i0 = threadIdx.x; i0 < n; i0 += kRfPer * kRfThreads) {
+                // kRfPer samples at a time, their loads in flight together
+                double x[kRfPer];
+                int p0[kRfPer], p1[kRfPer], p2[kRfPer], p3[kRfPer];
+#pragma unroll
+                for (int j = 0; j < kRfPer; ++j) {
+                    // past the line's end: its last sample again
+                    const double xj = i0 + j * kRfThreads < n ? xi : (double)(n - 1);
+                    const double coord = __dadd_rn(__dmul_rn(xj, sf), begin);
+                    // floor: the sum with 2^52 rounded down
+                    const double fl = __dadd_rd(coord, 4503599627370496.0);
+                    const int16_t* q = in + (__double2loint(fl) - 1);
+                    p0[j] = __ldg(q);
+                    p1[j] = __ldg(q + 1);
+                    p2[j] = __ldg(q + 2);
+                    p3[j] = __ldg(q + 3);
+                    x[j] = __dsub_rn(coord, __dsub_rn(fl, 4503599627370496.0));
+                    xi = __dadd_rn(xi, (double)kRfThreads);
+                }
+#pragma unroll
+                for (int j = 0; j < kRfPer; ++j) {
+                    // p1 + 0.5 x (p2 - p0 + x (2 p0 - 5 p1 + 4 p2 - p3 + x (3 (p1 - p2) + p3 - p0)))
+                    const double c = int_to_double(3 * (p1[j] - p2[j]) + p3[j] - p0[j]);
+                    const double b =
+                        __dadd_rn(int_to_double(2 * p0[j] - 5 * p1[j] + 4 * p2[j] - p3[j]), __dmul_rn(x[j], c));
+                    const double a = __dadd_rn(int_to_double(p2[j] - p0[j]), __dmul_rn(x[j], b));
+                    // half of x a is exact, so this rounds as (0.5 x) a and then p1 + that do
+                    const double v = __fma_rn(0.5, __dmul_rn(x[j], a), int_to_double(p1[j]));
+                    if (i0 + j * kRfThreads < n)
+                        out[i0 + j * kRfThreads] = (int16_t)__double2loint(__dadd_rn(v, kIntMagic));  // half to even
+                }
+            }
             continue;
         }
-        const long long ic = (long long)coord;
-        const long long s = ic - 1;
-        const double p0 = f.in[s], p1 = f.in[s + 1], p2 = f.in[s + 2], p3 = f.in[s + 3];
-        const double x = __dsub_rn(coord, (double)ic);
-        // p1 + 0.5 x (p2 - p0 + x (2 p0 - 5 p1 + 4 p2 - p3 + x (3 (p1 - p2) + p3 - p0)))
-        const double c = __dsub_rn(__dadd_rn(__dmul_rn(3.0, __dsub_rn(p1, p2)), p3), p0);
-        const double b = __dadd_rn(
-            __dsub_rn(__dadd_rn(__dsub_rn(__dmul_rn(2.0, p0), __dmul_rn(5.0, p1)), __dmul_rn(4.0, p2)), p3),
-            __dmul_rn(x, c));
-        const double a = __dadd_rn(__dsub_rn(p2, p0), __dmul_rn(x, b));
-        const double v = __dadd_rn(p1, __dmul_rn(__dmul_rn(0.5, x), a));
-        out[i] = (int16_t)(int)rint(v);
+        for (int i = threadIdx.x; i < n; i += kRfThreads) {
+            const double coord = __dadd_rn(__dmul_rn((double)i, sf), begin);
+            if (!(coord >= 1.0 && coord < limit)) {
+                atomicOr(f.status, LDG_TBC_OUT_OF_RANGE);
+                out[i] = 0;
+                continue;
+            }
+            const long long ic = (long long)coord;
+            const int16_t* q = in + (ic - 1);
+            const double p0 = q[0], p1 = q[1], p2 = q[2], p3 = q[3];
+            const double x = __dsub_rn(coord, (double)ic);
+            const double c = __dsub_rn(__dadd_rn(__dmul_rn(3.0, __dsub_rn(p1, p2)), p3), p0);
+            const double b = __dadd_rn(
+                __dsub_rn(__dadd_rn(__dsub_rn(__dmul_rn(2.0, p0), __dmul_rn(5.0, p1)), __dmul_rn(4.0, p2)), p3),
+                __dmul_rn(x, c));
+            const double a = __dadd_rn(__dsub_rn(p2, p0), __dmul_rn(x, b));
+            const double v = __dadd_rn(p1, __dmul_rn(__dmul_rn(0.5, x), a));
+            out[i] = (int16_t)(int)rint(v);
+        }
     }
 }
 
 cudaError_t launch_rf_tbc(const RfTbcField* dfields, int nfields, int max_lines, cudaStream_t stream) {
     if (nfields <= 0 || max_lines <= 0) return cudaSuccess;
+    // several lines per CTA once there are CTAs enough for every SM: what a line
+    // shares (its descriptor, its locations, a division) is a chain of latencies
+    const int per = std::min(kRfMaxLines, (int)std::max(1ll, (long long)max_lines * nfields / (148 * 8)));
+    const unsigned gx = (unsigned)((max_lines + per - 1) / per);
     for (int off = 0; off < nfields; off += 65535) {
         const int n = nfields - off < 65535 ? nfields - off : 65535;
-        rf_tbc_kernel<<<dim3((unsigned)max_lines, (unsigned)n), 256, 0, stream>>>(dfields + off);
+        rf_tbc_kernel<<<dim3(gx, (unsigned)n), kRfThreads, 0, stream>>>(dfields + off, per);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }

@@ -104,3 +104,49 @@ def test_gpu_batch_equals_oracle(cuda_ok):
                             rf.linelen, "NTSC", fl.lineoffset, fl.linecount)
         np.testing.assert_array_equal(got[offs[i]:offs[i + 1]], want)
     rf.close()
+
+
+@pytest.mark.gpu
+def test_gpu_lines_at_the_reads_ends(cuda_ok):
+    """Lines that touch, cross and leave the read at either end: the samples
+    whose four taps lie inside are the oracle's, the others 0 with the range
+    error raised; full-scale samples, lines running backwards."""
+    import torch
+    from ldgpu import RFDecode
+    from ldgpu import lib as L
+    from ldgpu.field import tbc_status
+    from ldgpu.rftbc import descriptor, line_samples, run
+    rf = RFDecode(system="NTSC")
+    n, m = line_samples(rf), 9000
+    rng = np.random.default_rng(5)
+    x = rng.choice(np.array([-32768, -1, 0, 1, 32767], np.int16), m)
+    d = torch.from_numpy(x).cuda()
+    pad = 6000
+    wide = np.concatenate([np.zeros(pad), x, np.zeros(pad)]).astype(np.float64)
+
+    def check(b, e):
+        ll = torch.tensor([0.0, b, e], dtype=torch.float64, device="cuda")
+        out = torch.full((n,), 77, dtype=torch.int16, device="cuda")
+        ds = [descriptor(rf, d.data_ptr(), m, ll.data_ptr(), 3, 1, 1, out.data_ptr(), 0.0)]
+        run(rf, ds)
+        got = out.cpu().numpy()
+        coord = np.arange(n) * ((e - b) / n) + b
+        ok = (coord >= 1) & (coord < m - 2)
+        if ok.all():
+            tbc_status(rf)
+        else:
+            with pytest.raises(L.LdgError):
+                tbc_status(rf)
+        want = np.zeros(n, np.int16)
+        for i in np.nonzero(ok)[0]:
+            ic = int(coord[i])
+            p0, p1, p2, p3 = wide[pad + ic - 1:pad + ic + 3]
+            t = coord[i] - ic
+            v = p1 + 0.5 * t * (p2 - p0 + t * (2 * p0 - 5 * p1 + 4 * p2 - p3 + t * (3 * (p1 - p2) + p3 - p0)))
+            want[i] = np.int64(np.rint(v)).astype(np.int16)
+        np.testing.assert_array_equal(got, want, err_msg=str((b, e)))
+
+    for b, e in [(1.0, 2543.0), (0.99, 2543.0), (0.5, 2000.25), (-3.0, 2500.0), (m - 2600.5, m - 2.0), (m - 2500.0, m + 50.0),
+                 (2600.75, 33.5), (4000.0, 4000.0), (17.3, 8800.9)]:
+        check(b, e)
+    rf.close()
