@@ -84,7 +84,7 @@ struct ldg_ctx {
     float4* d_fpair[LDG_NFILTERS] = {};
     int fband[LDG_NFILTERS][2] = {};  // first and last bin whose float32 value is not zero
     float2* d_fpos[LDG_NFILTERS] = {};
-    float2* d_twpair = nullptr;
+    float4* d_twpair = nullptr;
     int variant = ldg::kVariantStockham;
     int blocks_per_cta = 0;  // ldg_demod_blocks: consecutive blocks per CTA (0: 2 for large batches, else 1)
     float* d_lut = nullptr;
@@ -298,18 +298,20 @@ int ldg_ctx_create(ldg_ctx** out, int32_t device, int32_t system, int32_t blockl
         const double ang = -two_pi * (double)k / ldg::kN;
         t32[k] = make_float2((float)std::cos(ang), (float)std::sin(ang));
     }
-    std::vector<float2> twp(ldg::ip::kPairs);
+    std::vector<float4> twp(ldg::ip::kPairs);
     for (int u = 0; u < ldg::ip::kPairs; ++u) {
-        const int k = ldg::ip::bin_of(ldg::ip::pair_pos(u));
-        const double ang = -two_pi * (double)k / ldg::kN;
-        twp[u] = make_float2((float)std::cos(ang), (float)std::sin(ang));
+        const int p = ldg::ip::pair_pos(u), q = ldg::ip::partner_pos(p);
+        const double ang = -two_pi * (double)ldg::ip::bin_of(p) / ldg::kN;
+        const uint32_t at[2] = {(uint32_t)(p + (p >> 4)) | (uint32_t)(q + (q >> 4)) << 16, (uint32_t)p | (uint32_t)q << 16};
+        twp[u] = make_float4((float)std::cos(ang), (float)std::sin(ang), 0.0f, 0.0f);
+        memcpy(&twp[u].z, at, sizeof(at));
     }
     if (cudaMalloc(&c->d_tw16, t16.size() * sizeof(float2)) != cudaSuccess ||
         cudaMemcpy(c->d_tw16, t16.data(), t16.size() * sizeof(float2), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMalloc(&c->d_tw32, t32.size() * sizeof(float2)) != cudaSuccess ||
         cudaMemcpy(c->d_tw32, t32.data(), t32.size() * sizeof(float2), cudaMemcpyHostToDevice) != cudaSuccess ||
-        cudaMalloc(&c->d_twpair, twp.size() * sizeof(float2)) != cudaSuccess ||
-        cudaMemcpy(c->d_twpair, twp.data(), twp.size() * sizeof(float2), cudaMemcpyHostToDevice) != cudaSuccess ||
+        cudaMalloc(&c->d_twpair, twp.size() * sizeof(float4)) != cudaSuccess ||
+        cudaMemcpy(c->d_twpair, twp.data(), twp.size() * sizeof(float4), cudaMemcpyHostToDevice) != cudaSuccess ||
         cudaMalloc(&c->d_status, sizeof(int)) != cudaSuccess || cudaMemset(c->d_status, 0, sizeof(int)) != cudaSuccess) {
         const std::string msg = cudaGetErrorString(cudaGetLastError());
         ldg_ctx_destroy(c);

@@ -77,7 +77,7 @@ struct DemodParams {
     const float4* fp_efm;
     const float2* g_pos;             // G at positions: g_pos[p] = G[bin_of(p)], p < M
     const float2* godd_pos;
-    const float2* tw_pair;           // W_N^k of pair u
+    const float4* tw_pair;           // pair u: W_N^k, then pad(p) | pad(q) << 16 and p | q << 16 of its positions (as bits)
     // bins [efm_klo, efm_khi] outside which the EFM filter's float32 bins are
     // zero (its C2R input is zero there)
     int efm_klo, efm_khi;

@@ -134,6 +134,34 @@ def test_batched_equals_plain(rf):
                                       plain["audio"]["audio_left"])
 
 
+def _device_outputs(rf, nblocks, shift=0):
+    """Output tensors of a batch, each starting `shift` elements past an aligned address."""
+    import torch
+    sl = rf.output_slices(True)
+    names = {**{k: ("video", torch.float32) for k in video_keys(rf.system)}, "rfhpf": ("rfhpf", torch.float32),
+             "efm": ("efm", torch.int16), "audio_left": ("audio", torch.float32), "audio_right": ("audio", torch.float32)}
+    return {k: torch.full((nblocks * sl[s][1] + shift + 8,), 7, dtype=t, device="cuda")[shift:shift + nblocks * sl[s][1]]
+            for k, (s, t) in names.items()}
+
+
+def test_outputs_off_alignment_equal(rf):
+    """Outputs whose buffers do not start on a pair of samples (no paired
+    stores) hold the same values, and nothing beside them is written."""
+    import torch
+    nb, U = 3, rf.blocklen - rf.blockcut - rf.blockcut_end
+    rng = np.random.default_rng(8)
+    cap = torch.from_numpy(rng.integers(-2000, 2000, (nb - 1) * U + rf.blocklen).astype(np.int16)).cuda()
+    a, b = _device_outputs(rf, nb), _device_outputs(rf, nb, 1)
+    torch.cuda.synchronize()
+    for o in (a, b):
+        rf.demod_blocks_device(cap.data_ptr(), nb, U, {k: v.data_ptr() for k, v in o.items()}, mtf_level=1)
+    rf.synchronize()
+    for k in a:
+        assert torch.equal(a[k], b[k]), k
+        whole = b[k].as_strided((b[k].numel() + 4,), (1,), 0)
+        assert float(whole[0]) == 7 and bool((whole[-3:] == 7).all()), k
+
+
 def test_delays_match_reference(rf):
     """computedelays on the GPU reproduces the reference's calibration."""
     g = golden("filters_" + rf.system.lower())
