@@ -528,6 +528,8 @@ int ldg_demod_blocks(ldg_ctx* c, const ldg_demod_args* a) {
     const int grid = (int)((nb + per_cta - 1) / per_cta);
     int rc = grow((void**)&c->d_scratch, &c->scratch_bytes, (size_t)nslots * ldg::kScratchPerCta);
     if (rc) return rc;
+    // a small batch: several CTAs per block, unless blocks per CTA are set
+    const int split = c->blocks_per_cta ? 1 : ldg::demod_split(c->variant, nb, c->scratch_bytes);
     if (!c->d_slots) {
         LDG_CK(cudaMalloc(&c->d_slots, (nslots + 1) * sizeof(int)));
         LDG_CK(cudaMemset(c->d_slots, 0, (nslots + 1) * sizeof(int)));
@@ -620,7 +622,7 @@ int ldg_demod_blocks(ldg_ctx* c, const ldg_demod_args* a) {
     p.scratch = c->d_scratch;
     p.tw16 = c->d_tw16;
     p.tw32 = c->d_tw32;
-    LDG_CK(cudaMemsetAsync(c->d_slots, 0, c->nslots * sizeof(int), st));
+    if (split == 1) LDG_CK(cudaMemsetAsync(c->d_slots, 0, c->nslots * sizeof(int), st));
     p.slot_lock = c->d_slots;
     p.nslots = c->nslots;
     p.error = c->d_slots + c->nslots;
@@ -629,7 +631,7 @@ int ldg_demod_blocks(ldg_ctx* c, const ldg_demod_args* a) {
     p.notch_hi = c->notch_hi;
     variant_tables(c, &p);
 
-    cudaError_t e = ldg::launch_demod(p, grid, st);
+    cudaError_t e = split > 1 ? ldg::launch_demod_split(p, split, st) : ldg::launch_demod(p, grid, st);
     if (e != cudaSuccess) return fail(LDG_ERR_CUDA, std::string("demod launch: ") + cudaGetErrorString(e));
     if (any_host) {
         for (int i = 1; i < nbuf; ++i)

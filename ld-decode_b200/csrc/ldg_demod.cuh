@@ -142,6 +142,11 @@ struct SpectrumParams {
 };
 
 cudaError_t launch_demod(const DemodParams& p, int grid, cudaStream_t stream);
+// CTAs per block (1, 2 or 4) for a batch of nblocks on the current device, its
+// scratch being scratch_bytes long.
+int demod_split(int variant, long long nblocks, size_t scratch_bytes);
+// A batch with c = 2 or 4 CTAs per block.
+cudaError_t launch_demod_split(const DemodParams& p, int c, cudaStream_t stream);
 cudaError_t launch_spectrum_blocks(const SpectrumParams& p, int nblocks, cudaStream_t stream);
 cudaError_t launch_audio2(const Audio2Params& p, int nsegs, cudaStream_t stream);
 // Sets the queue kernel's shared-memory size (call before a stream capture).

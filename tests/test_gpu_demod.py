@@ -162,6 +162,29 @@ def test_outputs_off_alignment_equal(rf):
         assert float(whole[0]) == 7 and bool((whole[-3:] == 7).all()), k
 
 
+@pytest.mark.parametrize("nb", [1, 2, 33, 34, 74, 75])
+@pytest.mark.parametrize("only", ["all", "video", "rfhpf", "audio_left"])
+def test_small_batches_equal_large(rf, nb, only):
+    """A small batch puts several CTAs on each block (four, two or one, by
+    the number of blocks); its outputs, whichever are asked for, equal those
+    of the same blocks with one CTA per block."""
+    import torch
+    U = rf.blocklen - rf.blockcut - rf.blockcut_end
+    rng = np.random.default_rng(nb)
+    cap = torch.from_numpy(rng.integers(-2000, 2000, (nb - 1) * U + rf.blocklen).astype(np.int16)).cuda()
+    keys = {"all": None, "video": video_keys(rf.system)[:3], "rfhpf": ("rfhpf", "efm"), "audio_left": ("audio_left",)}[only]
+    a, b = _device_outputs(rf, nb), _device_outputs(rf, nb)
+    torch.cuda.synchronize()
+    for o, per_cta in ((a, 0), (b, 1)):
+        rf.blocks_per_cta = per_cta
+        rf.demod_blocks_device(cap.data_ptr(), nb, U,
+                               {k: v.data_ptr() for k, v in o.items() if keys is None or k in keys}, mtf_level=1)
+        rf.synchronize()
+    rf.blocks_per_cta = 0
+    for k in a:
+        assert torch.equal(a[k], b[k]), k
+
+
 def test_delays_match_reference(rf):
     """computedelays on the GPU reproduces the reference's calibration."""
     g = golden("filters_" + rf.system.lower())
