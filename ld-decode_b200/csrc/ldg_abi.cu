@@ -201,12 +201,10 @@ int check_tbc_field(const ldg_tbc_field& f, const std::string& who) {
     return LDG_OK;
 }
 
-// Doubles of spline scratch a field needs: its pieces, median and
-// threshold, and with smoothing the IIR state every 32 output pixels.
+// Doubles of spline scratch a field needs.
 size_t tbc_spline_doubles(const ldg_tbc_field& f) {
     if (f.wow_interp < LDG_WOW_QUADRATIC) return 0;
-    const size_t nout = (size_t)f.linesout * f.outwidth;
-    return (size_t)ldg::kSplStride * f.nlines + 2 + (f.wow_smoothing > 0 ? (nout + 31) / 32 : 0);
+    return ldg::spline_scratch_doubles(f.nlines, f.outwidth, f.lineoffset, f.linesout, f.wow_smoothing > 0);
 }
 
 // Device descriptor of one field: geometry, levels and scratch pointers
@@ -237,7 +235,7 @@ void fill_tbc_field(const ldg_tbc_field& f, ldg::TbcField& d, double* seg, size_
     if (d.spline_k >= 2) {
         d.spl = spl;
         d.stat = spl + (size_t)ldg::kSplStride * f.nlines;
-        d.ybefore = f.wow_smoothing > 0 ? d.stat + 2 : nullptr;
+        d.ybefore = f.wow_smoothing > 0 ? d.stat + 2 + ldg::kSplCtlDoubles + ldg::kSplKeep : nullptr;
     } else {
         d.spl = d.stat = d.ybefore = nullptr;
     }
@@ -696,7 +694,7 @@ int ldg_tbc_fields(ldg_ctx* c, const ldg_tbc_field* fields, int32_t nfields, voi
         if (rc) return rc;
     }
     size_t llo = 0, sego = 0, splo = 0;
-    bool any_spline = false;
+    bool any_spline = false, any_smooth = false;
     for (int i = 0; i < nfields; ++i) {
         const ldg_tbc_field& f = fields[i];
         ldg::TbcField& d = h[i];
@@ -708,6 +706,7 @@ int ldg_tbc_fields(ldg_ctx* c, const ldg_tbc_field* fields, int32_t nfields, voi
         d.linelocs = ll_dev ? f.linelocs : c->d_ll + llo;
         fill_tbc_field(f, d, c->d_seg, seg_total, sego, c->d_seg + 3 * seg_total + splo, c->d_status);
         any_spline |= d.spline_k >= 2;
+        any_smooth |= d.spline_k >= 2 && d.smooth_b > 0;
         d.out_f32 = x.f32 ? (float*)(c->d_stage + x.f32_off) : f.out_f32;
         d.out_u16 = x.u16 ? (uint16_t*)(c->d_stage + x.u16_off) : f.out_u16;
         llo += f.nlines;
@@ -725,7 +724,7 @@ int ldg_tbc_fields(ldg_ctx* c, const ldg_tbc_field* fields, int32_t nfields, voi
         }
     }
     LDG_CK(cudaMemcpyAsync(c->d_fields, h.data(), nfields * sizeof(ldg::TbcField), cudaMemcpyHostToDevice, st));
-    cudaError_t e = ldg::launch_tbc(c->d_fields, nfields, max_nout, c->d_lut, 15.0, any_spline, st);
+    cudaError_t e = ldg::launch_tbc(c->d_fields, nfields, max_nout, c->d_lut, 15.0, any_spline, any_smooth, st);
     if (e != cudaSuccess) return fail(LDG_ERR_CUDA, std::string("tbc launch: ") + cudaGetErrorString(e));
     if (any_host) {
         for (int i = 0; i < nfields; ++i) {
@@ -789,7 +788,7 @@ int ldg_tbc_fields_async(ldg_ctx* c, const ldg_tbc_field* fields, int32_t nfield
     int rc = grow((void**)&w.d_seg, &w.seg_cap, (3 * seg_total + spl_total) * sizeof(double));
     if (rc) return rc;
     size_t sego = 0, splo = 0;
-    bool any_spline = false;
+    bool any_spline = false, any_smooth = false;
     for (int i = 0; i < nfields; ++i) {
         const ldg_tbc_field& f = fields[i];
         ldg::TbcField& d = w.h_fields[i];
@@ -797,6 +796,7 @@ int ldg_tbc_fields_async(ldg_ctx* c, const ldg_tbc_field* fields, int32_t nfield
         d.linelocs = f.linelocs;
         fill_tbc_field(f, d, w.d_seg, seg_total, sego, w.d_seg + 3 * seg_total + splo, c->d_status);
         any_spline |= d.spline_k >= 2;
+        any_smooth |= d.spline_k >= 2 && d.smooth_b > 0;
         d.out_f32 = f.out_f32;
         d.out_u16 = f.out_u16;
         sego += f.nlines - 1;
@@ -810,7 +810,7 @@ int ldg_tbc_fields_async(ldg_ctx* c, const ldg_tbc_field* fields, int32_t nfield
     } else {
         LDG_CK(cudaMemcpyAsync(w.d_fields, w.h_fields, nfields * sizeof(ldg::TbcField), cudaMemcpyHostToDevice, st));
     }
-    cudaError_t e = ldg::launch_tbc(w.d_fields, nfields, max_nout, c->d_lut, 15.0, any_spline, st);
+    cudaError_t e = ldg::launch_tbc(w.d_fields, nfields, max_nout, c->d_lut, 15.0, any_spline, any_smooth, st);
     if (e != cudaSuccess) return fail(LDG_ERR_CUDA, std::string("tbc launch: ") + cudaGetErrorString(e));
     LDG_CK(cudaEventRecord(w.done, st));
     w.used = true;

@@ -8,10 +8,10 @@
 //                      (slopes of the expected->actual line-location spline),
 //                      their pixel-weighted median and 15*MAD outlier rule ->
 //                      one level-adjust factor per segment.
-//   wow_spline_kernel  (quadratic / cubic wow interpolation only) one CTA per
-//                      field: the spline's pieces, the exact median and MAD
-//                      of the per-pixel wow factors by radix selection, and
-//                      with level smoothing the IIR's state every 32 pixels.
+//   spline_*           (quadratic / cubic wow interpolation only) the spline's
+//                      pieces, the exact median and MAD of the per-pixel wow
+//                      factors, and with level smoothing the IIR's state
+//                      every 32 pixels.
 //   tbc_gather_kernel  one thread per output pixels: FP64 spline coordinate,
 //                      optional float32 rounding (the reference's own cast),
 //                      16-tap windowed-sinc gather with linear interpolation
@@ -105,7 +105,7 @@ __device__ double weighted_median(const double* key, const long long* wt, long l
 __global__ void __launch_bounds__(kWowThreads) wow_levels_kernel(const TbcField* fields,
                                                                  double threshold_mult) {
     const TbcField& f = fields[blockIdx.x];
-    if (f.spline_k >= 2) return;  // wow_spline_kernel's field
+    if (f.spline_k >= 2) return;  // the spline kernels' field
     __shared__ double key[kWowThreads];
     __shared__ long long wt[kWowThreads];
     __shared__ long long csum[kWowThreads];
@@ -430,11 +430,11 @@ __device__ unsigned long long min_key_above(Visit visit, long long n, unsigned l
     return m;
 }
 
-// numpy median of key(i), i in [0, n): the middle value, or the mean of the
-// two middle values for even n.
+// Of key(i), i in [0, n): the value of rank r1, or with `two` the mean of that
+// and the next in order (numpy's median of the whole set when r1 is its
+// middle rank).
 template <class Visit>
-__device__ double select_median(Visit visit, long long n, unsigned* hist, SelectShared& sh) {
-    const long long r1 = (n & 1) ? n / 2 : n / 2 - 1;
+__device__ double select_mean(Visit visit, long long n, long long r1, bool two, unsigned* hist, SelectShared& sh) {
     radix_select(visit, n, r1, hist, sh);
     const unsigned long long k1 = sh.prefix;
     const long long upto = sh.below + sh.eq;  // keys <= k1
@@ -442,34 +442,132 @@ __device__ double select_median(Visit visit, long long n, unsigned* hist, Select
     const unsigned long long kn = sh.next;
     __syncthreads();
     const double v1 = key_value(k1);
-    if (n & 1) return v1;
+    if (!two) return v1;
     const double v2 = has_next ? key_value(kn) : (upto >= r1 + 2 ? v1 : key_value(min_key_above(visit, n, k1, sh)));
     return __dadd_rn(v1, v2) / 2;
 }
 
-// One CTA per spline field.  Thread 0 solves the tridiagonal system, the
-// pieces are built in parallel (shared table and the field's scratch copy),
-// then the median and MAD of the wow factors over the whole wow array [0,
-// nwow) are selected exactly, and with level smoothing the IIR runs as a
-// scan of affine maps over 1024 contiguous chunks (each chunk's map from one
-// pass, the chunks' start values by a block scan, then a second pass that
-// records the level just before every 32nd output pixel for the gather).
-__global__ void __launch_bounds__(kSplThreads) wow_spline_kernel(const TbcField* fields, double threshold_mult) {
+// The wow factors' median and MAD of a field, and with level smoothing the
+// IIR's state every 32 pixels, in kernels of one CTA per field that decide
+// and kernels of kSplSlices CTAs per field that walk its pixels:
+//   spline_build    the pieces; a bracket for the median from kSplSamples
+//                   pixels at even steps
+//   spline_pass     counts the wow factors below the bracket, keeps those in it
+//   spline_median   the median, exactly, from those (their number below tells
+//                   which rank to take); a bracket for the MAD
+//   spline_pass     the same for |wow - median|
+//   spline_mad      the MAD
+//   spline_maps / spline_levels   (smoothing) the IIR over each 32 pixels as
+//                   a map y -> b^32 y + B, then the maps' scan
+// A bracket's ranks lie kSplMargin samples either side of the median's: the
+// factors are smooth along a line, so an evenly stepped sample misjudges a
+// rank by about one sample per crossing and square root of the crossings, ~10
+// of 4096.  Where it fails all the same (or keeps too many), the CTA selects
+// from all pixels by radix passes.
+// Bound: instruction issue of the walks (FP64 pipe next).  As one CTA per
+// field walking all pixels up to ten times: 672 us for 60 NTSC fields (cubic,
+// smoothing; as long for one); the seven launches together 215 us (ncu: build
+// 67, passes 34 and 33, median 31, MAD 12, maps 24, levels 14; the build is one
+// thread's chain of divisions and two rank selections).
+constexpr int kSplSlices = 16;
+constexpr int kSplPassThreads = 256;
+constexpr int kSplSamples = 4096;
+constexpr int kSplMargin = 48;
+static_assert(sizeof(SplCtl) <= kSplCtlDoubles * sizeof(double), "the control block's place");
+
+// Ranks of the median: r1, and r1 + 1 when the count is even.
+__device__ __forceinline__ long long median_rank(long long n) { return (n & 1) ? n / 2 : n / 2 - 1; }
+
+// The bracket [lo, hi] for the median of value(i), i in [0, L).
+template <class Value>
+__device__ void find_bracket(Value value, long long L, double* samp, unsigned* hist, SelectShared& sh, SplCtl* ctl) {
+    const int t = threadIdx.x;
+    double lo = -INFINITY, hi = INFINITY;
+    if (L > kSplKeep) {
+        for (int s = t; s < kSplSamples; s += kSplThreads)
+            samp[s] = value((long long)(((double)s + 0.5) * ((double)L / kSplSamples)));
+        __syncthreads();
+        auto visit = [&](long long a0, long long a1, auto body) {
+            for (long long i = a0; i < a1; ++i) body(i, order_key(samp[i]));
+        };
+        const double at = (double)median_rank(L) * ((double)kSplSamples / (double)L);
+        const long long rl = (long long)at - kSplMargin, rh = (long long)at + 1 + kSplMargin;
+        if (rl >= 0) {
+            radix_select(visit, kSplSamples, rl, hist, sh);
+            lo = key_value(sh.prefix);
+            __syncthreads();
+        }
+        if (rh < kSplSamples) {
+            radix_select(visit, kSplSamples, rh, hist, sh);
+            hi = key_value(sh.prefix);
+            __syncthreads();
+        }
+    }
+    if (t == 0) {
+        ctl->lo = lo;
+        ctl->hi = hi;
+        ctl->below = 0;
+        ctl->kept = 0;
+    }
+}
+
+// The median of all L values from what the pass kept, or (kept too few or too
+// many) from all of them, all(i0, i1, body) visiting them in order.
+template <class All>
+__device__ double bracket_median(const TbcField& f, All all, long long L, unsigned* hist, SelectShared& sh) {
+    const SplCtl* ctl = spline_ctl(f);
+    const long long r1 = median_rank(L), r2 = L / 2;
+    const long long below = ctl->below, kept = ctl->kept;
+    const bool usable = ctl->lo <= ctl->hi && kept <= kSplKeep && r1 >= below && r2 < below + kept;
+    __syncthreads();
+    if (usable) {
+        const double* v = spline_kept(f);
+        return select_mean(
+            [&](long long a0, long long a1, auto body) {
+                for (long long i = a0; i < a1; ++i) body(i, order_key(v[i]));
+            },
+            kept, r1 - below, !(L & 1), hist, sh);
+    }
+    return select_mean(all, L, r1, !(L & 1), hist, sh);
+}
+
+__device__ __forceinline__ WowWalk field_walk(const TbcField& f) {
+    return WowWalk{f.spl, f.npieces, f.outscale, f.inv_inl, f.spline_k == 3 ? 0.0 : 0.5};
+}
+
+__device__ __forceinline__ double wow_at(const TbcField& f, long long i) {
+    double c, w;
+    spline_eval(f.spl, f.npieces, __dmul_rn((double)i, f.outscale), f.inv_inl, f.spline_k == 3 ? 0.0 : 0.5, c, w);
+    return w;
+}
+
+// The tridiagonal system's rows in parallel, solved by thread 0 (Thomas), the
+// pieces in parallel.
+__global__ void __launch_bounds__(kSplThreads) spline_build_kernel(const TbcField* fields) {
     const TbcField& f = fields[blockIdx.x];
     if (f.spline_k < 2) return;
-    __shared__ double pc[kSplStride * kSplMaxLines];
-    __shared__ double cp[kSplMaxLines], dp[kSplMaxLines];
+    __shared__ double mem[kSplSamples];  // the rows while solving, then the samples
     __shared__ unsigned long long hist_mem[kHistBins / 2];  // 8-byte aligned: also the collected keys
-    unsigned* hist = reinterpret_cast<unsigned*>(hist_mem);
     __shared__ SelectShared sh;
-    __shared__ double wmapA[32], wmapB[32], wy[32];
-    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    double* ra = mem;
+    double* rb = ra + kSplMaxLines;
+    double* rc = rb + kSplMaxLines;
+    double* rd = rc + kSplMaxLines;
+    double* cp = rd + kSplMaxLines;
+    double* dp = cp + kSplMaxLines;
+    static_assert(6 * kSplMaxLines <= kSplSamples, "the rows' place");
+    const int t = threadIdx.x;
     const int n = f.nlines;
     const bool cubic = f.spline_k == 3;
+    SplCtl* ctl = spline_ctl(f);
     if (n < 4 || n > kSplMaxLines) {
-        if (t == 0) f.status[0] = LDG_TBC_BAD_LINES;
+        if (t == 0) {
+            f.status[0] = LDG_TBC_BAD_LINES;
+            ctl->bad = 1;
+        }
         return;
     }
+    if (t == 0) ctl->bad = 0;
     const double inl = f.inlinelen;
     const double* y = f.linelocs;
     auto X = [&](int i) { return (double)i * inl; };
@@ -477,44 +575,52 @@ __global__ void __launch_bounds__(kSplThreads) wow_spline_kernel(const TbcField*
     auto BK = [&](int j) {
         return j == 0 ? X(0) : (j == n - 2 ? X(n - 1) : __dmul_rn(__dadd_rn(X(j), X(j + 1)), 0.5));
     };
-    if (t == 0) {
-        const int m = n - 2 + (cubic ? 0 : 1);  // unknowns
-        for (int r = 0; r < m; ++r) {
-            double a = 0, b = 0, c = 0, d = 0;
-            if (cubic) {
-                const int i = r + 1;
-                const double h0 = X(i) - X(i - 1), h1 = X(i + 1) - X(i);
-                a = h0;
-                b = 2.0 * (h0 + h1);
-                c = h1;
-                d = 6.0 * ((y[i + 1] - y[i]) / h1 - (y[i] - y[i - 1]) / h0);
-            } else {
-                // integral of s' over [x_r, x_{r+1}], split at breakpoint r when it lies inside
-                auto add = [&](double p, double q, int j, double& cj, double& cj1) {
-                    const double b0 = BK(j), wj = BK(j + 1) - b0;
-                    const double rp = (p - b0) / wj, rq = (q - b0) / wj;
-                    const double hw = (q - p) / 2;
-                    cj += hw * ((1.0 - rp) + (1.0 - rq));
-                    cj1 += hw * (rp + rq);
-                };
-                if (r == 0) {
-                    add(X(0), X(1), 0, b, c);
-                } else if (r == n - 2) {
-                    add(X(n - 2), X(n - 1), n - 3, a, b);
-                } else {
-                    add(X(r), BK(r), r - 1, a, b);
-                    add(BK(r), X(r + 1), r, b, c);
-                }
-                d = y[r + 1] - y[r];
-            }
+    const int m = n - 2 + (cubic ? 0 : 1);  // unknowns
+    for (int r = t; r < m; r += kSplThreads) {
+        double a = 0, b = 0, c = 0, d = 0;
+        if (cubic) {
+            const int i = r + 1;
+            const double h0 = X(i) - X(i - 1), h1 = X(i + 1) - X(i);
+            a = h0;
+            b = 2.0 * (h0 + h1);
+            c = h1;
+            d = 6.0 * ((y[i + 1] - y[i]) / h1 - (y[i] - y[i - 1]) / h0);
+        } else {
+            // integral of s' over [x_r, x_{r+1}], split at breakpoint r when it lies inside
+            auto add = [&](double p, double q, int j, double& cj, double& cj1) {
+                const double b0 = BK(j), wj = BK(j + 1) - b0;
+                const double rp = (p - b0) / wj, rq = (q - b0) / wj;
+                const double hw = (q - p) / 2;
+                cj += hw * ((1.0 - rp) + (1.0 - rq));
+                cj1 += hw * (rp + rq);
+            };
             if (r == 0) {
-                cp[0] = c / b;
-                dp[0] = d / b;
+                add(X(0), X(1), 0, b, c);
+            } else if (r == n - 2) {
+                add(X(n - 2), X(n - 1), n - 3, a, b);
             } else {
-                const double den = b - a * cp[r - 1];
-                cp[r] = c / den;
-                dp[r] = (d - a * dp[r - 1]) / den;
+                add(X(r), BK(r), r - 1, a, b);
+                add(BK(r), X(r + 1), r, b, c);
             }
+            d = y[r + 1] - y[r];
+        }
+        ra[r] = a;
+        rb[r] = b;
+        rc[r] = c;
+        rd[r] = d;
+    }
+    __syncthreads();
+    if (t == 0) {
+        double cq = rc[0] / rb[0], dq = rd[0] / rb[0];
+        cp[0] = cq;
+        dp[0] = dq;
+        for (int r = 1; r < m; ++r) {
+            const double a = ra[r];
+            const double den = rb[r] - a * cq;
+            cq = rc[r] / den;
+            dq = (rd[r] - a * dq) / den;
+            cp[r] = cq;
+            dp[r] = dq;
         }
         for (int r = m - 2; r >= 0; --r) dp[r] = dp[r] - cp[r] * dp[r + 1];
     }
@@ -544,49 +650,134 @@ __global__ void __launch_bounds__(kSplThreads) wow_spline_kernel(const TbcField*
             e[5] = 0.0;
         }
 #pragma unroll
-        for (int q = 0; q < kSplStride; ++q) {
-            pc[p * kSplStride + q] = e[q];
-            f.spl[p * kSplStride + q] = e[q];
-        }
+        for (int q = 0; q < kSplStride; ++q) f.spl[p * kSplStride + q] = e[q];
     }
     __syncthreads();
+    find_bracket([&](long long i) { return wow_at(f, i); }, f.nwow, mem, reinterpret_cast<unsigned*>(hist_mem), sh, ctl);
+}
+
+// One slice of a field's pixels against the bracket: how many lie below it,
+// and the values inside it (in no order).
+template <bool Mad>
+__global__ void __launch_bounds__(kSplPassThreads) spline_pass_kernel(const TbcField* fields) {
+    const TbcField& f = fields[blockIdx.y];
+    if (f.spline_k < 2) return;
+    SplCtl* ctl = spline_ctl(f);
+    if (ctl->bad) return;
+    constexpr int kHold = 2048;
+    __shared__ double held[kHold];
+    __shared__ int s_n, s_at;
+    const int t = threadIdx.x;
+    if (t == 0) s_n = 0;
+    __syncthreads();
+    const double lo = ctl->lo, hi = ctl->hi, med = Mad ? f.stat[0] : 0.0;
+    double* kept = spline_kept(f);
     const long long L = f.nwow;
-    const double shift = cubic ? 0.0 : 0.5;
-    const double outscale = f.outscale, inv_inl = f.inv_inl;
-    const WowWalk walk{pc, np, outscale, inv_inl, shift};
-    const double med = select_median(
+    const long long per = (L + kSplSlices * kSplPassThreads - 1) / (kSplSlices * kSplPassThreads);
+    const long long i0 = ((long long)blockIdx.x * kSplPassThreads + t) * per, i1 = min(L, i0 + per);
+    int below = 0;
+    field_walk(f)(i0, i1, [&](long long, double w) {
+        const double v = Mad ? fabs(__dadd_rn(w, -med)) : w;
+        below += v < lo;
+        if (v >= lo && v <= hi) {
+            const int at = atomicAdd(&s_n, 1);
+            if (at < kHold) {
+                held[at] = v;
+            } else {
+                const int g = atomicAdd(&ctl->kept, 1);
+                if (g < kSplKeep) kept[g] = v;
+            }
+        }
+    });
+#pragma unroll
+    for (int o = 16; o; o >>= 1) below += __shfl_xor_sync(0xffffffffu, below, o);
+    if ((t & 31) == 0 && below) atomicAdd(&ctl->below, below);
+    __syncthreads();
+    const int n = min(s_n, kHold);
+    if (t == 0) s_at = n ? atomicAdd(&ctl->kept, n) : 0;
+    __syncthreads();
+    for (int i = t; i < n; i += kSplPassThreads)
+        if (s_at + i < kSplKeep) kept[s_at + i] = held[i];
+}
+
+__global__ void __launch_bounds__(kSplThreads) spline_median_kernel(const TbcField* fields) {
+    const TbcField& f = fields[blockIdx.x];
+    if (f.spline_k < 2 || spline_ctl(f)->bad) return;
+    __shared__ double samp[kSplSamples];
+    __shared__ unsigned long long hist_mem[kHistBins / 2];
+    __shared__ SelectShared sh;
+    unsigned* hist = reinterpret_cast<unsigned*>(hist_mem);
+    const WowWalk walk = field_walk(f);
+    const double med = bracket_median(
+        f,
         [&](long long a0, long long a1, auto body) {
             walk(a0, a1, [&](long long i, double w) { body(i, order_key(w)); });
         },
-        L, hist, sh);
-    const double mad = select_median(
+        f.nwow, hist, sh);
+    if (threadIdx.x == 0) f.stat[0] = med;
+    __syncthreads();
+    find_bracket([&](long long i) { return fabs(__dadd_rn(wow_at(f, i), -med)); }, f.nwow, samp, hist, sh,
+                 spline_ctl(f));
+}
+
+__global__ void __launch_bounds__(kSplThreads) spline_mad_kernel(const TbcField* fields, double threshold_mult) {
+    const TbcField& f = fields[blockIdx.x];
+    if (f.spline_k < 2 || spline_ctl(f)->bad) return;
+    __shared__ unsigned long long hist_mem[kHistBins / 2];
+    __shared__ SelectShared sh;
+    const WowWalk walk = field_walk(f);
+    const double med = f.stat[0];
+    const double mad = bracket_median(
+        f,
         [&](long long a0, long long a1, auto body) {
             walk(a0, a1, [&](long long i, double w) { body(i, order_key(fabs(__dadd_rn(w, -med)))); });
         },
-        L, hist, sh);
-    const double thr = mad > 0 ? threshold_mult * mad : 0.001;
-    if (t == 0) {
-        f.stat[0] = med;
-        f.stat[1] = thr;
+        f.nwow, reinterpret_cast<unsigned*>(hist_mem), sh);
+    if (threadIdx.x == 0) f.stat[1] = mad > 0 ? threshold_mult * mad : 0.001;
+}
+
+// Level-adjust IIR (utils.py:141-149), y[0] = la[0], y[i] = a la[i] + b y[i-1],
+// in groups of 32 pixels that end where the gather's warps begin (group 0 the
+// pixels before the first such place): the map of group g is y -> b^32 y + B.
+__device__ __forceinline__ long long level_group_end(const TbcField& f, long long g) {
+    return (long long)f.outwidth * (f.lineoffset + 1) % 32 + 32 * g;
+}
+
+__global__ void __launch_bounds__(kSplPassThreads) spline_maps_kernel(const TbcField* fields) {
+    const TbcField& f = fields[blockIdx.y];
+    if (f.spline_k < 2 || !(f.smooth_b > 0) || spline_ctl(f)->bad) return;
+    const double a = f.smooth_a, b = f.smooth_b, med = f.stat[0], thr = f.stat[1];
+    const long long ngroups = spline_level_groups(f);
+    for (long long g = (long long)blockIdx.x * kSplPassThreads + threadIdx.x; g < ngroups;
+         g += (long long)gridDim.x * kSplPassThreads) {
+        double B = 0.0;
+        field_walk(f)(g ? level_group_end(f, g - 1) : 0, min(level_group_end(f, g), f.nwow), [&](long long i, double wv) {
+            const double la = fabs(__dadd_rn(wv, -med)) > thr ? med : wv;
+            B = i == 0 ? la : __dadd_rn(__dmul_rn(a, la), __dmul_rn(b, B));
+        });
+        spline_maps(f)[g] = B;
     }
-    if (!(f.smooth_b > 0)) return;
-    auto level = [&](double wv) { return fabs(__dadd_rn(wv, -med)) > thr ? med : wv; };
-    // level-adjust IIR (utils.py:141-149): y[0] = la[0], y[i] = a la[i] + b y[i-1]
-    const double a = f.smooth_a, b = f.smooth_b;
-    const long long C = (L + kSplThreads - 1) / kSplThreads;
-    const long long i0 = (long long)t * C, i1 = min(L, i0 + C);
-    double A = 1.0, B = 0.0;  // this chunk as y_out = A y_in + B
-    walk(i0, i1, [&](long long i, double wv) {
-        const double la = level(wv);
-        if (i == 0) {
-            A = 0.0;
-            B = la;
-        } else {
-            A = __dmul_rn(b, A);
-            B = __dadd_rn(__dmul_rn(a, la), __dmul_rn(b, B));
-        }
-    });
-    // inclusive scan of the maps over the warp, then over the warps
+}
+
+__global__ void __launch_bounds__(kSplThreads) spline_levels_kernel(const TbcField* fields) {
+    const TbcField& f = fields[blockIdx.x];
+    if (f.spline_k < 2 || !(f.smooth_b > 0) || spline_ctl(f)->bad) return;
+    __shared__ double wA[32], wB[32], wy[32];
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const long long n = spline_level_groups(f);
+    const double* maps = spline_maps(f);
+    double b32 = 1.0;
+    for (int k = 0; k < 32; ++k) b32 = __dmul_rn(f.smooth_b, b32);
+    // the first pixel's group starts the recurrence: its map is a constant
+    const long long head = level_group_end(f, 0) > 0 ? 0 : 1;
+    const long long per = (n + kSplThreads - 1) / kSplThreads;
+    const long long g0 = min(n, t * per), g1 = min(n, g0 + per);
+    double A = 1.0, B = 0.0;
+    for (long long g = g0; g < g1; ++g) {
+        const double m = g <= head ? 0.0 : b32;
+        B = g < head ? B : __fma_rn(m, B, maps[g]);
+        A = g < head ? A : __dmul_rn(A, m);
+    }
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const double Ap = __shfl_up_sync(0xffffffffu, A, o), Bp = __shfl_up_sync(0xffffffffu, B, o);
@@ -596,34 +787,28 @@ __global__ void __launch_bounds__(kSplThreads) wow_spline_kernel(const TbcField*
         }
     }
     if (lane == 31) {
-        wmapA[w] = A;
-        wmapB[w] = B;
+        wA[w] = A;
+        wB[w] = B;
     }
     __syncthreads();
     if (t == 0) {
         double yy = 0.0;
         for (int q = 0; q < 32; ++q) {
             wy[q] = yy;
-            yy = __fma_rn(wmapA[q], yy, wmapB[q]);
+            yy = __fma_rn(wA[q], yy, wB[q]);
         }
     }
     __syncthreads();
     const double Ae = __shfl_up_sync(0xffffffffu, A, 1), Be = __shfl_up_sync(0xffffffffu, B, 1);
-    double yv = lane == 0 ? wy[w] : __fma_rn(Ae, wy[w], Be);
-    // second pass: record y just before output pixel 32*m (wow index igbase + 32*m)
-    const long long igbase = (long long)f.outwidth * (f.lineoffset + 1);
-    const long long nout = (long long)f.linesout * f.outwidth;
-    const long long nyb = (nout + 31) / 32;
-    long long mq = (i0 + 1 - igbase + 31) / 32;
-    if (i0 + 1 - igbase <= 0) mq = 0;
-    walk(i0, i1, [&](long long i, double wv) {
-        const double la = level(wv);
-        yv = i == 0 ? la : __dadd_rn(__dmul_rn(a, la), __dmul_rn(b, yv));
-        if (mq < nyb && i + 1 == igbase + 32 * mq) {
-            f.ybefore[mq] = yv;
-            ++mq;
-        }
-    });
+    double y = lane == 0 ? wy[w] : __fma_rn(Ae, wy[w], Be);
+    // the level just before output pixel 32 mq: after the group that ends there
+    const long long first = (long long)f.outwidth * (f.lineoffset + 1) / 32;  // group that ends at output pixel 0
+    const long long nyb = ((long long)f.linesout * f.outwidth + 31) / 32;
+    for (long long g = g0; g < g1; ++g) {
+        if (g >= head) y = __fma_rn(g <= head ? 0.0 : b32, y, maps[g]);
+        const long long mq = g - first;
+        if (mq >= 0 && mq < nyb) f.ybefore[mq] = y;
+    }
 }
 
 constexpr int kGatherThreads = 256;
@@ -802,13 +987,29 @@ __global__ void __launch_bounds__(kGatherThreads, 8) tbc_gather_kernel(const Tbc
 }
 
 cudaError_t launch_tbc(const TbcField* dfields, int nfields, long long max_nout, const float* lut,
-                       double threshold_mult, bool any_spline, cudaStream_t stream) {
+                       double threshold_mult, bool any_spline, bool any_smooth, cudaStream_t stream) {
     if (nfields <= 0) return cudaSuccess;
     wow_levels_kernel<<<nfields, kWowThreads, 0, stream>>>(dfields, threshold_mult);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     if (any_spline) {
-        wow_spline_kernel<<<nfields, kSplThreads, 0, stream>>>(dfields, threshold_mult);
+        spline_build_kernel<<<nfields, kSplThreads, 0, stream>>>(dfields);
+        for (int pass = 0; pass < 2; ++pass) {
+            for (int off = 0; off < nfields; off += 65535) {  // grid.y limit
+                const unsigned n = (unsigned)(nfields - off < 65535 ? nfields - off : 65535);
+                if (pass) spline_pass_kernel<true><<<dim3(kSplSlices, n), kSplPassThreads, 0, stream>>>(dfields + off);
+                else spline_pass_kernel<false><<<dim3(kSplSlices, n), kSplPassThreads, 0, stream>>>(dfields + off);
+            }
+            if (pass) spline_mad_kernel<<<nfields, kSplThreads, 0, stream>>>(dfields, threshold_mult);
+            else spline_median_kernel<<<nfields, kSplThreads, 0, stream>>>(dfields);
+        }
+        if (any_smooth) {
+            for (int off = 0; off < nfields; off += 65535) {
+                const unsigned n = (unsigned)(nfields - off < 65535 ? nfields - off : 65535);
+                spline_maps_kernel<<<dim3(2 * kSplSlices, n), kSplPassThreads, 0, stream>>>(dfields + off);
+            }
+            spline_levels_kernel<<<nfields, kSplThreads, 0, stream>>>(dfields);
+        }
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }

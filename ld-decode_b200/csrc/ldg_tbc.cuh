@@ -40,12 +40,46 @@ struct TbcField {
 };
 
 constexpr int kSplStride = 6;
+
+// Scratch of a spline field at TbcField.stat: median and outlier threshold,
+// the control block of the statistics, the values kept in a bracket, and with
+// smoothing the level before every 32nd output pixel and the IIR's maps.
+struct SplCtl {
+    double lo, hi;   // bracket
+    int below, kept; // values below it, inside it
+    int bad;
+};
+constexpr int kSplCtlDoubles = 4;
+constexpr int kSplKeep = 12288;  // values of a bracket kept (4.2 % of a PAL field's)
+
+// IIR groups: the pixels before the first 32-pixel place of the output, then 32 each.
+__host__ __device__ inline long long spline_level_groups(int outwidth, int lineoffset, int linesout) {
+    const long long head = (long long)outwidth * (lineoffset + 1);
+    return head / 32 + ((long long)linesout * outwidth + 31) / 32 + 1;
+}
+
+// Doubles of scratch a spline field needs.
+inline size_t spline_scratch_doubles(int nlines, int outwidth, int lineoffset, int linesout, bool smooth) {
+    size_t n = (size_t)kSplStride * nlines + 2 + kSplCtlDoubles + kSplKeep;
+    if (smooth)
+        n += ((size_t)linesout * outwidth + 31) / 32 + (size_t)spline_level_groups(outwidth, lineoffset, linesout);
+    return n;
+}
+
+__device__ __forceinline__ SplCtl* spline_ctl(const TbcField& f) { return reinterpret_cast<SplCtl*>(f.stat + 2); }
+__device__ __forceinline__ double* spline_kept(const TbcField& f) { return f.stat + 2 + kSplCtlDoubles; }
+__device__ __forceinline__ long long spline_level_groups(const TbcField& f) {
+    return spline_level_groups(f.outwidth, f.lineoffset, f.linesout);
+}
+__device__ __forceinline__ double* spline_maps(const TbcField& f) {
+    return f.ybefore + ((size_t)f.linesout * f.outwidth + 31) / 32;
+}
 constexpr int kLutPhases = 65536;  // sinc table phases (rows 0..65536, the last a copy)
 
 // lut: the sinc table interleaved for the gather (kLutPhases x 8 float4:
 // two taps of phase p and their differences to phase p + 1).
 cudaError_t launch_tbc(const TbcField* dfields, int nfields, long long max_nout, const float* lut,
-                       double threshold_mult, bool any_spline, cudaStream_t stream);
+                       double threshold_mult, bool any_spline, bool any_smooth, cudaStream_t stream);
 
 struct RfTbcField {
     const int16_t* in;   // raw samples of the field read (field-local sample 0)

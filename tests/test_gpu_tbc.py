@@ -305,3 +305,48 @@ def test_tbc_argument_checks(cuda_ok):
             desc(ll, wow_interpolation_method="spline")
     finally:
         rf.close()
+
+
+@pytest.mark.parametrize("method", ["quadratic", "cubic"])
+@pytest.mark.parametrize("shape", ["constant", "jitter", "two-level", "half and half"])
+@pytest.mark.parametrize("outl", [5, 40])
+@pytest.mark.parametrize("smoothing", [0.0, 2.0])
+def test_spline_statistics_extremes(cuda_ok, method, shape, outl, smoothing):
+    """Wow factors whose median's bracket keeps everything (few pixels), too
+    much (all factors alike) or little, odd and even pixel counts, and a
+    median between two plateaus, with displaced lines for the outlier rule:
+    the resampled field against the oracle's.  A wrong median or MAD moves
+    whole lines by 100 Hz and more; the coordinates' 3e-6 samples and the
+    float32 sums stay below 2 Hz on this signal."""
+    import torch
+    from ldgpu import RFDecode
+    from ldgpu.field import tbc_descriptor, tbc_fields
+    rf = RFDecode(system="NTSC")
+    outw, nlines, n = 911 if outl == 5 else 910, outl + 10, 60_000 if outl == 5 else 140_000
+    rng = np.random.default_rng(outl)
+    step = np.full(nlines, float(rf.linelen))
+    if shape == "jitter":
+        step += rng.normal(size=nlines) * 0.05
+    elif shape == "two-level":
+        step[::2] += 1.0
+    elif shape == "half and half":
+        step[nlines // 2:] += 0.7
+    ll = 300.0 + np.cumsum(step) - step[0]
+    ll[outl // 2] += 4.0
+    x = np.arange(n)
+    buf = (8.0e6 + 1.0e5 * np.sin(x * 0.01)).astype(np.float32)
+    levels = (rf.DecoderParams["ire0"], rf.DecoderParams["hz_ire"], rf.DecoderParams["vsync_ire"], 300.0, 1024.0)
+    for lineoffset in (0, 1):
+        out = torch.zeros(outl * outw, dtype=torch.float32, device="cuda")
+        dbuf, dll = torch.from_numpy(buf).cuda(), torch.from_numpy(ll).cuda()
+        d = tbc_descriptor(rf, dbuf.data_ptr(), dll.data_ptr(), lineoffset, outw, outl, outl, levels,
+                           out_f32=out.data_ptr(), buf_len=n, nlines=nlines, wow_smoothing=smoothing,
+                           wow_interpolation_method=method)
+        d.outlinelen = float(outw)
+        torch.cuda.synchronize()
+        tbc_fields(rf, [d])
+        coords, wow = otbc.pixel_coords(ll, rf.linelen, outw, outl, lineoffset, method=method)
+        want = otbc.scale_field(buf, coords, wow, rf.downscale_sinc_lut, lineoffset, outw, outl * outw,
+                                smoothing=smoothing)
+        assert np.abs(out.cpu().numpy().astype(np.float64) - want).max() < 2.0, lineoffset
+    rf.close()
