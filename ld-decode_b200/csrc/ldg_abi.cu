@@ -724,7 +724,7 @@ int ldg_tbc_fields(ldg_ctx* c, const ldg_tbc_field* fields, int32_t nfields, voi
         }
     }
     LDG_CK(cudaMemcpyAsync(c->d_fields, h.data(), nfields * sizeof(ldg::TbcField), cudaMemcpyHostToDevice, st));
-    cudaError_t e = ldg::launch_tbc(c->d_fields, nfields, max_nout, c->d_lut, 15.0, any_spline, any_smooth, st);
+    cudaError_t e = ldg::launch_tbc(c->d_fields, h.data(), nfields, max_nout, c->d_lut, 15.0, any_spline, any_smooth, st);
     if (e != cudaSuccess) return fail(LDG_ERR_CUDA, std::string("tbc launch: ") + cudaGetErrorString(e));
     if (any_host) {
         for (int i = 0; i < nfields; ++i) {
@@ -810,7 +810,7 @@ int ldg_tbc_fields_async(ldg_ctx* c, const ldg_tbc_field* fields, int32_t nfield
     } else {
         LDG_CK(cudaMemcpyAsync(w.d_fields, w.h_fields, nfields * sizeof(ldg::TbcField), cudaMemcpyHostToDevice, st));
     }
-    cudaError_t e = ldg::launch_tbc(w.d_fields, nfields, max_nout, c->d_lut, 15.0, any_spline, any_smooth, st);
+    cudaError_t e = ldg::launch_tbc(w.d_fields, w.h_fields, nfields, max_nout, c->d_lut, 15.0, any_spline, any_smooth, st);
     if (e != cudaSuccess) return fail(LDG_ERR_CUDA, std::string("tbc launch: ") + cudaGetErrorString(e));
     LDG_CK(cudaEventRecord(w.done, st));
     w.used = true;

@@ -813,12 +813,41 @@ __global__ void __launch_bounds__(kSplThreads) spline_levels_kernel(const TbcFie
 
 constexpr int kGatherThreads = 256;
 
+// What the gather reads of a field, in the launch's parameters: from the
+// constant bank a warp gets a value without the load pipe, which bounds the
+// kernel (read from the descriptors in memory they were some 20 of its ~145
+// wavefronts per warp: 50 PAL fields 352 us, so 311 us, 60 NTSC ones 334 and
+// 299 us; ncu).
+struct GatherField {
+    const float* buf;
+    const double* linelocs;
+    const double* seg_level;
+    const double* seg_start;
+    const long long* seg_lo;
+    int* status;
+    float* out_f32;
+    uint16_t* out_u16;
+    const double* spl;
+    const double* stat;
+    const double* ybefore;
+    double inlinelen, outscale, inv_inl, u16_scale, u16_offset, smooth_a, smooth_b;
+    long long buf_len, igbase, nout;
+    int nseg, npieces, spline_k, coord_f32;
+};
+
+template <int N>
+struct GatherBatch {
+    GatherField f[N];
+};
+constexpr int kGatherBatch = 160;  // fields of a launch (29 KB of parameters of at most 32)
+static_assert(sizeof(GatherBatch<kGatherBatch>) <= 32000, "kernel parameters");
+
 // Input coordinate (FP64) of output pixel ig, optionally rounded to float32
 // as the reference does; the spline segment j is also returned.  The
 // segment is found from x * (1/inlinelen) and then fixed by exact
 // comparisons with the integer knots; w = 1/(x1 - x0) = 1/inlinelen is
 // precomputed with the same rounding.
-__device__ __forceinline__ double pixel_coord(const TbcField& f, long long ig, int nseg, int& j) {
+__device__ __forceinline__ double pixel_coord(const GatherField& f, long long ig, int nseg, int& j) {
     const double inl = f.inlinelen;
     const double x = __dmul_rn((double)ig, f.outscale);
     j = (int)(x * f.inv_inl);
@@ -891,18 +920,17 @@ __device__ __noinline__ double gather_unpacked(const float* buf, const float* lu
     });
 }
 
-__global__ void __launch_bounds__(kGatherThreads, 8) tbc_gather_kernel(const TbcField* fields, const float* lut,
-                                                                    int nfields) {
-    const int fi = blockIdx.y;
-    if (fi >= nfields) return;
-    const TbcField& f = fields[fi];
-    const long long nout = (long long)f.linesout * f.outwidth;
+template <int N>
+__global__ void __launch_bounds__(kGatherThreads, 8) tbc_gather_kernel(const __grid_constant__ GatherBatch<N> batch,
+                                                                    const float* lut) {
+    const GatherField& f = batch.f[blockIdx.y];
+    const long long nout = f.nout;
     const long long wbase = (long long)blockIdx.x * kGatherThreads + (threadIdx.x & ~31);
     if (wbase >= nout) return;  // whole warps leave together
     const int lane = threadIdx.x & 31, grp = lane >> 3, k = lane & 7;
     const long long i = wbase + lane;
-    const int nseg = f.nlines - 1;
-    const long long igbase = (long long)f.outwidth * (f.lineoffset + 1);
+    const int nseg = f.nseg;
+    const long long igbase = f.igbase;
     int jj = 0;
     double cc, wv = 0.0;
     if (f.spline_k >= 2) {
@@ -986,8 +1014,24 @@ __global__ void __launch_bounds__(kGatherThreads, 8) tbc_gather_kernel(const Tbc
     }
 }
 
-cudaError_t launch_tbc(const TbcField* dfields, int nfields, long long max_nout, const float* lut,
-                       double threshold_mult, bool any_spline, bool any_smooth, cudaStream_t stream) {
+template <int N>
+static cudaError_t launch_gather(const TbcField* fields, int n, long long max_nout, const float* lut,
+                                 cudaStream_t stream) {
+    GatherBatch<N> batch;
+    for (int i = 0; i < n; ++i) {
+        const TbcField& f = fields[i];
+        batch.f[i] = {f.buf, f.linelocs, f.seg_level, f.seg_start, f.seg_lo, f.status, f.out_f32, f.out_u16, f.spl, f.stat,
+                      f.ybefore, f.inlinelen, f.outscale, f.inv_inl, f.u16_scale, f.u16_offset, f.smooth_a, f.smooth_b,
+                      f.buf_len, (long long)f.outwidth * (f.lineoffset + 1), (long long)f.linesout * f.outwidth,
+                      f.nlines - 1, f.npieces, f.spline_k, f.coord_f32};
+    }
+    const unsigned gx = (unsigned)((max_nout + kGatherThreads - 1) / kGatherThreads);
+    tbc_gather_kernel<N><<<dim3(gx, (unsigned)n), kGatherThreads, 0, stream>>>(batch, lut);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_tbc(const TbcField* dfields, const TbcField* hfields, int nfields, long long max_nout,
+                       const float* lut, double threshold_mult, bool any_spline, bool any_smooth, cudaStream_t stream) {
     if (nfields <= 0) return cudaSuccess;
     wow_levels_kernel<<<nfields, kWowThreads, 0, stream>>>(dfields, threshold_mult);
     cudaError_t e = cudaGetLastError();
@@ -1013,15 +1057,14 @@ cudaError_t launch_tbc(const TbcField* dfields, int nfields, long long max_nout,
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
-    const long long per_cta = kGatherThreads;
-    const unsigned gx = (unsigned)((max_nout + per_cta - 1) / per_cta);
-    for (int off = 0; off < nfields; off += 65535) {  // grid.y limit
-        const int n = nfields - off < 65535 ? nfields - off : 65535;
-        tbc_gather_kernel<<<dim3(gx, (unsigned)n), kGatherThreads, 0, stream>>>(dfields + off, lut, n);
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
+    for (int off = 0; off < nfields && e == cudaSuccess; off += kGatherBatch) {
+        const int n = nfields - off < kGatherBatch ? nfields - off : kGatherBatch;
+        // no more parameters than the batch needs
+        e = n <= 4 ? launch_gather<4>(hfields + off, n, max_nout, lut, stream)
+                   : n <= 32 ? launch_gather<32>(hfields + off, n, max_nout, lut, stream)
+                             : launch_gather<kGatherBatch>(hfields + off, n, max_nout, lut, stream);
     }
-    return cudaSuccess;
+    return e;
 }
 
 // RF TBC (Field.rf_tbc, lddecode/core.py:2724-2752): each output line l is
