@@ -99,6 +99,7 @@ struct ldg_ctx {
     double* d_ll = nullptr;
     size_t ll_cap = 0;
     int* d_status = nullptr;
+    int* h_status = nullptr;  // pinned
     void* d_lines = nullptr;  // sync-run scan scratch (ldg_sync_runs)
     int* d_slots = nullptr;   // demod scratch-slot locks (nslots) and the error word after them
     int nslots = 0;
@@ -342,6 +343,7 @@ void ldg_ctx_destroy(ldg_ctx* c) {
     if (c->drop_used) cudaEventSynchronize(c->drop_done);
     if (c->rftbc_used) cudaEventSynchronize(c->rftbc_done);
     if (c->h_word) cudaFreeHost(c->h_word);
+    if (c->h_status) cudaFreeHost(c->h_status);
     cudaFree(c->d_scan);
     if (c->a2_used) cudaEventSynchronize(c->a2_done);
     cudaFree(c->d_a2);
@@ -733,10 +735,13 @@ int ldg_tbc_fields(ldg_ctx* c, const ldg_tbc_field* fields, int32_t nfields, voi
             if (hs[i].u16) LDG_CK(cudaMemcpyAsync(fields[i].out_u16, h[i].out_u16, nout * 2, cudaMemcpyDeviceToHost, st));
         }
     }
-    // the host copies of h/lls must stay alive until the async copies are done
+    // the status word comes back behind the launch (a copy of its own after the
+    // wait took 8 us); the host copies of h/lls must stay alive until the
+    // async copies are done
+    if (!c->h_status) LDG_CK(cudaMallocHost(&c->h_status, sizeof(int)));
+    LDG_CK(cudaMemcpyAsync(c->h_status, c->d_status, sizeof(int), cudaMemcpyDeviceToHost, st));
     LDG_CK(cudaStreamSynchronize(st));
-    int status = 0;
-    LDG_CK(cudaMemcpy(&status, c->d_status, sizeof(int), cudaMemcpyDeviceToHost));
+    const int status = *c->h_status;
     if (status) {
         LDG_CK(cudaMemset(c->d_status, 0, sizeof(int)));
         if (status & ldg::LDG_TBC_BAD_LINES) return fail(LDG_ERR_ARG, "ldg_tbc_fields: too many lines for the wow statistics");

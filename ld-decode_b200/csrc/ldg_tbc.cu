@@ -811,7 +811,7 @@ __global__ void __launch_bounds__(kSplThreads) spline_levels_kernel(const TbcFie
     }
 }
 
-constexpr int kGatherThreads = 256;
+constexpr int kGatherThreads = 128;  // 16 CTAs per SM (256 and 8: 1 % slower, 512 and 4: 4 %)
 
 // What the gather reads of a field, in the launch's parameters: from the
 // constant bank a warp gets a value without the load pipe, which bounds the
@@ -871,12 +871,11 @@ __device__ __forceinline__ double pixel_coord(const GatherField& f, long long ig
 // span and its 128 bytes of LUT are each one contiguous access; the 8
 // partial sums meet in a transposing reduction (lane k of group g ends with
 // pixel 4k + g) and one shuffle takes each pixel's sum to its own lane.
-// One lane's share of a pixel: taps 2k and 2k+1 of the 16 starting at
-// buf[st], weights from LUT phase ps (the interleaved float4 of w and the
-// next-phase difference) at fraction alpha; float32 products, FP64 sum.
-__device__ __forceinline__ double two_taps(const float* buf, const float* lut, int st, int ps, float alpha, int k) {
-    const float4 q = __ldg(reinterpret_cast<const float4*>(lut + (size_t)ps * 32) + k);
-    const float* in = buf + st + 2 * k;
+// One lane's share of a pixel: taps in[0] and in[1], weights from the row
+// (the interleaved float4 of w and the next-phase difference of the pixel's LUT
+// phase) at fraction alpha; float32 products, FP64 sum.
+__device__ __forceinline__ double two_taps(const float* in, const float4* row, float alpha) {
+    const float4 q = __ldg(row);
     const float x0 = __ldg(in), x1 = __ldg(in + 1);
     const float w0 = fmaf(alpha, q.z, q.x), w1 = fmaf(alpha, q.w, q.y);
     return (double)(x0 * w0) + (double)(x1 * w1);
@@ -916,12 +915,12 @@ __device__ __noinline__ double gather_unpacked(const float* buf, const float* lu
         const int pst = __shfl_sync(0xffffffffu, sti, src);
         const int pps = __shfl_sync(0xffffffffu, psi, src);
         const float pal = __shfl_sync(0xffffffffu, alpha, src);
-        return pps >= 0 ? two_taps(buf, lut, pst, pps, pal, k) : 0.0;
+        return pps >= 0 ? two_taps(buf + pst + 2 * k, reinterpret_cast<const float4*>(lut) + (size_t)pps * 8 + k, pal) : 0.0;
     });
 }
 
 template <int N>
-__global__ void __launch_bounds__(kGatherThreads, 8) tbc_gather_kernel(const __grid_constant__ GatherBatch<N> batch,
+__global__ void __launch_bounds__(kGatherThreads, 16) tbc_gather_kernel(const __grid_constant__ GatherBatch<N> batch,
                                                                     const float* lut) {
     const GatherField& f = batch.f[blockIdx.y];
     const long long nout = f.nout;
@@ -951,31 +950,39 @@ __global__ void __launch_bounds__(kGatherThreads, 8) tbc_gather_kernel(const __g
     const int sti = ok ? (int)st : 0;
     const int psi = ok ? ps : -1;
     // The 32 pixels' first taps lie within a few hundred samples of each
-    // other: as offsets from the warp's lowest one they fit 16 bits, and
-    // each pixel's offset and phase travel in one shuffle instead of two
-    // (the shuffles share the load pipe's writeback with the tap loads).
-    // 0xffff as the offset marks a pixel left at 0.
+    // other: as offsets from the warp's lowest one they fit 16 bits, and each
+    // pixel's offset, phase and fraction travel through shared memory in one
+    // read (by shuffles, two per pixel: 312 against 298 us for 50 PAL fields;
+    // they share the load pipe's writeback with the tap loads).  A pixel left
+    // at 0 takes the lowest one's taps and is set to 0 after the sum (a test
+    // at every pixel, and full addresses formed there: 298 against 260 us).
     const int low = __reduce_min_sync(0xffffffffu, ok ? sti : INT_MAX);
-    const bool packed = __all_sync(0xffffffffu, !ok || sti - low < 0xffff);
-    const unsigned pk = ok ? ((unsigned)(sti - low) << 16) | (unsigned)ps : 0xffff0000u;
-    double held;  // after the group sum: the whole sum of pixel 4 k + grp
-    if (packed) {
+    const bool packed = __all_sync(0xffffffffu, !ok || sti - low <= 0xffff);
+    double held = 0.0;  // after the group sum: the whole sum of pixel 4 k + grp
+    if (low == INT_MAX) {
+        // no pixel of the warp has its taps inside the buffer
+    } else if (packed) {
+        __shared__ uint2 s_px[kGatherThreads];
+        uint2* px = s_px + (threadIdx.x & ~31);
+        px[lane] = make_uint2(ok ? ((unsigned)(sti - low) << 16) | (unsigned)ps : 0u, __float_as_uint(alpha));
+        __syncwarp();
+        const float* in = f.buf + low + 2 * k;
+        const float4* row = reinterpret_cast<const float4*>(lut) + k;
+        const uint2* mine = px + grp;
         held = group_sum(k, [&](int p) {
             // the group's p-th pixel: at each step the four groups take four
             // adjacent pixels, whose 16-tap windows overlap (fewer cache lines
             // per tap load)
-            const int src = 4 * p + grp;
-            const unsigned q = __shfl_sync(0xffffffffu, pk, src);
-            const float pal = __shfl_sync(0xffffffffu, alpha, src);
-            return (q >> 16) != 0xffffu ? two_taps(f.buf, lut, low + (int)(q >> 16), (int)(q & 0xffffu), pal, k)
-                                        : 0.0;
+            const uint2 v = mine[4 * p];
+            return two_taps(in + (v.x >> 16), row + (size_t)(v.x & 0xffffu) * 8, __uint_as_float(v.y));
         });
     } else {
         // first taps too far apart for 16-bit offsets (wild line locations): rare
         held = gather_unpacked(f.buf, lut, sti, psi, alpha, grp, k);
     }
     // pixel `lane` is at lane 8 (lane % 4) + lane / 4
-    const double mine = __shfl_sync(0xffffffffu, held, 8 * (lane & 3) + (lane >> 2));
+    double mine = __shfl_sync(0xffffffffu, held, 8 * (lane & 3) + (lane >> 2));
+    if (!ok) mine = 0.0;
     double level;
     if (f.spline_k >= 2) {
         const double med = f.stat[0];
