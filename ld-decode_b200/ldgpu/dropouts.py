@@ -105,9 +105,8 @@ def detect_host_field(rf, data, linelocs, lineoffset, linecount, isfirst, hsync_
     video recarray and rfhpf): uploads it and runs the kernel."""
     import torch
     dev = torch.device("cuda", torch.cuda.current_device())
-    v = data["video"]
-    t = {k: torch.from_numpy(np.ascontiguousarray(v[k], np.float32)).to(dev)
-         for k in ("demod", "demod_05", "demod_raw")}
+    from .lines import device_columns
+    t = device_columns(data["video"], ("demod", "demod_05", "demod_raw"), dev)
     t["rfhpf"] = torch.from_numpy(np.ascontiguousarray(data["rfhpf"], np.float32)).to(dev)
     ll = torch.from_numpy(np.ascontiguousarray(linelocs, np.float64)).to(dev)
     d = _field(t["demod"].data_ptr(), t["demod_05"].data_ptr(), t["demod_raw"].data_ptr(), t["rfhpf"].data_ptr(),

@@ -196,6 +196,31 @@ class FieldLogic:
         _length = self.usectoinpx(_length)
         return slice(int(_begin + begin_offset), int(_begin + _length + begin_offset + 1))
 
+    def line_areas(self, lines, begin, length):
+        """The demodulated video of lineslice(l, begin, length) for each l of
+        `lines`: (areas, rest), areas a list of (positions in `lines`, samples
+        as one float32 row per line) by slice length, rest the positions whose
+        slice does not lie inside the read (its bounds then follow Python's
+        slice rules, line by line)."""
+        lines = np.asarray(lines)
+        ll = np.asarray(self.linelocs, dtype=np.float64)
+        l_adj = lines + self.lineoffset
+        inner = (l_adj > 0) & (l_adj + 1 < len(ll))
+        k = np.where(inner, l_adj, 1)
+        # get_linelen, lineslice: the same operations, line by line
+        linelen = np.where(k >= self.linecount + self.lineoffset, ll[k] - ll[k - 1], (ll[k + 1] - ll[k - 1]) / 2)
+        linelen = np.where(linelen <= 0, float(self.rf.linelen), linelen)
+        b = ll[k] + begin * (self.rf.samplesperline * linelen)
+        e = b + length * (self.rf.samplesperline * self.rf.linelen) + 1
+        demod = self.data["video"]["demod"]
+        ok = inner & (b >= 0) & (e < len(demod) + 1)  # (not for a location that is no number)
+        lo, hi = np.where(ok, b, 0).astype(np.int64), np.where(ok, e, 0).astype(np.int64)
+        areas = []
+        for m in np.unique((hi - lo)[ok]):
+            rows = np.nonzero(ok & (hi - lo == m))[0]
+            areas.append((rows, demod[lo[rows][:, None] + np.arange(m)]))
+        return areas, np.nonzero(~ok)[0]
+
     def usectooutpx(self, x):
         return x * self.rf.SysParams["outfreq"]
 
@@ -824,7 +849,16 @@ class FieldLogicNTSC(FieldLogic):
         return adj_ll
 
     def calc_burstmedian(self):
-        return np.median([self.get_burstlevel(l) for l in range(11, 264)]) / self.rf.DecoderParams["hz_ire"]
+        # get_burstlevel of every line at once (a row's sums are numpy's of the line alone)
+        lines = range(11, 264)
+        levels = np.empty(len(lines))
+        areas, rest = self.line_areas(lines, 5.5, 2.4)
+        for rows, a in areas:
+            a = a.astype(np.float64)
+            levels[rows] = np.sqrt(np.mean(np.square(a - np.mean(a, axis=1)[:, None]), axis=1)) * np.sqrt(2)
+        for i in rest:
+            levels[i] = self.get_burstlevel(lines[i])
+        return np.median(levels) / self.rf.DecoderParams["hz_ire"]
 
     def apply_offsets(self, linelocs, phaseoffset, picoffset=0):
         return np.array(linelocs) + picoffset + (phaseoffset * (self.rf.freq / (4 * 315 / 88)))
@@ -884,7 +918,22 @@ class FieldLogicPAL(FieldLogic):
         return frms(area) * np.sqrt(2)
 
     def calc_burstmedian(self):
-        levels = [b for b in (self.get_burstlevel(l) for l in range(11, 313)) if b is not None]
+        # get_burstlevel of every line at once (a row's sums are numpy's of the line alone)
+        lines = range(11, 313)
+        levels = [None] * len(lines)
+        areas, rest = self.line_areas(lines, 5.5, 2.4)
+        for rows, a in areas:
+            a = a.astype(np.float32)
+            a -= np.mean(a.astype(np.float64), axis=1).astype(np.float32)[:, None]
+            high = np.max(a, axis=1) > (30 * self.rf.DecoderParams["hz_ire"])
+            nan = np.isnan(a).any(axis=1)
+            d = a.astype(np.float64)
+            level = np.sqrt(np.mean(np.square(d - np.mean(d, axis=1)[:, None]), axis=1)) * np.sqrt(2)
+            for i, h, bad, v in zip(rows, high, nan, level):
+                levels[i] = self.get_burstlevel(lines[i]) if bad else None if h else v
+        for i in rest:
+            levels[i] = self.get_burstlevel(lines[i])
+        levels = [b for b in levels if b is not None]
         if levels == []:
             return 0.0
         return np.median(levels) / self.rf.DecoderParams["hz_ire"]

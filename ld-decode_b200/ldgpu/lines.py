@@ -426,6 +426,22 @@ def _lib_stream(stream):
     return stream if stream else 1
 
 
+def device_columns(v, keys, device):
+    """Fields `keys` of a field read's video (Field.data["video"]) as float32
+    device tensors.  Records of float32 fields cross as they lie, in one copy,
+    and are taken apart on the device: gathering one column of 0.95 M records
+    on the host took 0.56 ms, copying all four 0.8 ms."""
+    import torch
+    fields = getattr(getattr(v, "dtype", None), "fields", None)
+    if (len(keys) > 1 and fields and v.ndim == 1 and v.flags.c_contiguous and v.flags.writeable
+            and v.dtype.itemsize == 4 * len(fields) and all(f[0] == np.float32 for f in fields.values())):
+        names = sorted(fields, key=lambda k: fields[k][1])
+        host = v.view(np.ndarray).view(np.float32).reshape(len(v), len(names))
+        whole = torch.from_numpy(host).to(device)
+        return {k: whole[:, names.index(k)].contiguous() for k in keys}
+    return {k: torch.from_numpy(np.ascontiguousarray(v[k], dtype=np.float32)).to(device) for k in keys}
+
+
 class LineLocator:
     """Batched Field.process() for a demodulated capture on the device."""
 
@@ -508,7 +524,7 @@ class LineLocator:
         U = rf.blocklen - rf.blockcut - rf.blockcut_end
         nblocks = n // U
         dev = torch.device("cuda", torch.cuda.current_device())
-        arrays = {k: torch.from_numpy(np.ascontiguousarray(v[k], dtype=np.float32)).to(dev) for k in keys}
+        arrays = device_columns(v, keys, dev)
         self.begin(arrays)
         runs = self.sync_runs(arrays["demod_05"].data_ptr(), n)
         prev = field.prevfield if getattr(field.prevfield, "valid", False) else None

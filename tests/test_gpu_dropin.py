@@ -82,3 +82,29 @@ def test_dropin_fields_equal_batched_and_reference(cuda_ok, name):
             print(name, i, "ok", f.fieldPhaseID)
     finally:
         rf.close()
+
+
+@pytest.mark.parametrize("form", ["records", "view", "dict", "mixed", "read-only"])
+def test_video_columns_cross_as_they_are(cuda_ok, form):
+    """A field read's video reaches the device column by column whatever
+    holds it: records of float32 fields (one copy), a strided part of them,
+    arrays by name, records with other types, records that may not be written."""
+    import torch
+    from ldgpu.lines import device_columns
+    names = ["demod", "demod_raw", "demod_05", "demod_burst", "demod_pilot"]
+    rng = np.random.default_rng(1)
+    cols = {k: rng.normal(size=1003).astype(np.float32) for k in names}
+    v = cols
+    if form in ("records", "view", "read-only"):
+        v = np.rec.fromarrays([cols[k] for k in names], names=names)
+    if form == "view":
+        v, cols = v[::2], {k: a[::2] for k, a in cols.items()}
+    if form == "read-only":
+        v.flags.writeable = False
+    if form == "mixed":
+        v = np.rec.fromarrays([cols[k] for k in names] + [np.arange(1003, dtype=np.float64)], names=names + ["t"])
+    for keys in (("demod", "demod_05", "demod_burst"), ("demod_pilot",)):
+        got = device_columns(v, keys, torch.device("cuda"))
+        for k in keys:
+            np.testing.assert_array_equal(got[k].cpu().numpy(), cols[k])
+            assert got[k].is_contiguous() and got[k].dtype == torch.float32

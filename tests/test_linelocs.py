@@ -133,3 +133,41 @@ def test_consecutive_fields_match_reference(case):
         prev = f
         i += 1
     np.testing.assert_allclose(skipped, g["skipped_starts"], atol=1e-6)
+
+
+@pytest.mark.parametrize("system", ["NTSC", "PAL"])
+@pytest.mark.parametrize("odd", ["regular", "off the read", "not a number", "out of order"])
+def test_burst_median_equals_line_by_line(system, odd):
+    """calc_burstmedian takes all lines at once; the same bits as
+    get_burstlevel line by line, also for slices that leave the read, samples
+    that are no numbers and lines that run backwards."""
+    rf = RFParams(system=system)
+    cls = FieldLogicPAL if system == "PAL" else FieldLogicNTSC
+    rng = np.random.default_rng(3)
+    nl = 326 if system == "PAL" else 273
+    f = cls.__new__(cls)
+    f.rf, f.linecount, f.lineoffset = rf, 262, 0
+    f.linelocs = 900.0 + 2550.3 * np.arange(nl) + rng.normal(size=nl) * 5
+    n = int(f.linelocs[-1]) + 3000
+    x = (rf.DecoderParams["ire0"] + rng.normal(0, 8e4, n)).astype(np.float32)
+    if odd == "off the read":
+        x = x[:int(f.linelocs[200])]
+        f.linelocs[20], f.linelocs[30] = -900.5, -150.0
+    elif odd == "not a number":
+        x[int(f.linelocs[50]) + 240] = np.nan
+    elif odd == "out of order":
+        f.linelocs[[40, 41]] = f.linelocs[[41, 40]]
+    for video in ({"demod": x}, np.rec.fromarrays([x, x * 2], names=["demod", "demod_05"])):
+        f.data = {"video": video}
+        if odd == "off the read" and system == "PAL":
+            # an empty slice has no largest sample, in the reference too
+            with pytest.raises(ValueError):
+                f.get_burstlevel(312)
+            with pytest.raises(ValueError):
+                f.calc_burstmedian()
+            continue
+        levels = [f.get_burstlevel(l) for l in (range(11, 313) if system == "PAL" else range(11, 264))]
+        levels = [v for v in levels if v is not None]
+        assert len(levels) > 100
+        want = np.median(levels) / rf.DecoderParams["hz_ire"]
+        assert np.array_equal(f.calc_burstmedian(), want, equal_nan=True)
