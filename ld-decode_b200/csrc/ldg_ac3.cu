@@ -133,8 +133,9 @@ __global__ void __launch_bounds__(kAc3Threads) ac3_frontend_kernel(const __grid_
 // its reads are contiguous.  Taps come from the kernel's parameters
 // (constant operands).  Each output is the same chain of multiply-adds as the
 // general kernel's, so the results are equal bit for bit.
-// 2 s of int16 samples (80 M), B200: 2093 us by the general kernel, 197 us by this one
-// (1.0 TB/s of the 200 MB it has to move).
+// 2 s of int16 samples (80 M), B200: 2058 us by the general kernel, 172 us by this
+// one (1.2 TB/s of the 200 MB it has to move); 197 us with the mixer's entries read
+// one by one and the matched filter's last taps by scalar loads.
 
 constexpr int kFastThreads = 512;
 constexpr int kHb19Nz = 11, kHb23Nz = 13, kMaxRrc = kMaxAc3Rrc;
@@ -149,7 +150,7 @@ __host__ __device__ constexpr int pad8(int i) { return i + 4 * (i >> 5); }
 constexpr int kHalf0 = pad8(8192 + 32), kHalf1 = pad8(4096 + 32), kHalf2 = pad8(2048 + 32), kHalf3 = 1024 + 32;
 constexpr int kXLen = 1024;  // a channel's stage-4 samples, shifted by up to three
 constexpr int kBufA = 2 * kHalf0, kBufB = 2 * kHalf1;
-static_assert(4 * kHalf2 <= kBufA && 4 * kHalf3 <= kBufB && 2 * kXLen <= kBufA, "stages share two buffers");
+static_assert(4 * kHalf2 <= kBufA && 4 * kHalf3 <= kBufB && 2 * kXLen + 4 <= kBufA, "stages share two buffers");
 
 struct Ac3FastParams {
     const void* in;
@@ -280,11 +281,14 @@ __global__ void __launch_bounds__(kFastThreads, 2) ac3_frontend_fast_kernel(cons
         const int k0 = 8 * t;
         float y[8], q[8];
         hb19x8(B, B + kHalf1, k0, p.hb19, y);
+        // two table entries per load (lo2 and k0 are even, the table's length too)
 #pragma unroll
-        for (int r = 0; r < 8; ++r) {
-            const float2 cs = __ldg(p.mix + (int)((lo2 + k0 + r) & p.mix_mask));
+        for (int r = 0; r < 8; r += 2) {
+            const float4 cs = __ldg(reinterpret_cast<const float4*>(p.mix + (int)((lo2 + k0 + r) & p.mix_mask)));
             q[r] = y[r] * cs.y;
             y[r] = y[r] * cs.x;
+            q[r + 1] = y[r + 1] * cs.w;
+            y[r + 1] = y[r + 1] * cs.z;
         }
         st4(A + pad8(k0 >> 1), y[0], y[2], y[4], y[6]);
         st4(A + kHalf2 + pad8(k0 >> 1), y[1], y[3], y[5], y[7]);
@@ -314,7 +318,7 @@ __global__ void __launch_bounds__(kFastThreads, 2) ac3_frontend_fast_kernel(cons
     // stage 4 (23 taps): B -> A, shifted so that the matched filter's reads
     // of four taps start on 16 bytes
     const int shift = (4 - p.n_rrc) & 3;
-    float* X = A + ch * kXLen;
+    float* X = A + 4 + ch * kXLen;  // (four words of room before the first sample)
     {
         const int k0 = 4 * tc;
         const float* E = B + 2 * ch * kHalf3;
@@ -373,12 +377,17 @@ __global__ void __launch_bounds__(kFastThreads, 2) ac3_frontend_fast_kernel(cons
                     acc[r] = fmaf(h, x[3 + r - m], acc[r]);
             }
             hi = lo;
-            if (g + 1 < groups) lo = ld4(w0 - 3 - 4 * (g + 1));
+            lo = ld4(w0 - 3 - 4 * (g + 1));  // (at the last group X[k0 ..] when taps remain, else discarded)
         }
-        for (int k = 4 * groups; k < p.n_rrc; ++k) {
-            const float h = p.rrc[k];
+        const int rest = p.n_rrc & 3;
+        const float x[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
 #pragma unroll
-            for (int r = 0; r < 4; ++r) acc[r] = fmaf(h, w0[r - k], acc[r]);
+        for (int m = 0; m < 3; ++m) {
+            if (m < rest) {
+                const float h = p.rrc[4 * groups + m];
+#pragma unroll
+                for (int r = 0; r < 4; ++r) acc[r] = fmaf(h, x[3 + r - m], acc[r]);
+            }
         }
         float* out = (ch ? p.out_q : p.out_i) + (J - p.out_first) + k0;
 #pragma unroll
