@@ -20,12 +20,13 @@
 // Bound: HBM, 20 bytes per sample of the field's lines.  One CTA doing all of
 // a field took 1.07 ms for one field and 1.36 ms for 60 (a span merge sample
 // by sample on one thread, and 16 conversions to FP64 per clock and SM);
-// the four kernels 64 us and 285 us (ncu; 72, 8, 168 and 36 us for 60 fields,
-// the mask at 3.8 TB/s).
+// the four kernels 58 us and 240 us (ncu; 68, 8, 128 and 36 us for 60 fields,
+// the mask at 5.0 TB/s).
 #include <cuda_runtime.h>
 #include <stdint.h>
 
 #include <algorithm>
+#include <climits>
 
 #include "ldg_attr.cuh"
 #include "ldg_dropouts.cuh"
@@ -258,7 +259,7 @@ constexpr int kHeld = 4;  // spans a thread keeps from the first merge of its se
 
 }  // namespace
 
-__global__ void __launch_bounds__(kStdThreads, 4) dropout_std_kernel(const DropField* fields, const DropConsts k,
+__global__ void __launch_bounds__(kStdThreads, 5) dropout_std_kernel(const DropField* fields, const DropConsts k,
                                                                   const DropScratch sc) {
     __shared__ double red[kStdThreads / 32];
     const DropField f = fields[blockIdx.y];
@@ -362,10 +363,17 @@ __global__ void __launch_bounds__(kMaskThreads) dropout_mask_kernel(const DropFi
     }
     __syncthreads();
     const float rf_hi = sc.rf_hi[blockIdx.y], fhalf = float_down(k.fhalf);
+    // 32-bit offsets from the tile's first sample: [from, to) the ones in the field's lines
+    const int from = (int)max(lo - i0, 0ll), to = (int)min(hi - i0, (long long)kDropMaskTile);
+    const int base = (int)i0, rot = (int)min((long long)k.video_rot - i0, (long long)kDropMaskTile);
+    const float* hp = f.rfhpf + i0 - k.video_rot;
+    const float* raw = f.raw + i0;
+    const float* dm = f.demod + i0;
+    const float* d5 = f.d05 + i0;
     // last area starting at or before this thread's first sample
     int idx = -1;
     {
-        const int i = (int)min(i0 + t, hi);
+        const int i = base + t;
         int a = 0, b = nreg - 1;
         while (a <= b) {
             const int mid = (a + b) >> 1;
@@ -377,34 +385,39 @@ __global__ void __launch_bounds__(kMaskThreads) dropout_mask_kernel(const DropFi
             }
         }
     }
+    // the area's end and the next one's start, as offsets
+    int end = idx >= 0 ? pm[idx] - base : INT_MIN;
+    int next = idx + 1 < nreg ? rs[idx + 1] - base : INT_MAX;
     unsigned* words = sc.words + (size_t)blockIdx.y * sc.nwords + (i0 >> 5);
     constexpr int kBatch = 8;  // samples whose loads are in flight together
 #pragma unroll 1
     for (int j0 = 0; j0 < kMaskPer; j0 += kBatch) {
         float h[kBatch], r[kBatch], d[kBatch], q[kBatch];
+        const int o0 = t + j0 * kMaskThreads;
 #pragma unroll
         for (int j = 0; j < kBatch; ++j) {
-            const long long i = i0 + t + (j0 + j) * kMaskThreads;
-            const bool in = i >= lo && i < hi;
-            h[j] = in && i >= k.video_rot ? __ldcs(f.rfhpf + i - k.video_rot) : 0.0f;
-            r[j] = in ? __ldcs(f.raw + i) : 0.0f;
-            d[j] = in ? __ldcs(f.demod + i) : 0.0f;
-            q[j] = in ? __ldcs(f.d05 + i) : 0.0f;
+            const int o = o0 + j * kMaskThreads;
+            const bool in = o >= from && o < to;
+            h[j] = in && o >= rot ? __ldcs(hp + o) : 0.0f;
+            r[j] = in ? __ldcs(raw + o) : 0.0f;
+            d[j] = in ? __ldcs(dm + o) : 0.0f;
+            q[j] = in ? __ldcs(d5 + o) : 0.0f;
         }
 #pragma unroll
         for (int j = 0; j < kBatch; ++j) {
-            const long long i = i0 + t + (j0 + j) * kMaskThreads;
-            bool e = false;
-            if (i >= lo && i < hi) {
-                while (idx + 1 < nreg && rs[idx + 1] <= i) ++idx;
-                const bool sync = idx >= 0 && i < pm[idx];
-                e = i >= k.video_rot && (h[j] > rf_hi || h[j] < -rf_hi);
-                e |= r[j] > fhalf;
-                e |= (d[j] < (sync ? k.smin : k.vmin)) || (d[j] > k.vmax);
-                e |= (q[j] < (sync ? k.smin05 : k.vmin05)) || (q[j] > k.vmax05);
+            const int o = o0 + j * kMaskThreads;
+            while (o >= next) {
+                ++idx;
+                end = pm[idx] - base;
+                next = idx + 1 < nreg ? rs[idx + 1] - base : INT_MAX;
             }
-            const unsigned m = __ballot_sync(0xffffffffu, e);
-            if ((t & 31) == 0) words[(t + (j0 + j) * kMaskThreads) >> 5] = m;
+            const bool sync = o < end;
+            bool e = o >= rot && (h[j] > rf_hi || h[j] < -rf_hi);
+            e |= r[j] > fhalf;
+            e |= (d[j] < (sync ? k.smin : k.vmin)) || (d[j] > k.vmax);
+            e |= (q[j] < (sync ? k.smin05 : k.vmin05)) || (q[j] > k.vmax05);
+            const unsigned m = __ballot_sync(0xffffffffu, e && o >= from && o < to);
+            if ((t & 31) == 0) words[o >> 5] = m;
         }
     }
 }
