@@ -1,13 +1,4 @@
-// Sync-pulse runs and per-line refinement of line locations on the GPU.
-//
-// ldg_sync_runs: runs of demod_05 at or below the sync threshold over a
-// whole capture-wide output array -- the pulses findpulses
-// (lddecode/utils.py:1101-1157) finds, for every field read window at once --
-// and the mean level inside the long ones (getpulses' VSYNC level check,
-// core.py:2242-2322).  Two launches: the edges of every tile counted,
-// scanned (decoupled look-back) and written in order by one single-pass
-// kernel; then the runs paired and the long runs' interiors averaged, the
-// results written straight into the caller's pinned buffers.
+// Per-line refinement of line locations on the GPU.
 //
 // ldg_lines_refine: the per-line refinement of Field.process() for all
 // fields of a capture (pulse-level line locations from the host chain):
@@ -41,8 +32,6 @@
 #include <string>
 
 #include "ldg_attr.cuh"
-#include "ldg_copy.cuh"
-#include "ldg_scan.cuh"
 #include "ldgpu.h"
 
 struct ldg_ctx;
@@ -51,239 +40,16 @@ namespace ldg {
 int lines_fail(int code, const std::string& msg);
 int ctx_device(const ldg_ctx* c);
 std::mutex& ctx_mutex(ldg_ctx* c);
-int ctx_lines_scratch(ldg_ctx* c, size_t need, void** out);
-int ctx_host_word(ldg_ctx* c, long long** host, long long** dev);
 }  // namespace ldg
 
 namespace {
 
 constexpr int kMaxL = LDG_CHAIN_MAX_LINES;
-constexpr int kEdgeTile = 16384;  // samples per sync-run scan tile
-constexpr int kEdgeThreads = 256;
 constexpr int kBurstLines = 266;    // compute_burst_offsets covers lines 0..265
 constexpr int kPilotLines = 323;    // refine_linelocs_pilot covers lines 0..322
 constexpr int kZc = 16;             // clb_findbursts' fixed zero-crossing slots
 constexpr int kBurstThreads = 288;  // >= kBurstLines, whole warps
 constexpr int kHsWin = 512;         // samples of a line's H-sync window in shared memory (40 MSPS needs ~480)
-
-// ---------------------------------------------------------------- sync runs
-
-__device__ __forceinline__ bool below(const float* x, long long i, double thr) { return (double)x[i] <= thr; }
-
-// the below-threshold flags of samples base .. base+3 (bit k: sample
-// base+k; none at or past n); a float4 load when the array is 16-byte aligned
-__device__ __forceinline__ unsigned four_flags(const float* __restrict__ x, long long n, long long base, double thr,
-                                               bool aligned) {
-    float v[4];
-    if (aligned && base + 3 < n) {
-        const float4 q = __ldcs(reinterpret_cast<const float4*>(x + base));
-        v[0] = q.x;
-        v[1] = q.y;
-        v[2] = q.z;
-        v[3] = q.w;
-    } else {
-#pragma unroll
-        for (int k = 0; k < 4; ++k) v[k] = base + k < n ? x[base + k] : 0.0f;
-    }
-    unsigned b = 0;
-#pragma unroll
-    for (int k = 0; k < 4; ++k)
-        if (base + k < n && (double)v[k] <= thr) b |= 1u << k;
-    return b;
-}
-
-// look-back states of a tile (low two bits of its flag word; the high bits
-// hold the call's number, so words of earlier calls never match)
-constexpr unsigned long long kTileAgg = 1, kTileIncl = 2;
-constexpr int kLookbackSpins = 1 << 20;  // ~0.1-1 s of polling; then the call fails
-constexpr int kEdgeSteps = kEdgeTile / (4 * kEdgeThreads);  // coalesced float4 steps per thread
-constexpr int kEdgeWords = kEdgeTile / 32;                  // flag words of a tile
-constexpr int kWordsPerThread = kEdgeWords / kEdgeThreads;
-static_assert(kWordsPerThread == 2, "a thread owns two consecutive flag words");
-
-// Sync-run edges in one pass (single-pass scan with decoupled look-back).
-// Each CTA takes the next tile by ticket (so every tile it waits on belongs
-// to a CTA that is already running); reads its samples with coalesced
-// float4 loads into a shared bitmap of below-threshold flags (bit b of word
-// w: sample 32 w + b); each thread then owns two consecutive words (64
-// samples), whose edges -- samples whose flag differs from the sample
-// before -- it counts; one CTA-wide scan of the counts; the tile's total
-// goes to the look-back (warp 0: publish the tile's count, add the counts
-// or the inclusive prefix of the tiles before it 32 at a time, publish its
-// own inclusive prefix); every thread writes its edges as 2*i + (run start ?
-// 1 : 0) in increasing i.  The last tile writes the total.  Each sample is
-// read once, and the scan costs one launch instead of three (count, scan of
-// the tile counts, write), which matters when it runs beside the
-// demodulator and each launch waits for SMs to come free.  A wait that
-// outlasts kLookbackSpins sets *err (host-mapped) and takes the missing
-// count as 0.
-__global__ void __launch_bounds__(kEdgeThreads) edge_pass_kernel(
-    const float* __restrict__ x, long long n, double thr, unsigned long long* ticket, unsigned long long base,
-    unsigned long long call, unsigned long long* flags, long long* agg, long long* incl, long long ntiles,
-    long long* __restrict__ edges, long long cap, long long* __restrict__ total, long long* err) {
-    __shared__ unsigned bm[kEdgeWords];
-    __shared__ long long s_tile, s_excl;
-    __shared__ int warp_tot[kEdgeThreads / 32];
-    __shared__ unsigned s_before;  // flag of the sample before the tile
-    if (threadIdx.x == 0) s_tile = (long long)(atomicAdd(ticket, 1ull) - base);
-    __syncthreads();
-    const long long tile = s_tile;
-    if (tile < 0 || tile >= ntiles) return;  // more CTAs than tiles: never launched so
-    const long long t0 = tile * kEdgeTile;
-    const bool aligned = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    if (threadIdx.x == 0) s_before = t0 > 0 && t0 - 1 < n && below(x, t0 - 1, thr) ? 1u : 0u;
-#pragma unroll 4
-    for (int j = 0; j < kEdgeSteps; ++j) {
-        const long long b0 = t0 + (long long)j * 4 * kEdgeThreads + 4 * threadIdx.x;
-        unsigned f = 0;  // flags of samples b0 .. b0+3 (none past n)
-        if (b0 < n) f = four_flags(x, n, b0, thr, aligned);
-        // eight lanes' four flags make one word (b0 % 32 == 4 * (lane % 8))
-        unsigned v = f << (4 * (lane & 7));
-        v |= __shfl_xor_sync(0xffffffffu, v, 1);
-        v |= __shfl_xor_sync(0xffffffffu, v, 2);
-        v |= __shfl_xor_sync(0xffffffffu, v, 4);
-        if ((lane & 7) == 0) bm[j * (kEdgeThreads / 8) + (threadIdx.x >> 3)] = v;
-    }
-    __syncthreads();
-    // this thread's 64 samples: words 2t and 2t+1, and the flag before them
-    const int w0 = kWordsPerThread * threadIdx.x;
-    const unsigned f0 = bm[w0], f1 = bm[w0 + 1];
-    const unsigned pb = w0 ? bm[w0 - 1] >> 31 : s_before;
-    const long long s0 = t0 + 32LL * w0;  // first sample of word w0
-    unsigned e0 = f0 ^ ((f0 << 1) | pb);
-    unsigned e1 = f1 ^ ((f1 << 1) | (f0 >> 31));
-    // no edges at or past n (flags there are 0, so a run open at n has no end edge)
-    if (s0 + 64 > n) {
-        const long long k0 = n - s0, k1 = n - s0 - 32;
-        e0 &= k0 <= 0 ? 0u : k0 >= 32 ? 0xffffffffu : (1u << k0) - 1u;
-        e1 &= k1 <= 0 ? 0u : k1 >= 32 ? 0xffffffffu : (1u << k1) - 1u;
-    }
-    const int cnt = __popc(e0) + __popc(e1);
-    // CTA-wide exclusive scan of the counts
-    int inc = cnt;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, inc, o);
-        if (lane >= o) inc += y;
-    }
-    if (lane == 31) warp_tot[warp] = inc;
-    __syncthreads();
-    int before = 0, tile_count = 0;
-#pragma unroll
-    for (int w = 0; w < kEdgeThreads / 32; ++w) {
-        before += w < warp ? warp_tot[w] : 0;
-        tile_count += warp_tot[w];
-    }
-    if (warp == 0) {
-        volatile unsigned long long* vf = flags;
-        volatile long long* va = agg;
-        volatile long long* vi = incl;
-        const long long count = tile_count;
-        long long excl = 0;
-        if (tile > 0) {
-            if (lane == 0) {
-                va[tile] = count;
-                __threadfence();
-                vf[tile] = (call << 2) | kTileAgg;
-            }
-            // the warp looks back 32 tiles at a time (lane l: tile p - l) and
-            // stops at the nearest one whose inclusive prefix is out; tiles
-            // before 0 count as an inclusive prefix of 0
-            bool timed_out = false;
-            for (long long p = tile - 1;; p -= 32) {
-                const long long q = p - lane;
-                unsigned long long f = (call << 2) | kTileIncl;
-                if (q >= 0) {
-                    f = vf[q];
-                    for (int spins = 0; (f >> 2) != call && spins < kLookbackSpins; ++spins) {
-                        __nanosleep(64);
-                        f = vf[q];
-                    }
-                }
-                if (__any_sync(0xffffffffu, (f >> 2) != call)) {
-                    timed_out = true;
-                    break;
-                }
-                __threadfence();
-                const unsigned inc_mask = __ballot_sync(0xffffffffu, (f & 3ull) == kTileIncl);
-                const int stop = inc_mask ? __ffs(inc_mask) - 1 : 32;
-                long long v = 0;
-                if (lane < stop && q >= 0) v = va[q];
-                if (lane == stop && q >= 0) v = vi[q];
-#pragma unroll
-                for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-                excl += v;
-                if (inc_mask) break;
-            }
-            if (timed_out && lane == 0) *reinterpret_cast<volatile long long*>(err) = 1;
-        }
-        if (lane == 0) {
-            vi[tile] = excl + count;
-            __threadfence();
-            vf[tile] = (call << 2) | kTileIncl;
-            if (tile == ntiles - 1) *total = excl + count;
-            s_excl = excl;
-        }
-    }
-    __syncthreads();
-    long long k = s_excl + before + inc - cnt;
-    for (unsigned e = e0; e; e &= e - 1) {
-        const int b = __ffs(e) - 1;
-        if (k < cap) edges[k] = 2 * (s0 + b) + ((f0 >> b) & 1u);
-        ++k;
-    }
-    for (unsigned e = e1; e; e &= e - 1) {
-        const int b = __ffs(e) - 1;
-        if (k < cap) edges[k] = 2 * (s0 + 32 + b) + ((f1 >> b) & 1u);
-        ++k;
-    }
-}
-
-// Pair edges 2r (start) and 2r+1 (end) into runs, with the interior mean of
-// long runs; the run count is total / 2 (an odd total leaves a run open at
-// the end), read on the device, and runs beyond `cap` are not written.  A
-// warp takes 32 consecutive runs, one per lane, so the outputs -- host-mapped
-// pinned memory, read by the host after a stream synchronisation without a
-// copy-engine transfer -- are written coalesced; the warp then averages its
-// long runs one at a time.  Block 0 writes the edge count to *count_out.
-__global__ void run_pair_kernel(const long long* __restrict__ edges, const long long* __restrict__ total,
-                                long long cap, const float* __restrict__ x, long long min_long, long long trim_lo,
-                                long long trim_hi, long long* rs, long long* rl, double* rm, long long* count_out) {
-    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
-    const int lane = threadIdx.x & 31;
-    const long long tot = *total;
-    const long long nruns = min(tot / 2, cap);
-    for (long long r0 = (((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * 32; r0 < nruns;
-         r0 += nwarps * 32) {
-        const long long r = r0 + lane;
-        const bool valid = r < nruns;
-        long long s = 0, len = 0;
-        if (valid) {
-            s = edges[2 * r] >> 1;
-            len = (edges[2 * r + 1] >> 1) - s;
-        }
-        double mean = nan("");
-        unsigned longs = __ballot_sync(0xffffffffu, valid && len > min_long);
-        while (longs) {
-            const int l = __ffs(longs) - 1;
-            longs &= longs - 1;
-            const long long ls = __shfl_sync(0xffffffffu, s, l), ll = __shfl_sync(0xffffffffu, len, l);
-            const long long lo = ls + trim_lo, hi = ls + ll - trim_hi;
-            double acc = 0;
-            for (long long i = lo + lane; i < hi; i += 32) acc += (double)x[i];
-#pragma unroll
-            for (int o = 16; o; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-            if (lane == l && hi > lo) mean = acc / (double)(hi - lo);
-        }
-        if (valid) {
-            rs[r] = s;
-            rl[r] = len;
-            rm[r] = mean;
-        }
-    }
-    if (count_out && blockIdx.x == 0 && threadIdx.x == 0) *count_out = tot;
-}
 
 // --------------------------------------------------------- per-line helpers
 
@@ -1423,86 +1189,6 @@ size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 }  // namespace
 
 extern "C" {
-
-int ldg_sync_runs(ldg_ctx* c, const float* d05, int64_t n, double threshold, int64_t min_long, int64_t trim_lo,
-                  int64_t trim_hi, int64_t* run_start, int64_t* run_len, double* run_mean, int64_t cap,
-                  int64_t* nruns, void* stream) {
-    if (!c || !d05 || !run_start || !run_len || !run_mean || !nruns)
-        return ldg::lines_fail(LDG_ERR_ARG, "ldg_sync_runs: NULL argument");
-    if (n < 2 || cap < 1 || trim_lo < 0 || trim_hi < 0) return ldg::lines_fail(LDG_ERR_ARG, "ldg_sync_runs: bad size");
-    std::lock_guard<std::mutex> lk(ldg::ctx_mutex(c));
-    int prev = -1;
-    cudaGetDevice(&prev);
-    cudaSetDevice(ldg::ctx_device(c));
-    cudaStream_t st = (cudaStream_t)stream;
-    const long long ntiles = (n + kEdgeTile - 1) / kEdgeTile;
-    const long long ecap = 2 * cap + 2;
-    const size_t b_tot = 256, b_edges = align256(ecap * sizeof(long long));
-    const size_t b_runs = align256(cap * sizeof(long long));
-    const size_t need = b_tot + b_edges + 2 * b_runs + align256(cap * sizeof(double));
-    void* scratch = nullptr;
-    auto done = [&](int rc) {
-        if (prev >= 0) cudaSetDevice(prev);
-        return rc;
-    };
-    if (ldg::ctx_lines_scratch(c, need, &scratch) != LDG_OK) return done(LDG_ERR_CUDA);
-    char* p = static_cast<char*>(scratch);
-    long long* total = reinterpret_cast<long long*>(p);
-    long long* edges = reinterpret_cast<long long*>(p + b_tot);
-    long long* rs = reinterpret_cast<long long*>(p + b_tot + b_edges);
-    long long* rl = rs + b_runs / sizeof(long long);
-    double* rm = reinterpret_cast<double*>(rl + b_runs / sizeof(long long));
-    auto cuda_fail = [&](const char* what) {
-        ldg::ctx_scan_invalidate(c);
-        return done(ldg::lines_fail(LDG_ERR_CUDA, std::string("ldg_sync_runs: ") + what + ": " +
-                                                      cudaGetErrorString(cudaGetLastError())));
-    };
-    // the look-back state (tickets, per-tile flags and counts) and the
-    // host-mapped words: [0] the edge count, [1] the look-back error flag
-    ldg::ScanState ss;
-    long long *hw = nullptr, *dw = nullptr;
-    if (ldg::ctx_scan_state(c, ntiles, st, &ss) != LDG_OK || ldg::ctx_host_word(c, &hw, &dw) != LDG_OK)
-        return cuda_fail("scan state");
-    volatile long long* vhw = hw;
-    vhw[0] = -1;
-    vhw[1] = 0;
-    edge_pass_kernel<<<(unsigned)ntiles, kEdgeThreads, 0, st>>>(d05, n, threshold, ss.ticket, ss.base, ss.call,
-                                                                ss.flags, ss.agg, ss.incl, ntiles, edges, ecap,
-                                                                total, dw + 1);
-    // runs straight into the caller's pinned (mapped) buffers when they are:
-    // the host then waits for the stream only (no copy-engine transfer, which
-    // would queue behind bulk copies of an end-to-end pipeline)
-    void* drs = ldg::device_view(run_start);
-    void* drl = ldg::device_view(run_len);
-    void* drm = ldg::device_view(run_mean);
-    const bool mapped = drs && drl && drm;
-    if (mapped) {
-        run_pair_kernel<<<4 * 148, 256, 0, st>>>(edges, total, cap, d05, min_long, trim_lo, trim_hi,
-                                                 static_cast<long long*>(drs), static_cast<long long*>(drl),
-                                                 static_cast<double*>(drm), dw);
-    } else {
-        run_pair_kernel<<<4 * 148, 256, 0, st>>>(edges, total, cap, d05, min_long, trim_lo, trim_hi, rs, rl, rm,
-                                                 dw);
-    }
-    if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess) return cuda_fail("scan");
-    if (vhw[1] != 0) {
-        ldg::ctx_scan_invalidate(c);
-        return done(ldg::lines_fail(LDG_ERR_CUDA, "ldg_sync_runs: a tile's look-back wait timed out"));
-    }
-    const long long nedges = vhw[0];
-    if (nedges < 0) return cuda_fail("run count not written");
-    const long long nr = nedges / 2;
-    *nruns = nr;
-    if (nr > cap || nedges > ecap) return done(ldg::lines_fail(LDG_ERR_RANGE, "ldg_sync_runs: more runs than cap"));
-    if (!mapped && nr > 0) {
-        if (cudaMemcpyAsync(run_start, rs, nr * sizeof(long long), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-            cudaMemcpyAsync(run_len, rl, nr * sizeof(long long), cudaMemcpyDeviceToHost, st) != cudaSuccess ||
-            cudaMemcpyAsync(run_mean, rm, nr * sizeof(double), cudaMemcpyDeviceToHost, st) != cudaSuccess)
-            return cuda_fail("D2H");
-        if (cudaStreamSynchronize(st) != cudaSuccess) return cuda_fail("run copy");
-    }
-    return done(LDG_OK);
-}
 
 int64_t ldg_lines_scratch_bytes(int32_t nfields) {
     if (nfields < 0) return -1;
