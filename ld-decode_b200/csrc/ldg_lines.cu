@@ -13,7 +13,7 @@
 //                        fix_badlines (2566-2589) -> final line locations;
 //                        the burst levels and line 7-19 burst crossings
 //                        of determine_field_number (3095-3203).
-//   pal_sequence_kernel  PAL, one warp walking the fields in order: the
+//   pal_sequence_kernel  PAL, one CTA walking the fields in order: the
 //                        8-field sequence (field phase IDs).
 //   burst_round_kernel   NTSC, one CTA per field, twice, and
 //   burst_verify_kernel  one CTA walking the fields in order: the burst
@@ -223,29 +223,40 @@ __device__ void fix_badlines_block(const double* ll, const unsigned char* bad, d
     __syncthreads();
 }
 
-// block-wide sort of up to 512 doubles in shared memory (NaN-free keys)
-__device__ void bitonic512(double* k) {
-    for (int size = 2; size <= 512; size <<= 1) {
-        for (int stride = size >> 1; stride > 0; stride >>= 1) {
-            for (int t = threadIdx.x; t < 256; t += blockDim.x) {
-                const int i = 2 * t - (t & (stride - 1));
-                const int jx = i + stride;
-                const bool up = (i & size) == 0;
-                const double a = k[i], b = k[jx];
-                if ((a > b) == up) {
-                    k[i] = b;
-                    k[jx] = a;
-                }
+// (key, index) pairs in a strict total order
+__device__ __forceinline__ bool pair_less(double ka, int ia, double kb, int ib) {
+    return ka < kb || (ka == kb && ia < ib);
+}
+
+// ascending bitonic sort of one (key, index) pair per lane across a warp
+__device__ __forceinline__ void warp_sort_pairs(double& key, int& idx) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int k = 2; k <= 32; k <<= 1) {
+#pragma unroll
+        for (int j = k >> 1; j > 0; j >>= 1) {
+            const double ok = __shfl_xor_sync(0xffffffffu, key, j);
+            const int oi = __shfl_xor_sync(0xffffffffu, idx, j);
+            const bool up = (lane & k) == 0;
+            const bool lower = (lane & j) == 0;
+            const bool partner_less = pair_less(ok, oi, key, idx);
+            // ascending block: the lower lane keeps the smaller pair
+            const bool take = lower == up ? partner_less : !partner_less;
+            if (take) {
+                key = ok;
+                idx = oi;
             }
-            __syncthreads();
         }
     }
 }
 
-// median of the first `cnt` entries of a sorted array (np.median)
-__device__ __forceinline__ double sorted_median(const double* k, int cnt) {
-    if (cnt & 1) return k[cnt / 2];
-    return (k[cnt / 2 - 1] + k[cnt / 2]) / 2.0;
+// number of pairs in a sorted run of 32 that order before (key, idx)
+__device__ __forceinline__ int run_rank(const double* rk, const int* ri, double key, int idx) {
+    int lo = 0;
+#pragma unroll
+    for (int step = 16; step > 0; step >>= 1)
+        if (pair_less(rk[lo + step - 1], ri[lo + step - 1], key, idx)) lo += step;
+    return lo + (pair_less(rk[lo], ri[lo], key, idx) ? 1 : 0);
 }
 
 struct LineParams {
@@ -454,8 +465,11 @@ __device__ __forceinline__ double phase_distance(double x, double c) {
 constexpr int kRefineWarps = 8;      // lines per CTA of the per-line kernels
 constexpr int kPalThreads = 1024;    // one CTA per PAL field
 constexpr int kLevelLines = 303;     // lines 11 .. 312 and line 6 of the sequence
+constexpr int kLevelWarps = (kLevelLines + 31) / 32;
+constexpr int kStage = 3;            // lines of a warp whose levels' samples are loaded at once
 constexpr int kLevelWin = 99;        // samples of a burst level (odd: lanes on different banks; 40 MSPS needs 98)
-static_assert(kMaxL <= kPalThreads && kLevelLines <= kPalThreads, "one thread per line");
+static_assert(kMaxL <= kPalThreads && kLevelWarps <= kPalThreads / 32 - 4, "one thread per line");
+static_assert(kLevelLines <= kPilotLines && kLevelWin <= 128, "the levels' windows");
 
 // For each of the first `count` threads the largest v of the threads up to and
 // including it.  All threads of the CTA; wsum: 32 ints.
@@ -473,83 +487,124 @@ __device__ __forceinline__ int block_max_scan(int v, int* wsum) {
     return v;
 }
 
-// one refine_linelocs_pilot pass over ll (shared), in place: a warp per line
-// finds the pilot's peak and the crossing after it, a thread per line the rest
-__device__ void pilot_pass(const LineParams& P, double* ll, const float* pilot, long long n, double* zcs,
-                           double* plen, unsigned char* ok, double* red, int* wsum) {
-    const int lane = threadIdx.x & 31;
-    for (int l = threadIdx.x >> 5; l < kPilotLines; l += kPalThreads / 32) {
+// A pilot pass's windows and crossings.
+struct PilotWin {
+    long long st[kPilotLines];              // the line's samples: pilot[st, st + m)
+    int m[kPilotLines];
+    int loc[kPilotLines];                   // the crossing lies between loc - 1 and loc (st's offset); 0: none
+    float a[kPilotLines], b[kPilotLines];   // those two samples
+    double mean;                            // the mean phase
+};
+
+constexpr int kPilotLoads = 8;  // loads in flight per line and lane (40 MSPS needs 241 samples)
+
+// One refine_linelocs_pilot pass over ll (shared), in place: a thread per line
+// computes its window, a warp per two lines finds their pilots' peaks and the
+// crossings after them, a thread per line the rest.  The line's FP64 work --
+// four divisions -- is done once per line, not by every lane of its warp: the
+// FP64 unit issues one warp's instruction per clock and SM, and bounded the
+// pass so.  What is left is mostly latency: the ordered sums of 323 terms, the
+// sines and cosines, the arctangent.
+__device__ void pilot_pass(const LineParams& P, double* ll, const float* pilot, long long n, PilotWin& W, double* zcs,
+                           double* red, int* wsum) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int l = threadIdx.x;
+    double pl = 0, lsoffset = 0;
+    if (l < kPilotLines) {
         double adjfreq = P.freq;
         if (l > 1) adjfreq /= (ll[l] - ll[l - 1]) / P.linelen;
-        const double pl = (adjfreq / P.pilot_mhz) / 2;
+        pl = (adjfreq / P.pilot_mhz) / 2;
         const double b0 = ll[l];
         const long long st = (long long)(b0 + 0.0);
         long long sp = (long long)(b0 + 6 * P.linefreq0 + 0.0 + 1);
         sp = min(sp, n);
-        const double lsoffset = ll[l] - (double)st;
-        double zc = 0;
-        bool good = false;
-        if (st >= 0 && sp > st) {
-            const float* seg = pilot + st;
-            const int m = (int)(sp - st);
-            // the first of the largest magnitudes
+        lsoffset = b0 - (double)st;
+        const bool some = st >= 0 && sp > st;
+        W.st[l] = some ? st : 0;
+        W.m[l] = some ? (int)(sp - st) : 0;
+    }
+    __syncthreads();
+    for (int l0 = warp; l0 < kPilotLines; l0 += 2 * (kPalThreads / 32)) {
+        float v[2][kPilotLoads];
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int line = l0 + q * (kPalThreads / 32);
+            const int m = line < kPilotLines ? W.m[line] : 0;
+            const float* seg = pilot + (line < kPilotLines ? W.st[line] : 0);
+#pragma unroll
+            for (int j = 0; j < kPilotLoads; ++j) v[q][j] = lane + 32 * j < m ? seg[lane + 32 * j] : -0.0f;
+        }
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const int line = l0 + q * (kPalThreads / 32);
+            if (line >= kPilotLines) break;
+            const int m = W.m[line];
+            const float* seg = pilot + W.st[line];
+            // the first of the largest magnitudes: magnitudes as integers, one
+            // up, so that 0 stands for none (a NaN is not larger than anything)
+            unsigned best = 0;
             int peak = 0x7fffffff;
-            float best = -1.0f;
-#pragma unroll 8
-            for (int k = lane; k < m; k += 32) {
-                const float v = fabsf(seg[k]);
-                if (v > best) {
-                    best = v;
+            auto look = [&](float x, int k) {
+                const unsigned key = k < m && fabsf(x) >= 0.0f ? __float_as_uint(fabsf(x)) + 1u : 0u;
+                if (key > best) {
+                    best = key;
                     peak = k;
                 }
-            }
+            };
 #pragma unroll
-            for (int o = 16; o; o >>= 1) {
-                const float bv = __shfl_xor_sync(0xffffffffu, best, o);
-                const int bp = __shfl_xor_sync(0xffffffffu, peak, o);
-                if (bv > best || (bv == best && bp < peak)) {
-                    best = bv;
-                    peak = bp;
-                }
-            }
+            for (int j = 0; j < kPilotLoads; ++j) look(v[q][j], lane + 32 * j);
+            for (int k = lane + 32 * kPilotLoads; k < m; k += 32) look(seg[k], k);
+            const unsigned most = __reduce_max_sync(0xffffffffu, best);
+            peak = (int)__reduce_min_sync(0xffffffffu, best == most ? (unsigned)peak : 0x7fffffffu);
             if (peak == 0x7fffffff) peak = 0;
-            double zb;
-            if (warp_calczc(seg, (long long)m, (double)peak, 0.0, 0, 16, zb)) {
-                zc = (zb - lsoffset) / pl;
-                good = true;
+            // calczc from the peak to 0 within 16 samples
+            const float x0 = lane <= 16 && peak + lane < m ? seg[peak + lane] : 0.0f;
+            const float x1 = __shfl_down_sync(0xffffffffu, x0, 1);
+            const float xp = __shfl_sync(0xffffffffu, x0, 0);
+            const bool hit = lane < 16 && peak + 1 + lane < m && (xp < 0 ? x0 < 0 && x1 >= 0 : x0 > 0 && x1 <= 0);
+            const unsigned hits = __ballot_sync(0xffffffffu, hit);
+            const int first = __ffs(hits) - 1;
+            if (hits ? lane == first : lane == 0) {
+                W.loc[line] = hits ? peak + 1 + first : 0;
+                W.a[line] = x0;
+                W.b[line] = x1;
             }
-        }
-        if (lane == 0) {
-            plen[l] = pl;
-            zcs[l] = zc;
-            ok[l] = good;
         }
     }
     __syncthreads();
+    bool good = false;
+    if (l < kPilotLines) {
+        const int loc = W.loc[l];
+        good = loc > 0;
+        if (good) {
+            const double a = (double)W.a[l], b = (double)W.b[l];
+            const double zb = (double)(loc - 1) + ((b - a != 0) ? -a / (-a + b) : 0.0);
+            zcs[l] = (zb - lsoffset) / pl;
+        }
+    }
     // a line without a crossing repeats the previous line's value (0 before any)
-    const int l = threadIdx.x;
-    const int from = block_max_scan(l < kPilotLines && ok[l] ? l : -1, wsum);
+    const int from = block_max_scan(good ? l : -1, wsum);
     const double z = l < kPilotLines && from >= 0 ? zcs[from] : 0.0;
     // mean phase of the fractional parts
     if (l < kPilotLines) {
         const double x2 = z - (double)(int)z;
         const double th = x2 * 3.14159265358979323846 * 2;
         red[l] = cos(th);
-        red[kMaxL + l] = sin(th);
+        red[kMaxL + 1 + l] = sin(th);
     }
     __syncthreads();
-    __shared__ double s_sum[2];
-    if (l == 0 || l == 32) {  // the two sums in line order, side by side
-        const double* v = red + (l ? kMaxL : 0);
+    if (warp == 0) {  // the two sums in line order, side by side (on different banks)
+        const double* v = red + (lane & 1 ? kMaxL + 1 : 0);
         double a = 0;
 #pragma unroll 8
         for (int k = 0; k < kPilotLines; ++k) a += v[k];
-        s_sum[l >> 5] = a;
+        const double c = __shfl_sync(0xffffffffu, a, 0), s = __shfl_sync(0xffffffffu, a, 1);
+        double am = atan2(s / kPilotLines, c / kPilotLines) / (3.14159265358979323846 * 2);
+        if (am < 0) am = 1 + am;
+        if (lane == 0) W.mean = am;
     }
     __syncthreads();
-    double am = atan2(s_sum[1] / kPilotLines, s_sum[0] / kPilotLines) / (3.14159265358979323846 * 2);
-    if (am < 0) am = 1 + am;
-    if (l < kPilotLines) ll[l] += phase_distance(z, am) * plen[l];
+    if (l < kPilotLines) ll[l] += phase_distance(z, W.mean) * pl;
     __syncthreads();
 }
 
@@ -561,7 +616,7 @@ __device__ void pilot_pass(const LineParams& P, double* ll, const float* pilot, 
 // independent, so they spread over the chip.  With one CTA walking a field's
 // lines, and one thread per line on the bursts or pilots after it, this stage
 // took 220 us for one NTSC field and 355 us for 15 PAL ones; with a warp per
-// line (ncu) 7 + 15 us and 14 + 107 us (this kernel and the next).
+// line (ncu) 7 + 15 us and, PAL, 14 us here (the rest: lines_pal_kernel).
 __global__ void __launch_bounds__(32 * kRefineWarps) lines_hsync_kernel(const __grid_constant__ LineParams P) {
     const int f = P.a.first_field + blockIdx.y;
     const ldg_lines_args& a = P.a;
@@ -639,7 +694,10 @@ __global__ void __launch_bounds__(32 * kRefineWarps) lines_burst_kernel(const __
 }
 
 // PAL, one CTA per field: second differences, two pilot passes, fix_badlines
-// (no backup, lines from 0), the inputs of the 8-field sequence.
+// (no backup, lines from 0), the inputs of the 8-field sequence.  Bound: one
+// field's chain of stages.  15 fields (ncu): 105 us with every lane dividing
+// for its warp's line, one line's loads in flight per warp, the bursts after the
+// levels and the levels' median by a block-wide sort; 51 us so.
 __global__ void __launch_bounds__(kPalThreads) lines_pal_kernel(const __grid_constant__ LineParams P) {
     extern __shared__ float lev[];  // kLevelLines x kLevelWin
     const int f = P.a.first_field + blockIdx.x;
@@ -647,11 +705,12 @@ __global__ void __launch_bounds__(kPalThreads) lines_pal_kernel(const __grid_con
     const long long base = a.startloc[f];
     const long long n = min((long long)a.wlen[f], (long long)(a.capture_len - base));
     const int nl = a.proclines;
-    __shared__ double ll[kMaxL], tmp[kMaxL], plen[kMaxL], red[2 * kMaxL];
-    __shared__ unsigned char bad[kMaxL], okf[kMaxL];
-    __shared__ int wsum[32];
+    __shared__ double ll[kMaxL], tmp[kMaxL], red[2 * kMaxL + 1], mid[2];
+    __shared__ unsigned char bad[kMaxL];
+    __shared__ int wsum[32], runs[kLevelWarps][32];
+    __shared__ PilotWin pw;
     __shared__ BurstWin win[4];
-    static_assert(2 * kMaxL >= 512, "the level sort's keys");
+    static_assert(2 * kMaxL + 1 >= kLevelWarps * 32, "the levels' sorted runs");
     const int i = threadIdx.x, lane = i & 31, warp = i >> 5;
     if (i < nl) {
         ll[i] = P.ll2[(long long)f * kMaxL + i];
@@ -659,8 +718,8 @@ __global__ void __launch_bounds__(kPalThreads) lines_pal_kernel(const __grid_con
     }
     __syncthreads();
     deriv_error_block(ll, bad, nl);
-    pilot_pass(P, ll, a.pilot + base, n, tmp, plen, okf, red, wsum);
-    pilot_pass(P, ll, a.pilot + base, n, tmp, plen, okf, red, wsum);
+    pilot_pass(P, ll, a.pilot + base, n, pw, tmp, red, wsum);
+    pilot_pass(P, ll, a.pilot + base, n, pw, tmp, red, wsum);
     deriv_error_block(ll, bad, nl);
     fix_badlines_block(ll, bad, tmp, nl, 0);
     if (i < nl) {
@@ -677,31 +736,70 @@ __global__ void __launch_bounds__(kPalThreads) lines_pal_kernel(const __grid_con
     const int off = isf ? 2 : 3;
     const int lc_seq = (isf ? 312 : 313) + off;
     const float* demod = a.demod + base;
-    // the levels' samples staged a warp per line, then a thread per line sums
-    // them in order
-    for (int e = warp; e < kLevelLines; e += kPalThreads / 32) {
-        const LevelWindow w = e < kLevelLines - 1 ? pal_level_window(P, tmp, 11 + e, lc_med, n)
-                                                  : pal_level_window(P, tmp, 6 + off, lc_seq, n);
-        if (w.hi - w.lo <= kLevelWin)
-            for (long long k = w.lo + lane; k < w.hi; k += 32) lev[e * kLevelWin + (int)(k - w.lo)] = demod[k];
+    // the levels' samples staged a warp per line, kStage lines' loads in
+    // flight, then a thread per line sums them in order; beside it the last
+    // four warps take the burst crossings of lines 7-19
+    const LevelWindow lw = i >= kLevelLines       ? LevelWindow{0, 0}
+                           : i < kLevelLines - 1 ? pal_level_window(P, tmp, 11 + i, lc_med, n)
+                                                 : pal_level_window(P, tmp, 6 + off, lc_seq, n);
+    const int lm = (int)max(lw.hi - lw.lo, 0LL);
+    if (i < kLevelLines) {
+        pw.st[i] = lm ? lw.lo : 0;
+        pw.m[i] = lm <= kLevelWin ? lm : 0;
+    }
+    __syncthreads();
+    for (int e0 = warp; e0 < kLevelLines; e0 += kStage * (kPalThreads / 32)) {
+        float v[kStage][4];
+#pragma unroll
+        for (int q = 0; q < kStage; ++q) {
+            const int e = e0 + q * (kPalThreads / 32);
+            const int m = e < kLevelLines ? pw.m[e] : 0;
+            const float* x = demod + (e < kLevelLines ? pw.st[e] : 0);
+#pragma unroll
+            for (int j = 0; j < 4; ++j) v[q][j] = lane + 32 * j < m ? x[lane + 32 * j] : 0.0f;
+        }
+#pragma unroll
+        for (int q = 0; q < kStage; ++q) {
+            const int e = e0 + q * (kPalThreads / 32);
+            const int m = e < kLevelLines ? pw.m[e] : 0;
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (lane + 32 * j < m) lev[e * kLevelWin + lane + 32 * j] = v[q][j];
+        }
     }
     __syncthreads();
     double lvl = INFINITY;
     if (i < kLevelLines) {
-        const LevelWindow w = i < kLevelLines - 1 ? pal_level_window(P, tmp, 11 + i, lc_med, n)
-                                                  : pal_level_window(P, tmp, 6 + off, lc_seq, n);
-        const int m = (int)max(w.hi - w.lo, 0LL);
-        const double b = pal_burstlevel(m <= kLevelWin ? lev + i * kLevelWin : demod + w.lo, m, P.hz_ire);
+        const double b = pal_burstlevel(lm <= kLevelWin ? lev + i * kLevelWin : demod + lw.lo, lm, P.hz_ire);
         if (i == kLevelLines - 1) P.adjs[(long long)f * kBurstLines] = b;
         else if (!isnan(b)) lvl = b;
+    } else if (warp >= kPalThreads / 32 - 4) {
+        const int j = warp - (kPalThreads / 32 - 4);
+        warp_burst_record(P, tmp, 7 + 4 * j + off, lc_seq, a.burst + base, demod, n, win[j],
+                          P.rec + (long long)f * kBurstLines + j);
     }
-    if (i < 512) red[i] = lvl;
-    const int cnt = __syncthreads_count(lvl != INFINITY);
-    bitonic512(red);
-    if (i == 0) P.adjs[(long long)f * kBurstLines + 1] = cnt ? sorted_median(red, cnt) / P.hz_ire : 0.0;
-    if (warp < 4)
-        warp_burst_record(P, tmp, 7 + 4 * warp + off, lc_seq, a.burst + base, demod, n, win[warp],
-                          P.rec + (long long)f * kBurstLines + warp);
+    // their median: a level's rank is the sum of its positions in the warps' sorted runs
+    const bool level = lvl != INFINITY;
+    if (warp < kLevelWarps) {
+        double key = lvl;
+        int idx = i;
+        warp_sort_pairs(key, idx);
+        red[i] = key;
+        runs[warp][lane] = idx;
+    }
+    const int cnt = __syncthreads_count(level);
+    if (level) {
+        int r = 0;
+#pragma unroll
+        for (int w = 0; w < kLevelWarps; ++w) r += run_rank(red + 32 * w, runs[w], lvl, i);
+        if (r == (cnt - 1) / 2) mid[0] = lvl;
+        if (r == cnt / 2) mid[1] = lvl;
+    }
+    __syncthreads();
+    if (i == 0) {
+        const double med = cnt & 1 ? mid[1] : (mid[0] + mid[1]) / 2.0;
+        P.adjs[(long long)f * kBurstLines + 1] = cnt ? med / P.hz_ire : 0.0;
+    }
 }
 
 // np.median of 16 doubles (mean of the two middle ones): Batcher's
@@ -736,42 +834,6 @@ __device__ __forceinline__ double median16(double* v) {
     return (v[kZc / 2 - 1] + v[kZc / 2]) / 2.0;
 }
 #undef LDG_CS
-
-// (key, index) pairs in a strict total order
-__device__ __forceinline__ bool pair_less(double ka, int ia, double kb, int ib) {
-    return ka < kb || (ka == kb && ia < ib);
-}
-
-// ascending bitonic sort of one (key, index) pair per lane across a warp
-__device__ __forceinline__ void warp_sort_pairs(double& key, int& idx) {
-    const int lane = threadIdx.x & 31;
-#pragma unroll
-    for (int k = 2; k <= 32; k <<= 1) {
-#pragma unroll
-        for (int j = k >> 1; j > 0; j >>= 1) {
-            const double ok = __shfl_xor_sync(0xffffffffu, key, j);
-            const int oi = __shfl_xor_sync(0xffffffffu, idx, j);
-            const bool up = (lane & k) == 0;
-            const bool lower = (lane & j) == 0;
-            const bool partner_less = pair_less(ok, oi, key, idx);
-            // ascending block: the lower lane keeps the smaller pair
-            const bool take = lower == up ? partner_less : !partner_less;
-            if (take) {
-                key = ok;
-                idx = oi;
-            }
-        }
-    }
-}
-
-// number of pairs in a sorted run of 32 that order before (key, idx)
-__device__ __forceinline__ int run_rank(const double* rk, const int* ri, double key, int idx) {
-    int lo = 0;
-#pragma unroll
-    for (int step = 16; step > 0; step >>= 1)
-        if (pair_less(rk[lo + step - 1], ri[lo + step - 1], key, idx)) lo += step;
-    return lo + (pair_less(rk[lo], ri[lo], key, idx) ? 1 : 0);
-}
 
 // ---- NTSC burst phase of every field (compute_burst_offsets, core.py:3360-3388)
 //
@@ -1033,79 +1095,104 @@ __global__ void __launch_bounds__(kBurstThreads) burst_verify_kernel(const __gri
 }
 
 // PAL 8-field sequence (determine_field_number, core.py:3128-3203), fields in
-// order.  Lane j follows line 7 + 4j: its burst phase starts from the
-// previous field's (0 when there is none, when that line had no result or
-// when that field decided its ID before measuring phases), two passes of
-// clb_findbursts' phase update, rising or not.  The field's ID comes from
-// line 6's burst level against the field's median (present / absent / out of
-// both ranges) and the majority of rising lines, or is the previous ID + 1
-// when that evidence is missing or split.
-__global__ void __launch_bounds__(32) pal_sequence_kernel(const __grid_constant__ LineParams P) {
+// order.  Sixteen lanes, one per zero-crossing slot, follow line 7 + 4j: its
+// burst phase starts from the previous field's (0 when there is none, when
+// that line had no result or when that field decided its ID before measuring
+// phases), two passes of clb_findbursts' phase update, rising or not.  The
+// field's ID comes from line 6's burst level against the field's median
+// (present / absent / out of both ranges) and the majority of rising lines,
+// or is the previous ID + 1 when that evidence is missing or split.  Bound: a
+// field's chain of FP64 latencies, since the next field starts from its
+// phases; the next field's inputs are loaded meanwhile and the slots' median
+// is found by rank.  15 fields, one lane per line sorting its slots: 43 us; so
+// 17 us (ncu).
+constexpr int kSeqThreads = 4 * kZc;
+
+__global__ void __launch_bounds__(kSeqThreads) pal_sequence_kernel(const __grid_constant__ LineParams P) {
     const ldg_lines_args& a = P.a;
     const int f0 = a.first_field, f1 = a.first_field + a.count;
-    const int j = threadIdx.x;
-    double seed = nan("");
+    const int j = threadIdx.x / kZc, slot = threadIdx.x % kZc, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    __shared__ int votes[2][2];  // [turn][warp]: lines | rising lines << 8
+    int turn = 0;  // the other turn's barrier lies between a vote's reads and the next writes
+    double seed;
     int prev_id;
     if (f0 > 0) {
-        if (j < 4) seed = a.phase_adjust[(long long)(f0 - 1) * 4 + j];
+        seed = a.phase_adjust[(long long)(f0 - 1) * 4 + j];
         prev_id = a.field_phase[f0 - 1];
     } else {
-        if (j < 4) seed = a.prev_pal_adjust_dev ? a.prev_pal_adjust_dev[j] : a.prev_pal_adjust[j];
+        seed = a.prev_pal_adjust_dev ? a.prev_pal_adjust_dev[j] : a.prev_pal_adjust[j];
         prev_id = a.prev_field_phase_dev ? *a.prev_field_phase_dev : a.prev_field_phase;
     }
+    struct Inputs {
+        double cyc, b6, bm;
+        int count, rising, valid, has_prev, isfirst;
+    };
+    auto inputs = [&](int f) {
+        const BurstRec& r = P.rec[(long long)f * kBurstLines + j];
+        const double* lev = P.adjs + (long long)f * kBurstLines;
+        return Inputs{r.cyc[slot], lev[0], lev[1], r.count, r.rising, r.valid, a.has_prev[f], a.isfirst[f]};
+    };
+    Inputs next{};
+    if (f0 < f1) next = inputs(f0);
     for (int f = f0; f < f1; ++f) {
-        const bool has_prev = a.has_prev[f] != 0;
+        const Inputs in = next;
+        if (f + 1 < f1) next = inputs(f + 1);
+        const bool has_prev = in.has_prev != 0;
         const int following = has_prev ? (prev_id + 1 == 9 ? 1 : prev_id + 1) : 1;
-        const double b6 = P.adjs[(long long)f * kBurstLines + 0];
-        const double bm = P.adjs[(long long)f * kBurstLines + 1];
         int hasburst = -1;
-        if (!isnan(b6)) {
-            const double b = b6 / P.hz_ire;
-            if (b >= bm * 0.8 && b <= bm * 1.2) hasburst = 1;
-            else if (b < bm * 0.2) hasburst = 0;
+        if (!isnan(in.b6)) {
+            const double b = in.b6 / P.hz_ire;
+            if (b >= in.bm * 0.8 && b <= in.bm * 1.2) hasburst = 1;
+            else if (b < in.bm * 0.2) hasburst = 0;
         }
         double out = nan("");
         int id = following;
-        if (hasburst >= 0) {  // warp-uniform
-            const bool isf = a.isfirst[f] != 0;
+        if (hasburst >= 0) {  // the same for all threads
+            const bool isf = in.isfirst != 0;
             const int m4 = isf ? (hasburst ? 3 : 1) : (hasburst ? 2 : 4);
-            bool valid = false, rising = false;
-            if (j < 4) {
-                const BurstRec r = P.rec[(long long)f * kBurstLines + j];
-                if (r.valid) {
-                    double pa = -((has_prev && !isnan(seed)) ? seed : 0.0);
-                    int rising_count = 0;
-                    for (int pass = 0; pass < 2; ++pass) {
-                        rising_count = 0;
-                        if (r.count) {
-                            double dev[kZc];
-                            int odd = 0;
+            double pa = -((has_prev && !isnan(seed)) ? seed : 0.0);
+            int rising_count = 0;
 #pragma unroll
-                            for (int k = 0; k < kZc; ++k) {
-                                const double cyc = r.cyc[k] + pa;
-                                const int rnd = (int)(cyc + .5);
-                                if (rnd % 2 != 0) odd |= 1 << k;
-                                dev[k] = (double)rnd - cyc;
-                            }
-                            pa += median16(dev);
-                            rising_count = __popc((unsigned)(r.rising ^ odd) & 0xffffu);
-                        }
-                    }
-                    rising = (double)rising_count > ((double)r.count / 2);
-                    out = -pa;
-                    valid = true;
+            for (int pass = 0; pass < 2; ++pass) {
+                const double cyc = in.cyc + pa;
+                const int rnd = (int)(cyc + .5);
+                const double dev = (double)rnd - cyc;
+                const unsigned odd = __ballot_sync(0xffffffffu, rnd % 2 != 0) >> (lane & kZc);
+                // np.median of the line's 16 slots (mean of the two middle ones)
+                int r = 0;
+#pragma unroll
+                for (int k = 0; k < kZc; ++k) {
+                    const double o = __shfl_sync(0xffffffffu, dev, k, kZc);
+                    r += pair_less(o, k, dev, slot);
+                }
+                const int group = lane & kZc;
+                const unsigned m0 = (__ballot_sync(0xffffffffu, r == kZc / 2 - 1) >> group) & 0xffffu;
+                const unsigned m1 = (__ballot_sync(0xffffffffu, r == kZc / 2) >> group) & 0xffffu;
+                const double v0 = __shfl_sync(0xffffffffu, dev, (__ffs(m0) - 1) & (kZc - 1), kZc);
+                const double v1 = __shfl_sync(0xffffffffu, dev, (__ffs(m1) - 1) & (kZc - 1), kZc);
+                if (in.count) {
+                    pa += (v0 + v1) / 2.0;
+                    rising_count = __popc((unsigned)(in.rising ^ odd) & 0xffffu);
                 }
             }
-            const int count = __popc(__ballot_sync(0xffffffffu, valid));
-            const int rcount = __popc(__ballot_sync(0xffffffffu, valid && rising));
+            const bool valid = in.valid != 0;
+            const bool rising = (double)rising_count > ((double)in.count / 2);
+            if (valid) out = -pa;
+            const int lines = __popc(__ballot_sync(0xffffffffu, slot == 0 && valid));
+            const int rlines = __popc(__ballot_sync(0xffffffffu, slot == 0 && valid && rising));
+            turn ^= 1;
+            if (lane == 0) votes[turn][warp] = lines | rlines << 8;
+            __syncthreads();
+            const int both = votes[turn][0] + votes[turn][1];
+            const int count = both & 255, rcount = both >> 8;
             if (count != 0 && rcount * 2 != count) {
                 bool firstfour = rcount * 2 > count;
                 if (m4 == 2) firstfour = !firstfour;
                 id = m4 + (firstfour ? 0 : 4);
             }
         }
-        if (j < 4) a.phase_adjust[(long long)f * 4 + j] = out;
-        if (j == 0) a.field_phase[f] = id;
+        if (slot == 0) a.phase_adjust[(long long)f * 4 + j] = out;
+        if (threadIdx.x == 0) a.field_phase[f] = id;
         seed = out;
         prev_id = id;
     }
@@ -1279,7 +1366,7 @@ extern "C" int ldg_lines_refine(ldg_ctx* c, const ldg_lines_args* a) {
         if (P.system == 1)
             lines_pal_kernel<<<P.a.count, kPalThreads, (size_t)kLevelLines * kLevelWin * sizeof(float), st>>>(P);
     }
-    if (P.system == 1 && (stages & 2)) pal_sequence_kernel<<<1, 32, 0, st>>>(P);
+    if (P.system == 1 && (stages & 2)) pal_sequence_kernel<<<1, kSeqThreads, 0, st>>>(P);
     if (P.system == 0) {
         if (stages & 2) {
             for (int r = 1; r <= kBurstRounds; ++r)

@@ -282,3 +282,28 @@ def test_consecutive_fields_match_reference(cuda_ok, case, variant):
             assert lsb.max() <= 1 and np.mean(lsb == 0) > 0.95
     finally:
         rf.close()
+
+
+@pytest.mark.parametrize("damage", ["pilot", "burst", "both"])
+def test_pal_damaged_pilot_and_burst(capture, damage):
+    """Lines whose pilot has no crossing (zero, constant, a peak at its end),
+    fields without burst: the line locations and field sequence of the host."""
+    import torch
+    rf, arrays, host, nb, ref = capture
+    if rf.system != "PAL":
+        pytest.skip("PAL only")
+    host = {k: v.copy() for k, v in host.items()}
+    line = int(rf.linelen)
+    n = len(host["demod_05"])
+    if damage != "burst":
+        p = host["demod_pilot"]
+        for k, at in enumerate(range(500_000, n - 40 * line, 171_717)):
+            seg = p[at:at + (1 + k % 3) * line]
+            seg[:] = (0.0, 1.0, np.linspace(1, 2, len(seg)))[k % 3]
+        p[2_000_000:2_000_000 + 30 * line] = 0.0
+    if damage != "pilot":
+        host["demod_burst"][1_500_000:2_300_000] = 0.0
+        host["demod"][3_000_000:3_000_000 + 20 * line] = host["demod"][0]
+    dev = {k: torch.from_numpy(v).cuda() for k, v in host.items()}
+    reads, _ = host_field_chain(rf, host, nb)
+    _compare(rf, LineLocator(rf).locate(dev, nb), [(w, f) for w, f in reads if f.valid])
