@@ -53,3 +53,28 @@ def test_gpu_unpack_equals_oracle(cuda_ok):
     for data, sample, readlen, want in _ref_cases():
         np.testing.assert_array_equal(load_packed_data_4_40(io.BytesIO(data.tobytes()), sample, readlen), want)
     assert load_packed_data_4_40(io.BytesIO(packed[:100].tobytes()), 0, 4096) is None
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("skew", [0, 4])  # samples the output lies past a 16-byte boundary
+@pytest.mark.parametrize("lead", [0, 4, 8, 12])  # bytes the packed buffer does
+def test_gpu_unpack_tile_edges(cuda_ok, skew, lead):
+    """Eight samples of a thread and 4096 of a CTA: every start within a
+    group, ends at, before and past those edges, nothing written outside."""
+    import torch
+    from ldgpu.ingest import unpack_lds
+    rng = np.random.default_rng(8 + lead)
+    groups = 6000
+    packed = rng.integers(0, 256, 5 * groups, dtype=np.uint8)
+    buf = torch.empty(lead + len(packed), dtype=torch.uint8, device="cuda")
+    d = buf[lead:]
+    d.copy_(torch.from_numpy(packed))
+    ref = oing.unpack_4_40(packed, 4 * groups, 0)
+    for first in (0, 1, 2, 3, 4, 7, 8191):
+        for n in (1, 3, 4, 5, 8, 9, 4095, 8187, 8188, 8189, 8191, 8192, 8193, 4 * groups - first):
+            n = min(n, 4 * groups - first)
+            out = torch.full((skew + n + 8,), 12345, dtype=torch.int16, device="cuda")
+            unpack_lds(d, first, n, out=out[skew:skew + n])
+            got = out.cpu().numpy()
+            np.testing.assert_array_equal(got[skew:skew + n], ref[first:first + n])
+            assert (got[:skew] == 12345).all() and (got[skew + n:] == 12345).all()
