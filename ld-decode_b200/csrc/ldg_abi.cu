@@ -198,7 +198,7 @@ int check_tbc_field(const ldg_tbc_field& f, const std::string& who) {
 // Doubles of spline scratch a field needs.
 size_t tbc_spline_doubles(const ldg_tbc_field& f) {
     if (f.wow_interp < LDG_WOW_QUADRATIC) return 0;
-    return ldg::spline_scratch_doubles(f.nlines, f.outwidth, f.lineoffset, f.linesout, f.wow_smoothing > 0);
+    return ldg::spline_scratch_doubles(f.nlines, f.outwidth, f.linesout, f.wow_smoothing > 0);
 }
 
 // Device descriptor of one field: geometry, levels and scratch pointers

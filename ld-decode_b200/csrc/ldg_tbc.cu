@@ -457,8 +457,8 @@ __device__ double select_mean(Visit visit, long long n, long long r1, bool two, 
 //                   which rank to take); a bracket for the MAD
 //   spline_pass     the same for |wow - median|
 //   spline_mad      the MAD
-//   spline_maps / spline_levels   (smoothing) the IIR over each 32 pixels as
-//                   a map y -> b^32 y + B, then the maps' scan
+//   spline_maps / spline_levels / spline_maps   (smoothing) the IIR over each
+//                   chunk of pixels as a map, the maps' scan, the states
 // A bracket's ranks lie kSplMargin samples either side of the median's: the
 // factors are smooth along a line, so an evenly stepped sample misjudges a
 // rank by about one sample per crossing and square root of the crossings, ~10
@@ -466,11 +466,12 @@ __device__ double select_mean(Visit visit, long long n, long long r1, bool two, 
 // from all pixels by radix passes.
 // Bound: instruction issue of the walks (FP64 pipe next).  As one CTA per
 // field walking all pixels up to ten times: 672 us for 60 NTSC fields (cubic,
-// smoothing; as long for one); the seven launches together 215 us (ncu: build
-// 67, passes 34 and 33, median 31, MAD 12, maps 24, levels 14; the build is one
-// thread's chain of divisions and two rank selections).
+// smoothing; as long for one); the eight launches together 250 us (ncu: build
+// 67, passes 33 and 32, median 31, MAD 12, maps 44 and 26, levels 8; the build
+// is one thread's chain of divisions and two rank selections).
 constexpr int kSplSlices = 16;
 constexpr int kSplPassThreads = 256;
+constexpr int kSplMapThreads = 64;
 constexpr int kSplSamples = 4096;
 constexpr int kSplMargin = 48;
 static_assert(sizeof(SplCtl) <= kSplCtlDoubles * sizeof(double), "the control block's place");
@@ -736,48 +737,64 @@ __global__ void __launch_bounds__(kSplThreads) spline_mad_kernel(const TbcField*
     if (threadIdx.x == 0) f.stat[1] = mad > 0 ? threshold_mult * mad : 0.001;
 }
 
-// Level-adjust IIR (utils.py:141-149), y[0] = la[0], y[i] = a la[i] + b y[i-1],
-// in groups of 32 pixels that end where the gather's warps begin (group 0 the
-// pixels before the first such place): the map of group g is y -> b^32 y + B.
-__device__ __forceinline__ long long level_group_end(const TbcField& f, long long g) {
-    return (long long)f.outwidth * (f.lineoffset + 1) % 32 + 32 * g;
+// Level-adjust IIR (utils.py:141-149), y[0] = la[0], y[i] = a la[i] + b y[i-1]:
+// kSplChunks contiguous chunks of a field's pixels, one thread each.  The first
+// launch finds each chunk's map y -> A y + B, spline_levels each chunk's y
+// before its first pixel, the second the levels where the gather's warps begin.
+// The chunks and the order of the scan decide the levels' last bits.
+template <class Body>
+__device__ __forceinline__ void walk_levels(const TbcField& f, int chunk, Body body) {
+    const double med = f.stat[0], thr = f.stat[1];
+    const long long C = (f.nwow + kSplChunks - 1) / kSplChunks;
+    const long long i0 = chunk * C;
+    field_walk(f)(i0, min(f.nwow, i0 + C), [&](long long i, double wv) {
+        const double la = fabs(__dadd_rn(wv, -med)) > thr ? med : wv;
+        body(i, __dmul_rn(f.smooth_a, la), la);
+    });
 }
 
-__global__ void __launch_bounds__(kSplPassThreads) spline_maps_kernel(const TbcField* fields) {
+template <bool Record>
+__global__ void __launch_bounds__(kSplMapThreads) spline_maps_kernel(const TbcField* fields) {
     const TbcField& f = fields[blockIdx.y];
     if (f.spline_k < 2 || !(f.smooth_b > 0) || spline_ctl(f)->bad) return;
-    const double a = f.smooth_a, b = f.smooth_b, med = f.stat[0], thr = f.stat[1];
-    const long long ngroups = spline_level_groups(f);
-    for (long long g = (long long)blockIdx.x * kSplPassThreads + threadIdx.x; g < ngroups;
-         g += (long long)gridDim.x * kSplPassThreads) {
+    const int chunk = blockIdx.x * kSplMapThreads + threadIdx.x;
+    const double b = f.smooth_b;
+    double* maps = spline_maps(f);
+    if (!Record) {
         double B = 0.0;
-        field_walk(f)(g ? level_group_end(f, g - 1) : 0, min(level_group_end(f, g), f.nwow), [&](long long i, double wv) {
-            const double la = fabs(__dadd_rn(wv, -med)) > thr ? med : wv;
-            B = i == 0 ? la : __dadd_rn(__dmul_rn(a, la), __dmul_rn(b, B));
+        walk_levels(f, chunk, [&](long long i, double ala, double la) {
+            B = i == 0 ? la : __dadd_rn(ala, __dmul_rn(b, B));
         });
-        spline_maps(f)[g] = B;
+        maps[chunk] = B;
+    } else {
+        // the level just before output pixel 32 m (wow index igbase + 32 m)
+        const long long igbase = (long long)f.outwidth * (f.lineoffset + 1);
+        const long long nyb = ((long long)f.linesout * f.outwidth + 31) / 32;
+        const long long i0 = chunk * ((f.nwow + kSplChunks - 1) / kSplChunks);
+        long long m = i0 + 1 - igbase <= 0 ? 0 : (i0 + 1 - igbase + 31) / 32;
+        double y = maps[kSplChunks + chunk];
+        walk_levels(f, chunk, [&](long long i, double ala, double la) {
+            y = i == 0 ? la : __dadd_rn(ala, __dmul_rn(b, y));
+            if (m < nyb && i + 1 == igbase + 32 * m) {
+                f.ybefore[m] = y;
+                ++m;
+            }
+        });
     }
 }
 
-__global__ void __launch_bounds__(kSplThreads) spline_levels_kernel(const TbcField* fields) {
+__global__ void __launch_bounds__(kSplChunks) spline_levels_kernel(const TbcField* fields) {
     const TbcField& f = fields[blockIdx.x];
     if (f.spline_k < 2 || !(f.smooth_b > 0) || spline_ctl(f)->bad) return;
     __shared__ double wA[32], wB[32], wy[32];
     const int t = threadIdx.x, lane = t & 31, w = t >> 5;
-    const long long n = spline_level_groups(f);
-    const double* maps = spline_maps(f);
-    double b32 = 1.0;
-    for (int k = 0; k < 32; ++k) b32 = __dmul_rn(f.smooth_b, b32);
-    // the first pixel's group starts the recurrence: its map is a constant
-    const long long head = level_group_end(f, 0) > 0 ? 0 : 1;
-    const long long per = (n + kSplThreads - 1) / kSplThreads;
-    const long long g0 = min(n, t * per), g1 = min(n, g0 + per);
-    double A = 1.0, B = 0.0;
-    for (long long g = g0; g < g1; ++g) {
-        const double m = g <= head ? 0.0 : b32;
-        B = g < head ? B : __fma_rn(m, B, maps[g]);
-        A = g < head ? A : __dmul_rn(A, m);
-    }
+    double* maps = spline_maps(f);
+    // the chunk's A: b times itself for each pixel, 0 when the first is among them
+    const long long C = (f.nwow + kSplChunks - 1) / kSplChunks;
+    const int pixels = (int)max(min(f.nwow - t * C, C), 0LL);
+    double A = t == 0 && pixels ? 0.0 : 1.0, B = maps[t];
+    for (int k = 0; k < pixels; ++k) A = __dmul_rn(f.smooth_b, A);
+    // inclusive scan of the maps over the warp, then over the warps
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const double Ap = __shfl_up_sync(0xffffffffu, A, o), Bp = __shfl_up_sync(0xffffffffu, B, o);
@@ -800,15 +817,7 @@ __global__ void __launch_bounds__(kSplThreads) spline_levels_kernel(const TbcFie
     }
     __syncthreads();
     const double Ae = __shfl_up_sync(0xffffffffu, A, 1), Be = __shfl_up_sync(0xffffffffu, B, 1);
-    double y = lane == 0 ? wy[w] : __fma_rn(Ae, wy[w], Be);
-    // the level just before output pixel 32 mq: after the group that ends there
-    const long long first = (long long)f.outwidth * (f.lineoffset + 1) / 32;  // group that ends at output pixel 0
-    const long long nyb = ((long long)f.linesout * f.outwidth + 31) / 32;
-    for (long long g = g0; g < g1; ++g) {
-        if (g >= head) y = __fma_rn(g <= head ? 0.0 : b32, y, maps[g]);
-        const long long mq = g - first;
-        if (mq >= 0 && mq < nyb) f.ybefore[mq] = y;
-    }
+    maps[kSplChunks + t] = lane == 0 ? wy[w] : __fma_rn(Ae, wy[w], Be);
 }
 
 constexpr int kGatherThreads = 128;  // 16 CTAs per SM (256 and 8: 1 % slower, 512 and 4: 4 %)
@@ -1057,9 +1066,13 @@ cudaError_t launch_tbc(const TbcField* dfields, const TbcField* hfields, int nfi
         if (any_smooth) {
             for (int off = 0; off < nfields; off += 65535) {
                 const unsigned n = (unsigned)(nfields - off < 65535 ? nfields - off : 65535);
-                spline_maps_kernel<<<dim3(2 * kSplSlices, n), kSplPassThreads, 0, stream>>>(dfields + off);
+                spline_maps_kernel<false><<<dim3(kSplChunks / kSplMapThreads, n), kSplMapThreads, 0, stream>>>(dfields + off);
             }
-            spline_levels_kernel<<<nfields, kSplThreads, 0, stream>>>(dfields);
+            spline_levels_kernel<<<nfields, kSplChunks, 0, stream>>>(dfields);
+            for (int off = 0; off < nfields; off += 65535) {
+                const unsigned n = (unsigned)(nfields - off < 65535 ? nfields - off : 65535);
+                spline_maps_kernel<true><<<dim3(kSplChunks / kSplMapThreads, n), kSplMapThreads, 0, stream>>>(dfields + off);
+            }
         }
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;

@@ -52,25 +52,18 @@ struct SplCtl {
 constexpr int kSplCtlDoubles = 4;
 constexpr int kSplKeep = 12288;  // values of a bracket kept (4.2 % of a PAL field's)
 
-// IIR groups: the pixels before the first 32-pixel place of the output, then 32 each.
-__host__ __device__ inline long long spline_level_groups(int outwidth, int lineoffset, int linesout) {
-    const long long head = (long long)outwidth * (lineoffset + 1);
-    return head / 32 + ((long long)linesout * outwidth + 31) / 32 + 1;
-}
+constexpr int kSplChunks = 1024;  // of a field's pixels in the level-adjust IIR, a thread each
 
 // Doubles of scratch a spline field needs.
-inline size_t spline_scratch_doubles(int nlines, int outwidth, int lineoffset, int linesout, bool smooth) {
+inline size_t spline_scratch_doubles(int nlines, int outwidth, int linesout, bool smooth) {
     size_t n = (size_t)kSplStride * nlines + 2 + kSplCtlDoubles + kSplKeep;
     if (smooth)
-        n += ((size_t)linesout * outwidth + 31) / 32 + (size_t)spline_level_groups(outwidth, lineoffset, linesout);
+        n += ((size_t)linesout * outwidth + 31) / 32 + 2 * kSplChunks;  // levels; the chunks' maps and levels before
     return n;
 }
 
 __device__ __forceinline__ SplCtl* spline_ctl(const TbcField& f) { return reinterpret_cast<SplCtl*>(f.stat + 2); }
 __device__ __forceinline__ double* spline_kept(const TbcField& f) { return f.stat + 2 + kSplCtlDoubles; }
-__device__ __forceinline__ long long spline_level_groups(const TbcField& f) {
-    return spline_level_groups(f.outwidth, f.lineoffset, f.linesout);
-}
 __device__ __forceinline__ double* spline_maps(const TbcField& f) {
     return f.ybefore + ((size_t)f.linesout * f.outwidth + 31) / 32;
 }
