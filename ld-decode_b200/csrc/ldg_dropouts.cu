@@ -3,10 +3,11 @@
 //
 //  1. dropout_std_kernel   one CTA per 4096 samples: sum and squared
 //     deviations of rfhpf (nb_std, core.py:2836) about the CTA's own mean,
-//     FP64 (merged later by the pairwise update of Chan, Golub and LeVeque:
-//     the mean squared deviation numba forms in another order, ~1e-13
-//     relative by dropout_merge_kernel); one more CTA per field for the sync areas of every line
-//     l >= 1 (core.py:2867-2873): whole lines for the vertical-sync lines,
+//     FP64, merged by dropout_merge_kernel with the pairwise update of Chan,
+//     Golub and LeVeque (the mean squared deviation numba forms in another
+//     order; its error measured 7.6e-17, 1.1e-16 before); one more CTA per field
+//     for the sync areas of every line l >= 1 (core.py:2867-2873): whole
+//     lines for the vertical-sync lines,
 //     otherwise the first hsync_len samples; Python slice bounds, then a
 //     prefix maximum of the area ends so that "inside any area" is one
 //     search.
