@@ -111,4 +111,5 @@ def detect_host_field(rf, data, linelocs, lineoffset, linecount, isfirst, hsync_
     ll = torch.from_numpy(np.ascontiguousarray(linelocs, np.float64)).to(dev)
     d = _field(t["demod"].data_ptr(), t["demod_05"].data_ptr(), t["demod_raw"].data_ptr(), t["rfhpf"].data_ptr(),
                t["demod"].numel(), ll.data_ptr(), ll.numel(), lineoffset, linecount, isfirst, hsync_len)
-    return run(rf, [d], **kw)[0]
+    # on the stream that run() allocates on and reads its results from
+    return run(rf, [d], **{"stream": torch.cuda.current_stream(dev).cuda_stream, **kw})[0]

@@ -527,9 +527,11 @@ class LineLocator:
         U = rf.blocklen - rf.blockcut - rf.blockcut_end
         nblocks = n // U
         dev = torch.device("cuda", torch.cuda.current_device())
+        # the library works on the stream of this call's tensors
+        stream = torch.cuda.current_stream(dev).cuda_stream
         arrays = device_columns(v, keys, dev)
         self.begin(arrays)
-        runs = self.sync_runs(arrays["demod_05"].data_ptr(), n)
+        runs = self.sync_runs(arrays["demod_05"].data_ptr(), n, stream)
         prev = field.prevfield if getattr(field.prevfield, "valid", False) else None
         st = L.ChainState()
         st.start = float(rf.blockcut)  # the read window at the first block of the data
@@ -561,7 +563,7 @@ class LineLocator:
         elif prev is not None:
             pam_host = float(prev.phase_adjust_median)
         ll2 = None if self.pal else torch.empty((1, L.LDG_CHAIN_MAX_LINES), dtype=torch.float64, device=dev)
-        ll, bad, pam, fph, _ = self._refine(self._ptrs, n, valid, pam_host, None, linelocs2=ll2)
+        ll, bad, pam, fph, _ = self._refine(self._ptrs, n, valid, pam_host, stream, linelocs2=ll2)
         torch.cuda.synchronize()
         nl = self.proclines
         field.linelocs1 = np.array(p.linelocs1[:nl], dtype=np.float64)

@@ -70,7 +70,7 @@ def rf_tbc_host_field(rf, inp, linelocs, lineoffset, linecount, delay=None):
     ll = line_samples(rf)
     out = torch.empty(int(linecount) * ll, dtype=torch.int16, device=dev)
     run(rf, [descriptor(rf, ti.data_ptr(), ti.numel(), tl.data_ptr(), tl.numel(), lineoffset, linecount,
-                        out.data_ptr(), delay)])
+                        out.data_ptr(), delay)], torch.cuda.current_stream(dev).cuda_stream)  # `out` is read there
     res = out.cpu().numpy()
     tbc_status(rf)
     return res

@@ -108,3 +108,61 @@ def test_video_columns_cross_as_they_are(cuda_ok, form):
         for k in keys:
             np.testing.assert_array_equal(got[k].cpu().numpy(), cols[k])
             assert got[k].is_contiguous() and got[k].dtype == torch.float32
+
+
+@pytest.mark.parametrize("system", ["NTSC", "PAL"])
+def test_field_on_a_side_stream_equals_default(cuda_ok, system):
+    """A field's calls inside torch.cuda.stream(s), with s and the default
+    stream busy as each begins: the results of the default stream alone, and
+    the same for a second field's data in the memory the first one left."""
+    import torch
+    from ldgpu import RFDecode
+    from ldgpu.field import FieldNTSC, FieldPAL
+    from ldgpu.fieldread import field_window
+    from ldgpu.synth import inject_dropouts, synth_capture
+    rf = RFDecode(system=system, decode_analog_audio=44100)
+    U = rf.blocklen - rf.blockcut - rf.blockcut_end
+    w = field_window(rf, 0.0)
+    keys = ["demod", "demod_raw", "demod_05", "demod_burst"] + (["demod_pilot"] if system == "PAL" else [])
+    reads = []
+    for seed in (11, 12):
+        frame = 1_334_666 if system == "NTSC" else 1_600_000
+        cap = synth_capture(system, (w.nblocks - 1) * U + rf.blocklen, seed=seed, start=frame - 30_000 - 911 * seed).numpy()
+        inject_dropouts(cap, seed, 6)
+        dcap = torch.from_numpy(cap).cuda()
+        outs = {k: torch.empty(w.nblocks * U, dtype=torch.float32, device="cuda") for k in keys + ["rfhpf"]}
+        torch.cuda.synchronize()
+        rf.demod_blocks_device(dcap.data_ptr(), w.nblocks, U, {k: v.data_ptr() for k, v in outs.items()}, mtf_level=1)
+        rf.synchronize()
+        host = {k: v.cpu().numpy() for k, v in outs.items()}
+        reads.append({"video": np.rec.fromarrays([host[k] for k in keys], names=keys), "rfhpf": host["rfhpf"],
+                      "input": cap[rf.blockcut:rf.blockcut + w.length], "startloc": w.startloc})
+    cls = FieldPAL if system == "PAL" else FieldNTSC
+
+    def decode(read, before):
+        f = cls(rf, read, initphase=True, readloc=w.readloc)
+        before()
+        f.process()
+        assert f.valid
+        before()
+        pic = f.downscale(linesout=f.outlinecount, final=True)[0]
+        before()
+        drops = f.dropout_detect()
+        before()
+        return [np.asarray(f.linelocs), np.asarray(f.linebad), [f.isFirstField, f.fieldPhaseID, f.linecount], pic,
+                *map(np.asarray, drops), f.rf_tbc()]
+
+    def busy():
+        torch.cuda._sleep(4_000_000)  # a few ms of this stream
+        with torch.cuda.stream(torch.cuda.default_stream()):
+            torch.cuda._sleep(8_000_000)
+
+    want = [decode(r, lambda: None) for r in reads]
+    assert len(want[0][4]) > 0
+    with torch.cuda.stream(torch.cuda.Stream()):
+        got = [decode(r, busy) for r in reads]
+    torch.cuda.synchronize()
+    for a, b in zip(want, got):
+        for x, y in zip(a, b):
+            np.testing.assert_array_equal(x, y)
+    rf.close()
