@@ -435,11 +435,11 @@ def device_columns(v, keys, device):
     import torch
     fields = getattr(getattr(v, "dtype", None), "fields", None)
     if (len(keys) > 1 and fields and v.ndim == 1 and v.flags.c_contiguous and v.flags.writeable
-            and v.dtype.itemsize == 4 * len(fields) and all(f[0] == np.float32 for f in fields.values())):
-        names = sorted(fields, key=lambda k: fields[k][1])
-        host = v.view(np.ndarray).view(np.float32).reshape(len(v), len(names))
+            and v.dtype.itemsize == 4 * len(fields)
+            and all(f[0] == np.float32 and f[1] % 4 == 0 for f in fields.values())):
+        host = v.view(np.ndarray).view(np.float32).reshape(len(v), len(fields))
         whole = torch.from_numpy(host).to(device)
-        cols = {k: whole[:, names.index(k)].contiguous() for k in keys}
+        cols = {k: whole[:, fields[k][1] // 4].contiguous() for k in keys}
         torch.cuda.current_stream(device).synchronize()  # the library's stream need not be torch's current one
         return cols
     return {k: torch.from_numpy(np.ascontiguousarray(v[k], dtype=np.float32)).to(device) for k in keys}

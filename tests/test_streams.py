@@ -97,3 +97,15 @@ def test_process_field_scans_and_refines_on_the_callers_stream(on_cpu, monkeypat
     with pytest.raises(Seen):
         loc.process_field(f)
     assert got == [0x5150, 0x5150]
+
+
+@pytest.mark.parametrize("offsets", [(0, 4), (4, 0), (0, 0), (4, 4), (0, 2), (0, 3)])
+def test_columns_are_found_by_their_offset(log, offsets):
+    """Records whose fields share bytes, or lie off a multiple of four."""
+    import torch
+    from ldgpu.lines import device_columns
+    dt = np.dtype({"names": ["demod", "demod_05"], "formats": [np.float32] * 2, "offsets": offsets, "itemsize": 8})
+    v = np.frombuffer(bytearray(np.arange(40, dtype=np.float32).tobytes()), dt)
+    got = device_columns(v, ("demod", "demod_05"), torch.device("cpu"))
+    for k in dt.names:
+        assert got[k].numpy().tobytes() == np.ascontiguousarray(v[k]).tobytes(), k
