@@ -199,11 +199,18 @@ class FieldLogic:
     def line_areas(self, lines, begin, length):
         """The demodulated video of lineslice(l, begin, length) for each l of
         `lines`: (areas, rest), areas a list of (positions in `lines`, samples
-        as one float32 row per line) by slice length, rest the positions whose
-        slice does not lie inside the read (its bounds then follow Python's
-        slice rules, line by line)."""
+        as one row per line) by slice length, rest the positions to take line
+        by line: those whose slice does not lie inside the read (its bounds
+        then follow Python's slice rules), and all of them when a step of the
+        slicing is replaced (a subclass, an instance, a patched class) or the
+        locations are not FP64 or the samples not a plain array, whose
+        arithmetic is their own."""
         lines = np.asarray(lines)
-        ll = np.asarray(self.linelocs, dtype=np.float64)
+        ll = np.asarray(self.linelocs)
+        demod = self.data["video"]["demod"]
+        if not (self._steps_are(_SLICE_STEPS) and ll.dtype == np.float64 and isinstance(demod, np.ndarray)
+                and not isinstance(demod, np.ma.MaskedArray)):
+            return [], np.arange(len(lines))
         l_adj = lines + self.lineoffset
         inner = (l_adj > 0) & (l_adj + 1 < len(ll))
         k = np.where(inner, l_adj, 1)
@@ -212,7 +219,6 @@ class FieldLogic:
         linelen = np.where(linelen <= 0, float(self.rf.linelen), linelen)
         b = ll[k] + begin * (self.rf.samplesperline * linelen)
         e = b + length * (self.rf.samplesperline * self.rf.linelen) + 1
-        demod = self.data["video"]["demod"]
         ok = inner & (b >= 0) & (e < len(demod) + 1)  # (not for a location that is no number)
         lo, hi = np.where(ok, b, 0).astype(np.int64), np.where(ok, e, 0).astype(np.int64)
         areas = []
@@ -220,6 +226,10 @@ class FieldLogic:
             rows = np.nonzero(ok & (hi - lo == m))[0]
             areas.append((rows, demod[lo[rows][:, None] + np.arange(m)]))
         return areas, np.nonzero(~ok)[0]
+
+    def _steps_are(self, steps):
+        """Are this object's methods the ones of `steps` (name, function)?"""
+        return all(getattr(type(self), n) is f and n not in self.__dict__ for n, f in steps)
 
     def usectooutpx(self, x):
         return x * self.rf.SysParams["outfreq"]
@@ -849,8 +859,10 @@ class FieldLogicNTSC(FieldLogic):
         return adj_ll
 
     def calc_burstmedian(self):
-        # get_burstlevel of every line at once (a row's sums are numpy's of the line alone)
         lines = range(11, 264)
+        if not self._steps_are(_LEVEL_STEPS[0]):
+            return np.median([self.get_burstlevel(l) for l in lines]) / self.rf.DecoderParams["hz_ire"]
+        # get_burstlevel of every line at once (a row's sums are numpy's of the line alone)
         levels = np.empty(len(lines))
         areas, rest = self.line_areas(lines, 5.5, 2.4)
         for rows, a in areas:
@@ -921,7 +933,7 @@ class FieldLogicPAL(FieldLogic):
         # get_burstlevel of every line at once (a row's sums are numpy's of the line alone)
         lines = range(11, 313)
         levels = [None] * len(lines)
-        areas, rest = self.line_areas(lines, 5.5, 2.4)
+        areas, rest = self.line_areas(lines, 5.5, 2.4) if self._steps_are(_LEVEL_STEPS[1]) else ([], range(len(lines)))
         for rows, a in areas:
             a = a.astype(np.float32)
             a -= np.mean(a.astype(np.float64), axis=1).astype(np.float32)[:, None]
@@ -993,3 +1005,8 @@ class FieldLogicPAL(FieldLogic):
         self.lineoffset = 2 if self.isFirstField else 3
         self.linecode = [self.decodephillipscode(l + self.lineoffset) for l in (16, 17, 18)]
         self.fieldPhaseID = self.determine_field_number()
+
+
+# the functions that line_areas and calc_burstmedian stand for
+_SLICE_STEPS = [(n, getattr(FieldLogic, n)) for n in ("lineslice", "usectoinpx", "get_linefreq", "get_linelen")]
+_LEVEL_STEPS = [[("get_burstlevel", c.get_burstlevel)] for c in (FieldLogicNTSC, FieldLogicPAL)]

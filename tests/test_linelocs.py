@@ -171,3 +171,77 @@ def test_burst_median_equals_line_by_line(system, odd):
         assert len(levels) > 100
         want = np.median(levels) / rf.DecoderParams["hz_ire"]
         assert np.array_equal(f.calc_burstmedian(), want, equal_nan=True)
+
+
+def _burst_field(system, cls=None):
+    rf = RFParams(system=system)
+    cls = cls or (FieldLogicPAL if system == "PAL" else FieldLogicNTSC)
+    rng = np.random.default_rng(3)
+    f = cls.__new__(cls)
+    f.rf, f.linecount, f.lineoffset = rf, 262, 0
+    f.linelocs = 900.0 + 2550.3 * np.arange(326) + rng.normal(size=326) * 5
+    x = (rf.DecoderParams["ire0"] + rng.normal(0, 8e4, int(f.linelocs[-1]) + 3000)).astype(np.float32)
+    f.data = {"video": {"demod": x}}
+    return f
+
+
+def _line_by_line(f, system):
+    levels = [f.get_burstlevel(l) for l in (range(11, 313) if system == "PAL" else range(11, 264))]
+    return np.median([v for v in levels if v is not None]) / f.rf.DecoderParams["hz_ire"]
+
+
+@pytest.mark.parametrize("system", ["NTSC", "PAL"])
+@pytest.mark.parametrize("step", ["get_burstlevel", "lineslice", "usectoinpx", "get_linefreq", "get_linelen"])
+@pytest.mark.parametrize("how", ["subclass", "object", "class"])
+def test_burst_median_takes_replaced_steps(system, step, how, monkeypatch):
+    """A get_burstlevel, or a step of its slicing, that a subclass, an object
+    or a patch of the class replaces is the one calc_burstmedian uses."""
+    cls = FieldLogicPAL if system == "PAL" else FieldLogicNTSC
+    own = getattr(cls, step)
+
+    def replaced(self, *args, **kwargs):
+        r = own(self, *args, **kwargs)
+        if r is None:  # PAL: a sample above 30 IRE
+            return None
+        return slice(r.start + 40, r.stop + 70) if step == "lineslice" else r * 1.5
+
+    plain = _line_by_line(_burst_field(system), system)
+    if how == "subclass":
+        f = _burst_field(system, type("Sub", (cls,), {step: replaced}))
+    else:
+        f = _burst_field(system)
+        if how == "object":
+            setattr(f, step, replaced.__get__(f))
+        else:
+            monkeypatch.setattr(cls, step, replaced)
+    want = _line_by_line(f, system)
+    assert want != plain
+    assert f.calc_burstmedian() == want
+
+
+@pytest.mark.parametrize("system", ["NTSC", "PAL"])
+@pytest.mark.parametrize("form", ["float32 locations", "location list", "whole locations", "masked samples",
+                                  "float64 samples"])
+def test_burst_median_forms(system, form):
+    """Other types of line locations and samples: the bits of line by line."""
+    f = _burst_field(system)
+    v = f.data["video"]
+    if form == "float32 locations":
+        f.linelocs = f.linelocs.astype(np.float32)
+    elif form == "location list":
+        f.linelocs = f.linelocs.tolist()
+    elif form == "whole locations":
+        f.linelocs = f.linelocs.astype(np.int64)
+    elif form == "masked samples":
+        v["demod"] = np.ma.masked_array(v["demod"], np.arange(len(v["demod"])) % 7 == 0)
+    else:
+        v["demod"] = v["demod"].astype(np.float64) + 1e-3
+    assert f.calc_burstmedian() == _line_by_line(f, system)
+
+
+def test_burst_median_of_a_tensor():
+    import torch
+    f = _burst_field("NTSC")
+    want = _line_by_line(f, "NTSC")
+    f.data["video"]["demod"] = torch.from_numpy(f.data["video"]["demod"])
+    assert f.calc_burstmedian() == want
