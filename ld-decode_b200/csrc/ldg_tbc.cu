@@ -452,9 +452,10 @@ __device__ double select_mean(Visit visit, long long n, long long r1, bool two, 
 // and kernels of kSplSlices CTAs per field that walk its pixels:
 //   spline_build    the pieces; a bracket for the median from kSplSamples
 //                   pixels at even steps
-//   spline_pass     counts the wow factors below the bracket, keeps those in it
-//   spline_median   the median, exactly, from those (their number below tells
-//                   which rank to take); a bracket for the MAD
+//   spline_pass     counts the wow factors below the bracket and at its ends,
+//                   keeps those between
+//   spline_median   the median, exactly, from those (the counts tell which rank
+//                   to take, or that it is an end); a bracket for the MAD
 //   spline_pass     the same for |wow - median|
 //   spline_mad      the MAD
 //   spline_maps / spline_levels / spline_maps   (smoothing) the IIR over each
@@ -462,8 +463,12 @@ __device__ double select_mean(Visit visit, long long n, long long r1, bool two, 
 // A bracket's ranks lie kSplMargin samples either side of the median's: the
 // factors are smooth along a line, so an evenly stepped sample misjudges a
 // rank by about one sample per crossing and square root of the crossings, ~10
-// of 4096.  Where it fails all the same (or keeps too many), the CTA selects
-// from all pixels by radix passes.
+// of 4096.  Evenly spaced lines make most factors equal, and such a value is
+// an end of its bracket: counted, however often it occurs (60 evenly spaced
+// NTSC fields, cubic, smoothing: 588 us the whole call; 1204 by one CTA per
+// field, 1320 with every such value kept until none fitted).  Where a bracket
+// fails all the same (or keeps too many), the CTA selects from all pixels by
+// radix passes.
 // Bound: instruction issue of the walks (FP64 pipe next).  As one CTA per
 // field walking all pixels up to ten times: 672 us for 60 NTSC fields (cubic,
 // smoothing; as long for one); the eight launches together 250 us (ncu: build
@@ -509,27 +514,41 @@ __device__ void find_bracket(Value value, long long L, double* samp, unsigned* h
         ctl->hi = hi;
         ctl->below = 0;
         ctl->kept = 0;
+        ctl->at_lo = 0;
+        ctl->at_hi = 0;
     }
 }
 
-// The median of all L values from what the pass kept, or (kept too few or too
-// many) from all of them, all(i0, i1, body) visiting them in order.
+// The median of all L values from what the pass counted and kept, or (kept too
+// many, or the median outside the bracket) from all of them, all(i0, i1, body)
+// visiting them in order.  `signs`: zeros of both signs occur, whose order at a
+// bracket's end is not known from a count.
 template <class All>
-__device__ double bracket_median(const TbcField& f, All all, long long L, unsigned* hist, SelectShared& sh) {
+__device__ double bracket_median(const TbcField& f, All all, long long L, bool signs, unsigned* hist, SelectShared& sh) {
     const SplCtl* ctl = spline_ctl(f);
+    const bool two = !(L & 1);
     const long long r1 = median_rank(L), r2 = L / 2;
+    const double lo = ctl->lo, hi = ctl->hi;
     const long long below = ctl->below, kept = ctl->kept;
-    const bool usable = ctl->lo <= ctl->hi && kept <= kSplKeep && r1 >= below && r2 < below + kept;
+    // ranks: below the bracket, its low end, what was kept, its high end
+    const long long n1 = below + ctl->at_lo, n2 = n1 + kept, n3 = n2 + ctl->at_hi;
+    const bool usable = lo <= hi && kept <= kSplKeep && r1 >= below && r2 < n3 && !(signs && (lo == 0 || hi == 0));
     __syncthreads();
-    if (usable) {
-        const double* v = spline_kept(f);
-        return select_mean(
+    if (!usable) return select_mean(all, L, r1, two, hist, sh);
+    const bool in1 = r1 >= n1 && r1 < n2, in2 = r2 >= n1 && r2 < n2;
+    double v = 0.0;
+    if (in1 || in2) {
+        const double* k = spline_kept(f);
+        v = select_mean(
             [&](long long a0, long long a1, auto body) {
-                for (long long i = a0; i < a1; ++i) body(i, order_key(v[i]));
+                for (long long i = a0; i < a1; ++i) body(i, order_key(k[i]));
             },
-            kept, r1 - below, !(L & 1), hist, sh);
+            kept, (in1 ? r1 : r2) - n1, in1 && in2 && two, hist, sh);
+        if (in1 && in2) return v;
     }
-    return select_mean(all, L, r1, !(L & 1), hist, sh);
+    const double v1 = in1 ? v : r1 < n1 ? lo : hi;
+    const double v2 = in2 ? v : r2 < n1 ? lo : hi;
+    return two ? __dadd_rn(v1, v2) / 2 : v1;
 }
 
 __device__ __forceinline__ WowWalk field_walk(const TbcField& f) {
@@ -657,8 +676,8 @@ __global__ void __launch_bounds__(kSplThreads) spline_build_kernel(const TbcFiel
     find_bracket([&](long long i) { return wow_at(f, i); }, f.nwow, mem, reinterpret_cast<unsigned*>(hist_mem), sh, ctl);
 }
 
-// One slice of a field's pixels against the bracket: how many lie below it,
-// and the values inside it (in no order).
+// One slice of a field's pixels against the bracket: how many lie below it and
+// at its ends, and the values between (in no order).
 template <bool Mad>
 __global__ void __launch_bounds__(kSplPassThreads) spline_pass_kernel(const TbcField* fields) {
     const TbcField& f = fields[blockIdx.y];
@@ -668,31 +687,47 @@ __global__ void __launch_bounds__(kSplPassThreads) spline_pass_kernel(const TbcF
     constexpr int kHold = 2048;
     __shared__ double held[kHold];
     __shared__ int s_n, s_at;
+    __shared__ volatile int s_full;  // more kept than the field's scratch holds: the bracket is of no use
     const int t = threadIdx.x;
-    if (t == 0) s_n = 0;
+    if (t == 0) s_n = s_full = 0;
     __syncthreads();
     const double lo = ctl->lo, hi = ctl->hi, med = Mad ? f.stat[0] : 0.0;
     double* kept = spline_kept(f);
     const long long L = f.nwow;
     const long long per = (L + kSplSlices * kSplPassThreads - 1) / (kSplSlices * kSplPassThreads);
     const long long i0 = ((long long)blockIdx.x * kSplPassThreads + t) * per, i1 = min(L, i0 + per);
-    int below = 0;
+    int below = 0, at_lo = 0, at_hi = 0;
     field_walk(f)(i0, i1, [&](long long, double w) {
         const double v = Mad ? fabs(__dadd_rn(w, -med)) : w;
-        below += v < lo;
-        if (v >= lo && v <= hi) {
-            const int at = atomicAdd(&s_n, 1);
-            if (at < kHold) {
-                held[at] = v;
+        const bool less = v < lo;
+        below += less;
+        if (!less && v <= hi) {
+            if (v == lo) {
+                ++at_lo;
+            } else if (v == hi) {
+                ++at_hi;
             } else {
-                const int g = atomicAdd(&ctl->kept, 1);
-                if (g < kSplKeep) kept[g] = v;
+                const int at = atomicAdd(&s_n, 1);
+                if (at < kHold) {
+                    held[at] = v;
+                } else if (!s_full) {
+                    const int g = atomicAdd(&ctl->kept, 1);
+                    if (g < kSplKeep) kept[g] = v; else s_full = 1;
+                }
             }
         }
     });
 #pragma unroll
-    for (int o = 16; o; o >>= 1) below += __shfl_xor_sync(0xffffffffu, below, o);
-    if ((t & 31) == 0 && below) atomicAdd(&ctl->below, below);
+    for (int o = 16; o; o >>= 1) {
+        below += __shfl_xor_sync(0xffffffffu, below, o);
+        at_lo += __shfl_xor_sync(0xffffffffu, at_lo, o);
+        at_hi += __shfl_xor_sync(0xffffffffu, at_hi, o);
+    }
+    if ((t & 31) == 0) {
+        if (below) atomicAdd(&ctl->below, below);
+        if (at_lo) atomicAdd(&ctl->at_lo, at_lo);
+        if (at_hi) atomicAdd(&ctl->at_hi, at_hi);
+    }
     __syncthreads();
     const int n = min(s_n, kHold);
     if (t == 0) s_at = n ? atomicAdd(&ctl->kept, n) : 0;
@@ -714,7 +749,7 @@ __global__ void __launch_bounds__(kSplThreads) spline_median_kernel(const TbcFie
         [&](long long a0, long long a1, auto body) {
             walk(a0, a1, [&](long long i, double w) { body(i, order_key(w)); });
         },
-        f.nwow, hist, sh);
+        f.nwow, true, hist, sh);
     if (threadIdx.x == 0) f.stat[0] = med;
     __syncthreads();
     find_bracket([&](long long i) { return fabs(__dadd_rn(wow_at(f, i), -med)); }, f.nwow, samp, hist, sh,
@@ -733,7 +768,7 @@ __global__ void __launch_bounds__(kSplThreads) spline_mad_kernel(const TbcField*
         [&](long long a0, long long a1, auto body) {
             walk(a0, a1, [&](long long i, double w) { body(i, order_key(fabs(__dadd_rn(w, -med)))); });
         },
-        f.nwow, reinterpret_cast<unsigned*>(hist_mem), sh);
+        f.nwow, false, reinterpret_cast<unsigned*>(hist_mem), sh);
     if (threadIdx.x == 0) f.stat[1] = mad > 0 ? threshold_mult * mad : 0.001;
 }
 

@@ -350,3 +350,78 @@ def test_spline_statistics_extremes(cuda_ok, method, shape, outl, smoothing):
                                 smoothing=smoothing)
         assert np.abs(out.cpu().numpy().astype(np.float64) - want).max() < 2.0, lineoffset
     rf.close()
+
+
+@pytest.mark.parametrize("method", ["quadratic", "cubic"])
+@pytest.mark.parametrize("outw", [910, 911])
+def test_spline_statistics_plateaus(cuda_ok, method, outw):
+    """Fields of two line lengths and some irregular lines, the change so
+    placed that the median falls into either plateau, onto the edge between
+    one and the factors beside it, or between them: the ends of its bracket,
+    and of the deviations' one, are values that many pixels share.  Neither
+    plateau holds half of the pixels, so the MAD is their distance and the
+    outlier rule's limit far from rounding; the displaced line takes the median
+    as its level, 2200 Hz apart between the plateaus.  Against the oracle;
+    tolerance as in test_spline_statistics_extremes."""
+    import torch
+    from ldgpu import RFDecode
+    from ldgpu.field import tbc_descriptor, tbc_fields
+    rf = RFDecode(system="NTSC")
+    outl, nlines, n = 263, 273, 700_000
+    buf = (8.0e6 + 1.0e5 * np.sin(np.arange(n) * 0.01)).astype(np.float32)
+    dbuf = torch.from_numpy(buf).cuda()
+    levels = (rf.DecoderParams["ire0"], rf.DecoderParams["hz_ire"], rf.DecoderParams["vsync_ire"], 300.0, 1024.0)
+    lls, outs, descs = [], [], []
+    rng = np.random.default_rng(outw)
+    irregular = np.sign(np.arange(50) % 2 - 0.5) * rng.uniform(1.0, 3.0, 50)
+    for lineoffset, first in [(0, c) for c in (90, 100, 103, 104, 105, 106, 107, 108, 109, 112, 120)] + [(1, 106)]:
+        step = np.full(nlines, float(rf.linelen))
+        step[:50] += irregular
+        step[50 + first:] += 0.7
+        ll = 300.0 + np.cumsum(step) - step[0]
+        ll[30] += 40.0
+        lls.append((lineoffset, ll, torch.from_numpy(ll).cuda()))
+        outs.append(torch.zeros(outl * outw, dtype=torch.float32, device="cuda"))
+        d = tbc_descriptor(rf, dbuf.data_ptr(), lls[-1][2].data_ptr(), lineoffset, outw, outl, outl, levels,
+                           out_f32=outs[-1].data_ptr(), buf_len=n, nlines=nlines, wow_interpolation_method=method)
+        d.outlinelen = float(outw)
+        descs.append(d)
+    torch.cuda.synchronize()
+    tbc_fields(rf, descs)
+    for (lineoffset, ll, _), out in zip(lls, outs):
+        coords, wow = otbc.pixel_coords(ll, rf.linelen, outw, outl, lineoffset, method=method)
+        want = otbc.scale_field(buf, coords, wow, rf.downscale_sinc_lut, lineoffset, outw, outl * outw)
+        assert np.abs(out.cpu().numpy().astype(np.float64) - want).max() < 2.0, (lineoffset, int(ll[-1]))
+    rf.close()
+
+
+@pytest.mark.parametrize("method", ["quadratic", "cubic"])
+def test_spline_regular_lines_take_no_longer(cuda_ok, method):
+    """Evenly spaced lines, whose wow factors are all alike, go through the
+    same few launches as lines with jitter (205 against 169 us a field; 905
+    when every factor was kept until they no longer fitted)."""
+    import torch
+    from ldgpu import RFDecode
+    from ldgpu.field import tbc_descriptor, tbc_fields
+    rf = RFDecode(system="NTSC")
+    outl, outw, nlines, n = 263, 910, 273, 700_000
+    buf = torch.full((n,), 8.0e6, device="cuda")
+    out = torch.zeros(outl * outw, dtype=torch.float32, device="cuda")
+    levels = (rf.DecoderParams["ire0"], rf.DecoderParams["hz_ire"], rf.DecoderParams["vsync_ire"], 300.0, 1024.0)
+    even = 300.0 + float(rf.linelen) * np.arange(nlines)
+    took = []
+    for ll in (even, even + np.random.default_rng(1).normal(size=nlines) * 0.05):
+        dll = torch.from_numpy(ll).cuda()
+        d = tbc_descriptor(rf, buf.data_ptr(), dll.data_ptr(), 0, outw, outl, outl, levels, out_f32=out.data_ptr(),
+                           buf_len=n, nlines=nlines, wow_interpolation_method=method)
+        times = []
+        for _ in range(25):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            tbc_fields(rf, [d])
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        took.append(float(np.median(times)))
+    assert took[0] < 2.5 * took[1], took
+    rf.close()
