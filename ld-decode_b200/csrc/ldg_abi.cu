@@ -520,8 +520,6 @@ int ldg_demod_blocks(ldg_ctx* c, const ldg_demod_args* a) {
     const int grid = (int)((nb + per_cta - 1) / per_cta);
     int rc = grow((void**)&c->d_scratch, &c->scratch_bytes, (size_t)nslots * ldg::kScratchPerCta);
     if (rc) return rc;
-    // a small batch: several CTAs per block, unless blocks per CTA are set
-    const int split = c->blocks_per_cta ? 1 : ldg::demod_split(c->variant, nb, c->scratch_bytes);
     if (!c->d_slots) {
         LDG_CK(cudaMalloc(&c->d_slots, (nslots + 1) * sizeof(int)));
         LDG_CK(cudaMemset(c->d_slots, 0, (nslots + 1) * sizeof(int)));
@@ -568,6 +566,16 @@ int ldg_demod_blocks(ldg_ctx* c, const ldg_demod_args* a) {
         if (!bufs[i].user) return nullptr;
         return bufs[i].host ? (void*)(c->d_stage + bufs[i].off) : bufs[i].user;
     };
+    // a small batch: several CTAs per block, unless blocks per CTA are set, or an
+    // output that one of them writes while another may still read the block
+    // shares its memory (the video outputs come after all have read it)
+    auto over_input = [&](int i) {
+        const char *a = (const char*)dev(i), *b = (const char*)dev(i_in);
+        return a && a < b + bufs[i_in].bytes && b < a + bufs[i].bytes;
+    };
+    const int split = c->blocks_per_cta || over_input(i_hp) || over_input(i_efm) || over_input(i_al) || over_input(i_ar)
+                          ? 1
+                          : ldg::demod_split(c->variant, nb, c->scratch_bytes);
     // the kernel reads samples in pairs: 4-byte (int16) / 8-byte (float32) aligned block starts
     if ((a->in_stride & 1) != 0 || (reinterpret_cast<uintptr_t>(dev(i_in)) & (esz == 2 ? 3 : 7)) != 0)
         return fail(LDG_ERR_ARG, "ldg_demod_blocks: input blocks must start on an even sample of an aligned buffer");

@@ -291,3 +291,28 @@ def test_variants_agree(cuda_ok, system):
     finally:
         a.close()
         b.close()
+
+
+@pytest.mark.parametrize("which", ["rfhpf", "audio_left", "demod"])
+def test_one_block_over_its_input(rf, which):
+    """An output in the memory of its block's samples: the values it has in
+    memory of its own (the block is read whole before the output is written)."""
+    import torch
+    from ldgpu.lib import LDG_IN_FLOAT32
+    U = rf.blocklen - rf.blockcut - rf.blockcut_end
+    block = torch.from_numpy(np.random.default_rng(5).integers(-2000, 2000, rf.blocklen).astype(np.float32)).cuda()
+
+    def run(x, outs):
+        torch.cuda.synchronize()
+        rf.demod_blocks_device(x.data_ptr(), 1, U, {k: v.data_ptr() for k, v in outs.items()}, mtf_level=1,
+                               in_kind=LDG_IN_FLOAT32)
+        rf.synchronize()
+        return outs
+
+    want = run(block, _device_outputs(rf, 1))
+    for _ in range(20):
+        x, outs = block.clone(), _device_outputs(rf, 1)
+        outs[which] = x[2:2 + want[which].numel()]
+        got = run(x, outs)
+        for k in want:
+            assert torch.equal(got[k], want[k]), k
