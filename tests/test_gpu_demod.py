@@ -316,3 +316,32 @@ def test_one_block_over_its_input(rf, which):
         got = run(x, outs)
         for k in want:
             assert torch.equal(got[k], want[k]), k
+
+
+@pytest.mark.parametrize("variant", [0, 1], ids=["stockham", "inplace"])
+@pytest.mark.parametrize("kind", ["int16", "float32"])
+@pytest.mark.parametrize("notch", [False, True])
+def test_cluster_forms_equal_one_cta(cuda_ok, variant, kind, notch):
+    """Both sample types, with and without the PAL notch on 8.5 MHz carriers:
+    four and two CTAs per block give the bits of one CTA per block."""
+    import torch
+    from ldgpu import RFDecode
+    from ldgpu.lib import LDG_IN_FLOAT32, LDG_IN_INT16
+    rf = RFDecode(system="PAL", decode_analog_audio=44100, decode_digital_audio=True,
+                  extra_options={"PAL_V4300D_NotchFilter": notch}, fft_variant=variant)
+    U = rf.blocklen - rf.blockcut - rf.blockcut_end
+    for nb in (1, 40):
+        n = (nb - 1) * U + rf.blocklen
+        x = np.random.default_rng(nb).normal(0, 900, n) + 4000 * np.cos(2 * np.pi * 8.5 / 40 * np.arange(n))
+        cap = torch.from_numpy(x.astype(kind)).cuda()
+        out = []
+        for per_cta in (0, 1):
+            out.append(_device_outputs(rf, nb))
+            rf.blocks_per_cta = per_cta
+            torch.cuda.synchronize()
+            rf.demod_blocks_device(cap.data_ptr(), nb, U, {k: v.data_ptr() for k, v in out[-1].items()}, mtf_level=1,
+                                   in_kind=LDG_IN_INT16 if kind == "int16" else LDG_IN_FLOAT32)
+            rf.synchronize()
+        for k in out[0]:
+            assert torch.equal(out[0][k], out[1][k]), (k, nb)
+    rf.close()
