@@ -990,15 +990,17 @@ int ldg_dropouts(ldg_ctx* c, const ldg_dropout_params* p, const ldg_dropout_fiel
     int rc = grow((void**)&c->d_drop_fields, &c->drop_fields_cap, (size_t)nfields * sizeof(ldg::DropField));
     if (rc) return rc;
     long long max_len = 0;
-    for (int i = 0; i < nfields; ++i) max_len = std::max(max_len, (long long)fields[i].len);
-    rc = grow((void**)&c->d_drop_scratch, &c->drop_scratch_cap, ldg::dropout_scratch(nfields, max_len, nullptr, nullptr));
-    if (rc) return rc;
     std::vector<ldg::DropField> h(nfields);
     for (int i = 0; i < nfields; ++i) {
         const ldg_dropout_field& f = fields[i];
         h[i] = {f.demod, f.demod_05, f.demod_raw, f.rfhpf, f.len, f.linelocs, f.nlines, f.lineoffset, f.linecount,
-                f.isfirst, f.hsync_len};
+                f.isfirst, f.hsync_len, 0, 0};
+        max_len = std::max(max_len, (long long)f.len);
     }
+    rc = grow((void**)&c->d_drop_scratch, &c->drop_scratch_cap, ldg::dropout_scratch(h.data(), nfields, nullptr, nullptr));
+    if (rc) return rc;
+    ldg::DropScratch sc;
+    ldg::dropout_scratch(h.data(), nfields, c->d_drop_scratch, &sc);
     // pageable source: the copy has taken the data when the call returns
     LDG_CK(cudaMemcpyAsync(c->d_drop_fields, h.data(), h.size() * sizeof(ldg::DropField), cudaMemcpyHostToDevice, st));
     const bool pal = p->system == LDG_PAL;
@@ -1018,8 +1020,7 @@ int ldg_dropouts(ldg_ctx* c, const ldg_dropout_params* p, const ldg_dropout_fiel
     k.vmax05 = hz(115);
     k.smin = hz(pal ? p->vsync_ire - 60 : p->vsync_ire - 35);
     k.smin05 = hz(p->vsync_ire - 10);
-    cudaError_t e = ldg::launch_dropouts(c->d_drop_fields, nfields, max_len, k, c->d_drop_scratch, drops, counts,
-                                          rfstd, st);
+    cudaError_t e = ldg::launch_dropouts(c->d_drop_fields, nfields, max_len, k, sc, drops, counts, rfstd, st);
     if (e != cudaSuccess) return fail(LDG_ERR_CUDA, std::string("dropout launch: ") + cudaGetErrorString(e));
     LDG_CK(cudaEventRecord(c->drop_done, st));
     c->drop_used = true;

@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(kStdThreads, 5) dropout_std_kernel(const DropF
             m2 = fma(d, d, m2);
         }
         m2 = block_sum<kStdThreads>(m2, red);
-        if (t == 0) sc.part[(size_t)blockIdx.y * sc.tiles + blockIdx.x] = make_double2(s, m2);
+        if (t == 0) sc.part[f.tile0 + blockIdx.x] = make_double2(s, m2);
         return;
     }
     // the sync areas
@@ -332,7 +332,7 @@ __global__ void __launch_bounds__(128) dropout_merge_kernel(const DropField* fie
                                                             double* rfstd_out) {
     const int f = blockIdx.x * 4 + (threadIdx.x >> 5);
     if (f >= nfields) return;
-    const double sd = merge_std(sc.part + (size_t)f * sc.tiles, fields[f].len);
+    const double sd = merge_std(sc.part + fields[f].tile0, fields[f].len);
     if ((threadIdx.x & 31) == 0) {
         sc.rf_hi[f] = float_down(sd * 3.0);
         if (rfstd_out) rfstd_out[f] = sd;
@@ -389,7 +389,7 @@ __global__ void __launch_bounds__(kMaskThreads) dropout_mask_kernel(const DropFi
     // the area's end and the next one's start, as offsets
     int end = idx >= 0 ? pm[idx] - base : INT_MIN;
     int next = idx + 1 < nreg ? rs[idx + 1] - base : INT_MAX;
-    unsigned* words = sc.words + (size_t)blockIdx.y * sc.nwords + (i0 >> 5);
+    unsigned* words = sc.words + f.word0 + (i0 >> 5);
     constexpr int kBatch = 8;  // samples whose loads are in flight together
 #pragma unroll 1
     for (int j0 = 0; j0 < kMaskPer; j0 += kBatch) {
@@ -458,7 +458,7 @@ __global__ void __launch_bounds__(kPlaceThreads) dropout_place_kernel(const Drop
     const long long w0 = lo >> 5, nw = hi > lo ? ((hi + 31) >> 5) - w0 : 0;
     // the mask in shared memory when it fits (a field of 1.5 M samples does):
     // the searches below are chains of single-word reads
-    ErrorBits bits{sc.words + (size_t)blockIdx.x * sc.nwords, (int)hi};
+    ErrorBits bits{sc.words + f.word0, (int)hi};
     if (nw <= sc.place_words) {
 #pragma unroll 8
         for (int w = t; w < (int)nw; w += kPlaceThreads) swords[w] = bits.words[w0 + w];
@@ -595,44 +595,46 @@ __global__ void __launch_bounds__(kPlaceThreads) dropout_place_kernel(const Drop
     if (t == 0) counts[2 * blockIdx.x] = total > k.out_cap ? -1 : total;
 }
 
-size_t dropout_scratch(int nfields, long long max_len, char* base, DropScratch* sc) {
+size_t dropout_scratch(DropField* fields, int nfields, char* base, DropScratch* sc) {
     const size_t nf = (size_t)nfields;
+    size_t tiles = 0, words = 0;
+    for (int i = 0; i < nfields; ++i) {
+        fields[i].tile0 = (long long)tiles;
+        fields[i].word0 = (long long)words;
+        tiles += (size_t)((fields[i].len + kDropStdTile - 1) / kDropStdTile);
+        // whole mask tiles (32 words beyond a field's last sample are not written)
+        words += (size_t)((fields[i].len + kDropMaskTile - 1) / kDropMaskTile) * (kDropMaskTile / 32);
+    }
     DropScratch q;
-    q.tiles = (int)((max_len + kDropStdTile - 1) / kDropStdTile);
-    // whole mask tiles (32 words beyond a field's last sample are not written)
-    q.nwords = (max_len + kDropMaskTile - 1) / kDropMaskTile * (kDropMaskTile / 32);
     char* p = base;
     auto take = [&](size_t bytes) {
         char* r = p;
         p += (bytes + 255) & ~(size_t)255;
         return r;
     };
-    q.part = reinterpret_cast<double2*>(take(nf * q.tiles * sizeof(double2)));
+    q.part = reinterpret_cast<double2*>(take(tiles * sizeof(double2)));
     q.areas = reinterpret_cast<int2*>(take(nf * kMaxDropRegions * sizeof(int2)));
     q.bad = reinterpret_cast<int*>(take(nf * sizeof(int)));
     q.rf_hi = reinterpret_cast<float*>(take(nf * sizeof(float)));
-    q.words = reinterpret_cast<unsigned*>(take(nf * (size_t)q.nwords * sizeof(unsigned)));
+    q.words = reinterpret_cast<unsigned*>(take(words * sizeof(unsigned)));
     q.place_words = 0;
     if (sc) *sc = q;
     return (size_t)(p - base);
 }
 
-cudaError_t launch_dropouts(const DropField* fields, int nfields, long long max_len, const DropConsts& k, char* scratch,
-                            int* drops, int* counts, double* rfstd, cudaStream_t stream) {
+cudaError_t launch_dropouts(const DropField* fields, int nfields, long long max_len, const DropConsts& k,
+                            DropScratch sc, int* drops, int* counts, double* rfstd, cudaStream_t stream) {
     if (nfields <= 0) return cudaSuccess;
-    DropScratch sc;
-    dropout_scratch(nfields, max_len, scratch, &sc);
     sc.place_words = (int)std::min((long long)kPlaceWords, max_len / 32 + 2);
+    const unsigned std_tiles = (unsigned)((max_len + kDropStdTile - 1) / kDropStdTile);
     const unsigned mask_tiles = (unsigned)((max_len + kDropMaskTile - 1) / kDropMaskTile);
     for (int lo = 0; lo < nfields; lo += 65535) {  // grid.y limit
         const unsigned n = (unsigned)(nfields - lo < 65535 ? nfields - lo : 65535);
         DropScratch q = sc;
-        q.part += (size_t)lo * sc.tiles;
         q.areas += (size_t)lo * kMaxDropRegions;
         q.bad += lo;
         q.rf_hi += lo;
-        q.words += (size_t)lo * sc.nwords;
-        dropout_std_kernel<<<dim3((unsigned)sc.tiles + 1, n), kStdThreads, 0, stream>>>(fields + lo, k, q);
+        dropout_std_kernel<<<dim3(std_tiles + 1, n), kStdThreads, 0, stream>>>(fields + lo, k, q);
         dropout_merge_kernel<<<(n + 3) / 4, 128, 0, stream>>>(fields + lo, (int)n, q, rfstd ? rfstd + lo : nullptr);
         dropout_mask_kernel<<<dim3(mask_tiles, n), kMaskThreads, 0, stream>>>(fields + lo, k, q);
     }

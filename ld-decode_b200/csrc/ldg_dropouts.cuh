@@ -16,6 +16,7 @@ struct DropField {
     long long len;
     const double* ll;
     int nlines, lineoffset, linecount, isfirst, hsync_len;
+    long long tile0, word0;  // its first entries of DropScratch.part and .words
 };
 
 struct DropConsts {
@@ -26,22 +27,22 @@ struct DropConsts {
 
 // Device scratch of a call, per field: tiles' rfhpf sums and squared
 // deviations, sync areas (start, prefix maximum of the ends), a flag for areas
-// that cannot be built, the error mask.
+// that cannot be built, the error mask.  Tiles and mask words follow each
+// field's own length (one long read among short ones costs its own).
 struct DropScratch {
     double2* part;
     int2* areas;
     int* bad;
     float* rf_hi;       // the error limit of rfhpf (3 standard deviations)
     unsigned* words;
-    int tiles;          // entries of part per field
-    long long nwords;   // mask words per field
     int place_words;    // mask words the placement's shared memory holds
 };
 
-// Bytes of scratch for fields of up to max_len samples; with sc, its layout at base.
-size_t dropout_scratch(int nfields, long long max_len, char* base, DropScratch* sc);
+// Bytes of scratch for these fields, setting their tile0 and word0; with sc, its layout at base.
+size_t dropout_scratch(DropField* fields, int nfields, char* base, DropScratch* sc);
 
-cudaError_t launch_dropouts(const DropField* fields, int nfields, long long max_len, const DropConsts& k, char* scratch,
-                            int* drops, int* counts, double* rfstd, cudaStream_t stream);
+// scratch: as dropout_scratch laid it out; max_len: the longest field's samples.
+cudaError_t launch_dropouts(const DropField* fields, int nfields, long long max_len, const DropConsts& k,
+                            DropScratch sc, int* drops, int* counts, double* rfstd, cudaStream_t stream);
 
 }  // namespace ldg

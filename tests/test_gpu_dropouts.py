@@ -192,3 +192,35 @@ def test_reference_golden_fields(cuda_ok, system):
     print(system, "dropouts", total, "identical", same)
     assert total > 20
     rf.close()
+
+
+def test_one_long_read_among_short_ones(cuda_ok):
+    """The device scratch of a call follows each field's own length: a read of
+    48 M samples beside 400 of 40,000 (3 GB when every field took the
+    longest one's), with the lists of the fields on their own."""
+    import torch
+    from ldgpu import RFDecode
+    from ldgpu.dropouts import _field, run
+    rf = RFDecode(system="NTSC")
+    rng = np.random.default_rng(4)
+    n, short = 48_000_000, 40_000
+    x = torch.full((n,), float(rf.iretohz(20)), device="cuda")
+    for a in rng.integers(0, short, 12).tolist() + rng.integers(0, n - 900, 200).tolist():
+        x[a:a + 300] = 2e6
+    hp = torch.zeros(n, device="cuda")
+    ll = torch.from_numpy(1500.3 + 2542.2 * np.arange(14)).cuda()
+    wide = torch.from_numpy(1500.3 + 90_000.0 * np.arange(500)).cuda()
+
+    def field(m, lines):
+        return _field(x.data_ptr(), x.data_ptr(), x.data_ptr(), hp.data_ptr(), m, lines.data_ptr(), len(lines), 0,
+                      len(lines) - 3, True, 190)
+
+    alone = [run(rf, [field(short, ll)])[0], run(rf, [field(n, wide)])[0]]
+    assert len(alone[0][0]) > 2 and len(alone[1][0]) > 100
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    got = run(rf, [field(short, ll)] * 200 + [field(n, wide)] + [field(short, ll)] * 200)
+    assert free - torch.cuda.mem_get_info()[0] < 500e6
+    assert got == [alone[0]] * 200 + [alone[1]] + [alone[0]] * 200
+    rf.close()
