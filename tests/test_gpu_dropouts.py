@@ -224,3 +224,36 @@ def test_one_long_read_among_short_ones(cuda_ok):
     assert free - torch.cuda.mem_get_info()[0] < 500e6
     assert got == [alone[0]] * 200 + [alone[1]] + [alone[0]] * 200
     rf.close()
+
+
+def test_long_mask_equals_oracle(cuda_ok):
+    """A field whose lines span 1.75 M samples, more mask bits than the
+    placement keeps in shared memory, and a short one in the same call: the
+    oracle's lists exactly."""
+    import torch
+    from ldgpu import RFDecode
+    from ldgpu.dropouts import _field, run
+    rf = RFDecode(system="NTSC")
+    rng = np.random.default_rng(9)
+    lim = odrop.limits(rf.system, rf.DecoderParams["ire0"], rf.DecoderParams["hz_ire"], rf.SysParams["vsync_ire"])
+    descs, keep, want = [], [], []
+    for n, nlines, step in ((1_760_000, 350, 5007.3), (40_000, 14, 2542.2)):
+        ll = 1500.3 + step * np.arange(nlines)
+        demod = rng.normal(rf.iretohz(20), 1e5, n).astype(np.float32)
+        bad = rng.random(n) < 2e-5
+        for s, k in zip(rng.integers(0, n, 40), rng.integers(1, 1600, 40)):
+            bad[s:s + k] = True
+        demod[bad] = 2e6
+        d05 = np.full(n, rf.iretohz(20), np.float32)
+        hp = rng.normal(0, 100, n).astype(np.float32)
+        iserr, _ = odrop.mask(demod, d05, demod, hp, ll, 0, nlines - 3, True, 190, rf.system,
+                              int(rf.delays["video_rot"]), rf.freq_hz_half, lim)
+        want.append(odrop.detect(iserr, ll, 0, nlines - 3, rf.freq, rf.SysParams["outlinelen"]))
+        t = [torch.from_numpy(v).cuda() for v in (demod, d05, demod, hp, ll)]
+        keep.append(t)
+        descs.append(_field(*(v.data_ptr() for v in t[:4]), n, t[4].data_ptr(), nlines, 0, nlines - 3, True, 190))
+    got = run(rf, descs, out_cap=1 << 15)  # the 3-sigma samples of rfhpf alone are some 5000
+    for g, (lines, starts, ends) in zip(got, want):
+        assert len(lines) > 20
+        assert g == (list(lines), list(starts), list(ends))
+    rf.close()
