@@ -452,10 +452,10 @@ __device__ double select_mean(Visit visit, long long n, long long r1, bool two, 
 // and kernels of kSplSlices CTAs per field that walk its pixels:
 //   spline_build    the pieces; a bracket for the median from kSplSamples
 //                   pixels at even steps
-//   spline_pass     counts the wow factors below the bracket and at its ends,
-//                   keeps those between
-//   spline_median   the median, exactly, from those (the counts tell which rank
-//                   to take, or that it is an end); a bracket for the MAD
+//   spline_pass     counts the wow factors up to the bracket's low end, keeps
+//                   those between its ends
+//   spline_median   the median, exactly, from those (their number below tells
+//                   which rank to take, or that it is an end); a bracket for the MAD
 //   spline_pass     the same for |wow - median|
 //   spline_mad      the MAD
 //   spline_maps / spline_levels / spline_maps   (smoothing) the IIR over each
@@ -464,11 +464,11 @@ __device__ double select_mean(Visit visit, long long n, long long r1, bool two, 
 // factors are smooth along a line, so an evenly stepped sample misjudges a
 // rank by about one sample per crossing and square root of the crossings, ~10
 // of 4096.  Evenly spaced lines make most factors equal, and such a value is
-// an end of its bracket: counted, however often it occurs (60 evenly spaced
-// NTSC fields, cubic, smoothing: 588 us the whole call; 1204 by one CTA per
-// field, 1320 with every such value kept until none fitted).  Where a bracket
-// fails all the same (or keeps too many), the CTA selects from all pixels by
-// radix passes.
+// an end of its bracket: not kept, and where the median is an end the CTA counts
+// the factors beyond it in one more walk (60 evenly spaced NTSC fields, cubic,
+// smoothing: 660 us the whole call; 1204 by one CTA per field, 1320 with every
+// such value kept until none fitted).  Where a bracket fails all the same (or
+// keeps too many), the CTA selects from all pixels by radix passes.
 // Bound: instruction issue of the walks (FP64 pipe next).  As one CTA per
 // field walking all pixels up to ten times: 672 us for 60 NTSC fields (cubic,
 // smoothing; as long for one); the eight launches together 250 us (ncu: build
@@ -512,30 +512,54 @@ __device__ void find_bracket(Value value, long long L, double* samp, unsigned* h
     if (t == 0) {
         ctl->lo = lo;
         ctl->hi = hi;
-        ctl->below = 0;
+        ctl->low = 0;
         ctl->kept = 0;
-        ctl->at_lo = 0;
-        ctl->at_hi = 0;
     }
 }
 
-// The median of all L values from what the pass counted and kept, or (kept too
-// many, or the median outside the bracket) from all of them, all(i0, i1, body)
-// visiting them in order.  `signs`: zeros of both signs occur, whose order at a
-// bracket's end is not known from a count.
+// Of key(i), i in [0, n): how many lie below `lo`, and how many up to `hi`.
+template <class Visit>
+__device__ void count_keys(Visit visit, long long n, unsigned long long lo, unsigned long long hi, SelectShared& sh,
+                           long long& below, long long& upto) {
+    const int t = threadIdx.x, lane = t & 31, w = t >> 5;
+    const long long chunk = (n + kSplThreads - 1) / kSplThreads;
+    unsigned long long both = 0;  // counts in 32 bits each
+    visit((long long)t * chunk, min(n, (long long)t * chunk + chunk), [&](long long, unsigned long long kk) {
+        both += (unsigned long long)(kk <= hi) << 32 | (unsigned long long)(kk < lo);
+    });
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) both += __shfl_xor_sync(0xffffffffu, both, o);
+    if (lane == 0) sh.wmin[w] = both;
+    __syncthreads();
+    both = sh.wmin[lane];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) both += __shfl_xor_sync(0xffffffffu, both, o);
+    __syncthreads();
+    below = (long long)(both & 0xffffffffu);
+    upto = (long long)(both >> 32);
+}
+
+// The median of all L values from what the pass counted and kept, all(i0, i1, body)
+// visiting them in order: one that was kept, an end of the bracket (whose ranks
+// one more walk tells), or (kept too many, or the median outside the bracket)
+// selected from all.  `signs`: zeros of both signs occur, which a bracket's end
+// does not tell apart.
 template <class All>
 __device__ double bracket_median(const TbcField& f, All all, long long L, bool signs, unsigned* hist, SelectShared& sh) {
     const SplCtl* ctl = spline_ctl(f);
     const bool two = !(L & 1);
     const long long r1 = median_rank(L), r2 = L / 2;
     const double lo = ctl->lo, hi = ctl->hi;
-    const long long below = ctl->below, kept = ctl->kept;
-    // ranks: below the bracket, its low end, what was kept, its high end
-    const long long n1 = below + ctl->at_lo, n2 = n1 + kept, n3 = n2 + ctl->at_hi;
-    const bool usable = lo <= hi && kept <= kSplKeep && r1 >= below && r2 < n3 && !(signs && (lo == 0 || hi == 0));
+    const long long n1 = ctl->low, kept = ctl->kept, n2 = n1 + kept;  // ranks up to the low end, of what was kept
+    bool usable = lo <= hi && kept <= kSplKeep && !(signs && (lo == 0 || hi == 0));
     __syncthreads();
-    if (!usable) return select_mean(all, L, r1, two, hist, sh);
     const bool in1 = r1 >= n1 && r1 < n2, in2 = r2 >= n1 && r2 < n2;
+    if (usable && !(in1 && in2)) {
+        long long below, upto;
+        count_keys(all, L, order_key(lo), order_key(hi), sh, below, upto);
+        usable = r1 >= below && r2 < upto;
+    }
+    if (!usable) return select_mean(all, L, r1, two, hist, sh);
     double v = 0.0;
     if (in1 || in2) {
         const double* k = spline_kept(f);
@@ -676,8 +700,8 @@ __global__ void __launch_bounds__(kSplThreads) spline_build_kernel(const TbcFiel
     find_bracket([&](long long i) { return wow_at(f, i); }, f.nwow, mem, reinterpret_cast<unsigned*>(hist_mem), sh, ctl);
 }
 
-// One slice of a field's pixels against the bracket: how many lie below it and
-// at its ends, and the values between (in no order).
+// One slice of a field's pixels against the bracket: how many lie up to its low
+// end, and the values between its ends (in no order).
 template <bool Mad>
 __global__ void __launch_bounds__(kSplPassThreads) spline_pass_kernel(const TbcField* fields) {
     const TbcField& f = fields[blockIdx.y];
@@ -696,38 +720,23 @@ __global__ void __launch_bounds__(kSplPassThreads) spline_pass_kernel(const TbcF
     const long long L = f.nwow;
     const long long per = (L + kSplSlices * kSplPassThreads - 1) / (kSplSlices * kSplPassThreads);
     const long long i0 = ((long long)blockIdx.x * kSplPassThreads + t) * per, i1 = min(L, i0 + per);
-    int below = 0, at_lo = 0, at_hi = 0;
+    int low = 0;
     field_walk(f)(i0, i1, [&](long long, double w) {
         const double v = Mad ? fabs(__dadd_rn(w, -med)) : w;
-        const bool less = v < lo;
-        below += less;
-        if (!less && v <= hi) {
-            if (v == lo) {
-                ++at_lo;
-            } else if (v == hi) {
-                ++at_hi;
-            } else {
-                const int at = atomicAdd(&s_n, 1);
-                if (at < kHold) {
-                    held[at] = v;
-                } else if (!s_full) {
-                    const int g = atomicAdd(&ctl->kept, 1);
-                    if (g < kSplKeep) kept[g] = v; else s_full = 1;
-                }
+        low += v <= lo;
+        if (v > lo && v < hi) {
+            const int at = atomicAdd(&s_n, 1);
+            if (at < kHold) {
+                held[at] = v;
+            } else if (!s_full) {
+                const int g = atomicAdd(&ctl->kept, 1);
+                if (g < kSplKeep) kept[g] = v; else s_full = 1;
             }
         }
     });
 #pragma unroll
-    for (int o = 16; o; o >>= 1) {
-        below += __shfl_xor_sync(0xffffffffu, below, o);
-        at_lo += __shfl_xor_sync(0xffffffffu, at_lo, o);
-        at_hi += __shfl_xor_sync(0xffffffffu, at_hi, o);
-    }
-    if ((t & 31) == 0) {
-        if (below) atomicAdd(&ctl->below, below);
-        if (at_lo) atomicAdd(&ctl->at_lo, at_lo);
-        if (at_hi) atomicAdd(&ctl->at_hi, at_hi);
-    }
+    for (int o = 16; o; o >>= 1) low += __shfl_xor_sync(0xffffffffu, low, o);
+    if ((t & 31) == 0 && low) atomicAdd(&ctl->low, low);
     __syncthreads();
     const int n = min(s_n, kHold);
     if (t == 0) s_at = n ? atomicAdd(&ctl->kept, n) : 0;

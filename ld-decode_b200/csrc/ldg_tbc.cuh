@@ -45,12 +45,11 @@ constexpr int kSplStride = 6;
 // the control block of the statistics, the values kept in a bracket, and with
 // smoothing the level before every 32nd output pixel and the IIR's maps.
 struct SplCtl {
-    double lo, hi;     // bracket
-    int below, kept;   // values below it, between its ends
-    int at_lo, at_hi;  // values equal to its ends (at_hi: 0 where the ends are one)
+    double lo, hi;  // bracket
+    int low, kept;  // values up to its low end, between its ends
     int bad;
 };
-constexpr int kSplCtlDoubles = 5;
+constexpr int kSplCtlDoubles = 4;
 constexpr int kSplKeep = 12288;  // values of a bracket kept (4.2 % of a PAL field's)
 
 constexpr int kSplChunks = 1024;  // of a field's pixels in the level-adjust IIR, a thread each

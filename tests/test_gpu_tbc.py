@@ -398,7 +398,7 @@ def test_spline_statistics_plateaus(cuda_ok, method, outw):
 @pytest.mark.parametrize("method", ["quadratic", "cubic"])
 def test_spline_regular_lines_take_no_longer(cuda_ok, method):
     """Evenly spaced lines, whose wow factors are all alike, go through the
-    same few launches as lines with jitter (205 against 169 us a field; 905
+    same few launches as lines with jitter (285 against 166 us a field; 905
     when every factor was kept until they no longer fitted)."""
     import torch
     from ldgpu import RFDecode
