@@ -16,13 +16,15 @@
 //  3. dropout_place_kernel one CTA per field: the error samples merged into
 //     spans (build_errlist, core.py:2889-2908) and the spans placed on TBC
 //     lines (dropout_errlist_to_tbc, core.py:2910-2960), in the reference's
-//     FP64 arithmetic.
+//     FP64 arithmetic (or integers that decide the same).
 //
 // Bound: HBM, 20 bytes per sample of the field's lines.  One CTA doing all of
 // a field took 1.07 ms for one field and 1.36 ms for 60 (a span merge sample
 // by sample on one thread, and 16 conversions to FP64 per clock and SM);
 // the four kernels 58 us and 240 us (ncu; 68, 8, 128 and 36 us for 60 fields,
-// the mask at 5.0 TB/s).
+// the mask at 5.0 TB/s).  The whole call by the errors in one NTSC field: none
+// 0.69 and 0.05 ms, 200 bursts of 100 samples 3.0 and 0.08, 1 % of the samples 2.8
+// and 0.55, every 40th 6.7 and 2.6, every third 26.7 and 0.53.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -39,7 +41,8 @@ namespace {
 constexpr int kStdThreads = 256, kStdPer = kDropStdTile / kStdThreads;
 constexpr int kMaskThreads = 256, kMaskPer = kDropMaskTile / kMaskThreads;
 constexpr int kPlaceThreads = 1024;
-constexpr int kPlaceWords = 48 * 1024;  // mask words of a field held in shared memory (192 KB)
+constexpr int kPlaceWords = 26112;  // mask words of a field held in shared memory, with its spans' starts (204 KB)
+constexpr int kListWords = 2 * (2 * kPlaceThreads + 2);  // pairs: a word's fresh errors, at most two per thread, and an end
 
 __device__ __forceinline__ long long py_index(long long x, long long n) {
     // a slice bound as Python normalises it
@@ -194,69 +197,177 @@ __device__ int block_scan(int v, int* wsum, int* total) {
     return before + inc - v;
 }
 
-// The error samples of a field as bits, those before `end` (samples fit 31 bits).
-struct ErrorBits {
-    const unsigned* words;
-    int end;
-    // the first error sample at or after i, `end` when there is none before `limit`
-    __device__ int next(int i, int limit) const {
-        limit = min(limit, end);
-        while (i < limit) {
-            const unsigned m = words[i >> 5] >> (i & 31);
-            if (m) {
-                i += __ffs(m) - 1;
-                return i < limit ? i : end;
-            }
-            i = (i | 31) + 1;
-        }
-        return end;
+// ---- spans (build_errlist's merge)
+//
+// A span that starts with error sample c0 ends, after each error sample e that
+// joins it, at c0 + min(1.7 (e - c0), cap); the next one joins if it lies up
+// to 20 samples past that end, else it starts the next span.  So a span reaches
+// c0 + cap + 20 at most, and short of that a sample with an error among the 20
+// before it always joins: only the others, the fresh ones, are tested.
+
+struct SpanRule {
+    double cap;
+    int reach;   // samples past c0 that a span can reach
+    bool plain;  // ... for every c0, and the test below in integers
+    int gap;     // no sample more than this past the last one joins
+
+    __device__ explicit SpanRule(double c) : cap(c) {
+        // c0 + cap + 20 is rounded twice, by 5e-7 at most (samples fit 31 bits)
+        const double part = cap - floor(cap);
+        plain = cap < 1e6 && (part == 0 || (part > 1e-6 && part < 1 - 1e-6));
+        reach = plain ? (int)cap + 20 : 0;
+        // up to 20 + min(0.7 d, cap - d) samples past a span of d samples: at most at d = cap / 1.7
+        gap = (int)fmin(cap * (0.7 / 1.7) + 22.0, 1.0e9);
     }
-    // the last sample of the run of error samples that i is in
-    __device__ int run_end(int i) const {
-        for (;;) {
-            const unsigned m = ~(words[i >> 5] >> (i & 31));  // zeros shifted in count as no error
-            const int k = m ? __ffs(m) - 1 : 32;
-            i += k;
-            if ((i & 31) != 0 || i >= end || !(words[i >> 5] & 1u)) return min(i, end) - 1;
-        }
+    __device__ int last_reached(int c0) const {
+        return plain && c0 < 0x7fffffff - reach ? c0 + reach : (int)fmin(floor(((double)c0 + cap) + 20.0), 2147483646.0);
     }
+    // the end of a span of error samples c0 .. last
+    __device__ double end(int c0, int last) const {
+        double pad = (double)(last - c0) * 1.7;
+        if (cap < pad) pad = cap;
+        return (double)c0 + pad;
+    }
+    // does error sample e, the next after `last` and within the span's reach, join it?  (1.7 d is a whole
+    // number, and then exact in FP64 too, or a tenth away from one)
+    __device__ bool joins(int c0, int last, int e) const {
+        return plain ? 10 * (e - c0 - 20) <= 17 * (last - c0) : (double)e <= end(c0, last) + 20.0;
+    }
+    // is error sample e, the next after `prev` (-1: none), the first of a segment?  Its spans do not
+    // depend on what came before.  (Only a mask word's first error: a word then belongs to one segment.)
+    __device__ bool heads(int e, int prev) const { return prev < 0 || (e - prev > gap && e >> 5 != prev >> 5); }
 };
 
-// build_errlist's merge from error sample `e` on, which starts a span.  Within
-// a run of errors every sample extends the span until the span's cap (12 us,
-// and 20 samples) is behind it, so a run takes one step per cap.  Stops at the
-// first error more than `gap` samples after the last (no span reaches
-// that far: it starts a new one whatever came before) and returns the last
-// error sample before it; span(c0, c1, last) gets each span, `last` for the
-// one that ends with the field's last error sample, `top`.
-template <class Span>
-__device__ int merge_segment(const ErrorBits& bits, int e, int gap, double cap, int top, Span&& span) {
-    int c0 = e, b;
-    double c1 = (double)e;
-    for (;;) {
-        b = bits.run_end(e);
-        while (e <= b) {
-            if (e > c0 && (double)e <= c1 + 20.0) {
-                const int last = (int)min((double)b, floor(((double)c0 + cap) + 20.0));
-                e = max(e, last);
-                double pad = (double)(e - c0) * 1.7;
-                if (cap < pad) pad = cap;
-                c1 = (double)c0 + pad;
-            } else if (e > c0) {
-                span(c0, c1, false);
-                c0 = e;
-                c1 = (double)e;
-            }
-            ++e;
-        }
-        e = b + 1 > bits.end - gap ? bits.next(b + 1, bits.end) : bits.next(b + 1, b + 1 + gap);
-        if (e >= bits.end) break;
-    }
-    span(c0, c1, b >= top);
-    return b;
+// The error samples of word m with none among the 20 before them; pm: the word before.
+__device__ __forceinline__ unsigned fresh_errors(unsigned m, unsigned pm) {
+    const unsigned long long both = (unsigned long long)m << 32 | pm;
+    unsigned long long x = both << 1;
+    x |= x << 1;
+    x |= x << 2;
+    x |= x << 4;
+    x |= x << 8;
+    x |= x << 4;
+    return m & ~(unsigned)(x >> 32);
 }
 
-constexpr int kHeld = 4;  // spans a thread keeps from the first merge of its segments
+// The spans of the segment that starts with the first error of word w, in order:
+// span(its first error sample, its last).  words[w], w < wend: the errors, fresh[w]
+// the fresh ones.  A step for every word and every error tested; returns what is
+// left of `steps`, less than 0 when they did not do.
+template <class Span>
+__device__ __forceinline__ int walk_segment(const SpanRule& rule, const unsigned* words, const unsigned* fresh, int w,
+                                            int wend, int steps, Span&& span) {
+    unsigned m = words[w];
+    int c0 = 32 * w + __ffs(m) - 1, far = rule.last_reached(c0);
+    unsigned todo = fresh[w] & (m - 1);  // (the first error is fresh)
+    int last = c0;                       // the last error of the words before, then of this one
+    for (;;) {
+        const int base = 32 * w;
+        // the word's errors past the reach, and its fresh ones, in order
+        if (todo != 0 || far < base + 31) {
+            for (;; --steps) {
+                const unsigned over = far < base ? m : far - base < 31 ? m & (0xfffffffeu << (far - base)) : 0u;
+                const unsigned any = over | todo;
+                if (!any) break;
+                const unsigned bit = any & (0u - any), low = m & (bit - 1u);
+                todo &= ~bit;
+                const int e = base + __ffs(any) - 1, prev = low ? base + 31 - __clz(low) : last;
+                if (!(over & bit) && rule.joins(c0, prev, e)) continue;
+                span(c0, prev);
+                c0 = e;
+                far = rule.last_reached(c0);
+            }
+        }
+        last = base + 31 - __clz(m);
+        // on to the next word with errors, if they still belong to the segment
+        bool on = true;
+        do {
+            if (++w >= wend || 32 * w - last > rule.gap) {
+                on = false;
+                break;
+            }
+            m = words[w];
+        } while (!m);
+        if (--steps < 0) return steps;
+        if (!on || rule.heads(32 * w + __ffs(m) - 1, last)) {
+            span(c0, last);
+            return steps;
+        }
+        todo = fresh[w];
+    }
+}
+
+// The starts of the field's spans among its error words [w0, wend), to marks, by
+// the CTA, a window of a word per thread at a time (plain rules only).  A fresh
+// error f, the next after p, joins the span from c0 on if c0 <= T, by the rule
+// p - (10 (f - p) - 200) / 7: the threads list the window's pairs (f, T), and one of
+// them steps through the list: a comparison per fresh error, a search per span
+// that ends at its reach.  marks holds the fresh errors before.
+__device__ __forceinline__ void walk_windows(const SpanRule& rule, const unsigned* words, unsigned* marks, int w0, int wend,
+                                             int2* list, int* wsum) {
+    const int t = threadIdx.x;
+    int c0 = INT_MAX, far = INT_MAX;  // (before any span)
+    for (int wb = w0; wb < wend; wb += kPlaceThreads) {
+        const int w = wb + t, wtop = min(wend, wb + kPlaceThreads), we = (int)min(32ll * wtop, 0x7fffffffll);
+        const unsigned m = w < wend ? words[w] : 0u;
+        if (!__syncthreads_or(m != 0)) continue;  // (its marks are 0)
+        unsigned fresh = m ? marks[w] : 0u;
+        int n;
+        int at = block_scan(__popc(fresh), wsum, &n);
+        if (t == 0) list[n] = make_int2(INT_MAX, 0);
+        for (; fresh; fresh &= fresh - 1) {
+            const int f = 32 * w + __ffs(fresh) - 1;
+            const unsigned low = m & ((fresh & (0u - fresh)) - 1u);
+            int p = -1;
+            if (low) {
+                p = 32 * w + 31 - __clz(low);
+            } else {  // none within `gap`: a new segment
+                for (int u = w - 1; u >= w0 && f - 32 * u <= rule.gap + 31; --u) {
+                    const unsigned v = words[u];
+                    if (v) {
+                        p = 32 * u + 31 - __clz(v);
+                        break;
+                    }
+                }
+            }
+            list[at++] = make_int2(f, p < 0 ? -1 : p - (10 * (f - p) - 194) / 7);
+        }
+        if (m) marks[w] = 0;
+        __syncthreads();
+        if (t == 0) {
+            int2 r = list[0];
+            for (int i = 0;;) {
+                if (r.x <= far) {
+                    if (r.x == INT_MAX) break;  // (only before any span)
+                    const int2 next = list[++i];
+                    const bool starts = c0 > r.y;
+                    if (starts) {
+                        c0 = r.x;
+                        far = rule.last_reached(c0);
+                        atomicOr(marks + (c0 >> 5), 1u << (c0 & 31));
+                    }
+                    r = next;
+                } else {
+                    // the first error past the reach: one of the next 20 samples, or a fresh one
+                    int x = far + 1;
+                    if (x >= we) break;
+                    const unsigned after = (x >> 5) + 1 < wtop ? words[(x >> 5) + 1] : 0u;
+                    const unsigned v = __funnelshift_r(words[x >> 5], after, x & 31) & 0xfffffu;
+                    x = v ? x + __ffs(v) - 1 : r.x;
+                    if (x >= we) break;
+                    if (x == r.x) r = list[++i];
+                    c0 = x;
+                    far = rule.last_reached(c0);
+                    atomicOr(marks + (c0 >> 5), 1u << (c0 & 31));
+                }
+            }
+        }
+        __syncthreads();
+    }
+}
+
+constexpr int kHeld = 4;    // spans a thread keeps from counting its dropouts
+constexpr int kSteps = 256;  // of a thread's walk before the field goes by windows
 
 }  // namespace
 
@@ -423,20 +534,23 @@ __global__ void __launch_bounds__(kMaskThreads) dropout_mask_kernel(const DropFi
     }
 }
 
-// Threads own consecutive words of the mask.  An error sample more than a
-// span's reach after the one before it starts a segment, whose merge
-// does not depend on what came before: the thread that owns it merges the
-// segment (past its words where it runs on) and keeps its spans; their
-// dropouts are counted, then written.  (More spans than it keeps: the
-// merge runs again for each of the two.)
+// Threads own consecutive words of the mask.  An error sample further from the
+// one before it than any span lets one join starts a segment: the thread that
+// owns it walks the segment's spans (past its words where it runs on), keeps
+// them and counts their dropouts, which it writes after a scan (walking again
+// when there are more than it keeps).  Noise (a carrier lost for lines on end) is
+// one segment of thousands of spans; there the whole field is walked by windows,
+// which mark the spans' starts for all threads to place.  Bound: a thread's chain of
+// instructions.
 __global__ void __launch_bounds__(kPlaceThreads) dropout_place_kernel(const DropField* fields, const DropConsts k,
                                                                       const DropScratch sc, int* drops, int* counts) {
-    extern __shared__ unsigned swords[];  // kPlaceWords
-    __shared__ int wsum[32];
-    __shared__ int s_first, s_down;
+    extern __shared__ unsigned swords[];  // the list of walk_windows, 2 * place_words words
+    int2* list = reinterpret_cast<int2*>(swords);
+    __shared__ int wsum[32], wmax[32];
+    __shared__ int s_down;
     __shared__ double ll[kMaxDropRegions + 1];  // the line locations (the placement searches them)
     const DropField f = fields[blockIdx.x];
-    const int t = threadIdx.x;
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
     for (int l = t; l < f.nlines; l += kPlaceThreads) ll[l] = f.ll[l];
     const int bad = sc.bad[blockIdx.x];
     if (bad) {
@@ -446,36 +560,25 @@ __global__ void __launch_bounds__(kPlaceThreads) dropout_place_kernel(const Drop
         }
         return;
     }
-    if (t == 0) {
-        s_first = 0x7fffffff;
-        s_down = 0;
-    }
+    if (t == 0) s_down = 0;
     __syncthreads();
     long long lo, hi;
     mask_range(f, lo, hi);
     const double ll0 = ll[f.lineoffset];
     const int from = (int)min(max(lo, (long long)ceil(ll0)), hi);  // the errors before line `lineoffset` start no span
-    const long long w0 = lo >> 5, nw = hi > lo ? ((hi + 31) >> 5) - w0 : 0;
-    // the mask in shared memory when it fits (a field of 1.5 M samples does):
-    // the searches below are chains of single-word reads
-    ErrorBits bits{sc.words + f.word0, (int)hi};
-    if (nw <= sc.place_words) {
+    // samples fit 31 bits, and words and bits are counted in int
+    const int w0 = (int)(lo >> 5), nw = hi > lo ? (int)((hi + 31) >> 5) - w0 : 0, wend = w0 + nw;
+    // the mask from `from` on and the spans' starts, in shared memory when they fit (a field of 0.83 M samples does)
+    unsigned* const gwords = sc.words + f.word0;
+    const bool held = nw <= sc.place_words;
+    int n = 0;  // errors of the field
 #pragma unroll 8
-        for (int w = t; w < (int)nw; w += kPlaceThreads) swords[w] = bits.words[w0 + w];
-        bits.words = swords - w0;
-    }
-    __syncthreads();
-    const long long per = (nw + kPlaceThreads - 1) / kPlaceThreads;
-    // this thread's samples
-    const int a = (int)min(max((long long)from, (w0 + t * per) << 5), hi);
-    const int b = (int)min(hi, (w0 + (t + 1) * per) << 5);
-    // errors of the field; this thread's last one, and the last one before its words
-    int n = 0;
-    long long last = -1;
-    for (long long w = w0 + t * per; w < min(w0 + nw, w0 + (t + 1) * per); ++w) {
-        const unsigned m = bits.words[w];
+    for (int w = w0 + t; w < wend; w += kPlaceThreads) {
+        unsigned m = gwords[w];
         n += __popc(m);
-        if (m) last = 32 * w + 31 - __clz(m);
+        if (w <= from >> 5) m = w < from >> 5 ? 0u : m & (0xffffffffu << (from & 31));
+        if (held) swords[kListWords + w - w0] = m;
+        else gwords[w] = m;
     }
     int nerr;
     block_scan(n, wsum, &nerr);
@@ -484,115 +587,139 @@ __global__ void __launch_bounds__(kPlaceThreads) dropout_place_kernel(const Drop
         if (t == 0) counts[2 * blockIdx.x] = 0;
         return;
     }
-    if (last < from) last = -1;  // (the last error alone decides whether there are spans: it must lie past ll0)
-    __shared__ int wmax[32];
-    int before = (int)last;
-    const int lane = t & 31, warp = t >> 5;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int y = __shfl_up_sync(0xffffffffu, before, o);
-        if (lane >= o) before = max(before, y);
-    }
-    if (lane == 31) wmax[warp] = before;
-    before = __shfl_up_sync(0xffffffffu, before, 1);
-    if (lane == 0) before = -1;
     // are the line locations in order?
     for (int l = f.lineoffset + t; l < f.lineoffset + f.linecount; l += kPlaceThreads)
         if (!(ll[l] <= ll[l + 1])) s_down = 1;
-    __syncthreads();
-    int top = -1;
-    for (int w = 0; w < 32; ++w) {
-        if (w < warp) before = max(before, wmax[w]);
-        top = max(top, wmax[w]);
-    }
-    if (top < 0 || !((double)top > ll0)) {  // no error, or none past ll0
-        if (t == 0) counts[2 * blockIdx.x] = 0;
-        return;
-    }
-    const double cap = k.freq_mhz * 12.0;
-    const int gap = (int)min(cap + 21.0, 1.0e9);
-    // every segment that starts among this thread's samples, in order
-    auto segments = [&](auto&& span) {
-        int prev = before;
-        for (int e = bits.next(a, b); e < bits.end;) {
-            if (prev < 0 || e - prev > gap) {
-                prev = merge_segment(bits, e, gap, cap, top, span);
-            } else {
-                prev = bits.run_end(e);
-            }
-            e = bits.next(prev + 1, b);
-        }
-    };
+    const int per = (nw + kPlaceThreads - 1) / kPlaceThreads;
+    const int wa = w0 + min(nw, t * per), wb = w0 + min(nw, (t + 1) * per);
+    const SpanRule rule(k.freq_mhz * 12.0);
     // a span as the placement gets it: 8 samples ahead and 4 behind, but the last one as it is
     auto start_of = [](int c0, bool is_last) { return (double)(is_last ? c0 : c0 - 8); };
-    Emitter em{drops + (size_t)blockIdx.x * k.out_cap * 3, k.out_cap, 0, false};
-    if (s_down) {
-        // line locations out of order: the placement's search depends on the spans before
-        if (t == 0) {
-            LinePlacer lp{ll, f.lineoffset, f.lineoffset + f.linecount, f.lineoffset, (double)k.outlinelen, ll0,
-                          false, false, 0.0, 0.0, &em};
-            int e = bits.next(from, bits.end);
-            while (e < bits.end) {
-                const int l = merge_segment(bits, e, gap, cap, top, [&](int c0, double c1, bool is_last) {
-                    lp.feed(start_of(c0, is_last), is_last ? c1 : c1 + 4.0);
-                });
-                e = bits.next(l + 1, bits.end);
+
+    auto place_field = [&](const unsigned* words, unsigned* marks) {
+        // the last error of the words before this thread's, and of the field
+        int before = -1, top = -1;
+        for (int w = wa; w < wb; ++w) {
+            const unsigned m = words[w];
+            if (m) before = 32 * w + 31 - __clz(m);
+        }
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, before, o);
+            if (lane >= o) before = max(before, y);
+        }
+        if (lane == 31) wmax[warp] = before;
+        before = __shfl_up_sync(0xffffffffu, before, 1);
+        if (lane == 0) before = -1;
+        for (int w = w0 + t; w < wend; w += kPlaceThreads) {
+            const unsigned m = words[w];
+            marks[w] = m ? fresh_errors(m, w > w0 ? words[w - 1] : 0u) : 0u;
+        }
+        __syncthreads();
+        for (int w = 0; w < 32; ++w) {
+            if (w < warp) before = max(before, wmax[w]);
+            top = max(top, wmax[w]);
+        }
+        if (top < 0 || !((double)top > ll0)) {  // no error, or none past ll0 (the last one decides whether there are spans)
+            if (t == 0) counts[2 * blockIdx.x] = 0;
+            return;
+        }
+        Emitter em{drops + (size_t)blockIdx.x * k.out_cap * 3, k.out_cap, 0, false}, dry{nullptr, 0, 0, false};
+        auto place = [&](Emitter& out, int c0, int end) {
+            const bool is_last = end >= top;
+            const double s0 = start_of(c0, is_last), c1 = rule.end(c0, end);
+            if (s0 < ll0 && !is_last) return;  // skipped while a later span exists
+            // the line of a span: the first one it starts in
+            int x = f.lineoffset, y = f.lineoffset + f.linecount;  // first line with s0 <= its end
+            while (x < y) {
+                const int mid = (x + y) >> 1;
+                if (ll[mid + 1] >= s0) y = mid; else x = mid + 1;
             }
-            lp.finish();
-            counts[2 * blockIdx.x] = em.over ? -1 : em.n;
-        }
-        return;
-    }
-    // the first span the placement keeps: the first from ll0 on, else the last
-    int nspans = 0, first = 0x7fffffff;
-    int held0[kHeld];
-    double held1[kHeld];
-    bool ends = false;  // the last span is the field's last
-    segments([&](int c0, double c1, bool is_last) {
-        if (nspans < kHeld) {
-            held0[nspans] = c0;
-            held1[nspans] = c1;
-        }
-        ends = is_last;
-        if (first == 0x7fffffff && start_of(c0, is_last) >= ll0) first = nspans;
-        ++nspans;
-    });
-    int total;
-    const int base = block_scan(nspans, wsum, &total);
-    if (first != 0x7fffffff) atomicMin(&s_first, base + first);
-    __syncthreads();
-    const int keep = min(s_first, total - 1);
-    // the line of a span: the first one it starts in
-    auto line_of = [&](double c0) {
-        int x = f.lineoffset, y = f.lineoffset + f.linecount;  // first line with c0 <= its end
-        while (x < y) {
-            const int mid = (x + y) >> 1;
-            if (ll[mid + 1] >= c0) y = mid; else x = mid + 1;
-        }
-        return x < f.lineoffset + f.linecount && c0 >= ll[x] ? x : -1;
-    };
-    auto place = [&](Emitter& out) {
-        int i = base;
-        auto one = [&](int c0, double c1, bool is_last) {
-            if (i++ < keep) return;
-            const double s0 = start_of(c0, is_last);
-            const int line = line_of(s0);
-            if (line < 0) return;
-            LinePlacer lp{ll, line, line + 1, f.lineoffset, (double)k.outlinelen, ll0, true, false, 0.0, 0.0, &out};
+            if (x == f.lineoffset + f.linecount || s0 < ll[x]) return;
+            LinePlacer lp{ll, x, x + 1, f.lineoffset, (double)k.outlinelen, ll0, true, false, 0.0, 0.0, &out};
             lp.place(s0, is_last ? c1 : c1 + 4.0);
         };
-        if (nspans <= kHeld) {
-            for (int q = 0; q < nspans; ++q) one(held0[q], held1[q], ends && q == nspans - 1);
-        } else {
-            segments(one);
+        // the spans of the segments that start in this thread's words, in order
+        auto segments = [&](int steps, auto&& span) {
+            int prev = before;
+            for (int w = wa; w < wb && steps >= 0; ++w) {
+                const unsigned m = words[w];
+                if (!m) continue;
+                if (rule.heads(32 * w + __ffs(m) - 1, prev)) steps = walk_segment(rule, words, marks, w, wend, steps, span);
+                prev = 32 * w + 31 - __clz(m);
+            }
+            return steps;
+        };
+        int nspans = 0, held0[kHeld], held1[kHeld], total;
+        const int left = s_down ? -1 : segments(rule.plain ? kSteps : INT_MAX, [&](int c0, int end) {
+            if (nspans < kHeld) {
+                held0[nspans] = c0;
+                held1[nspans] = end;
+            }
+            ++nspans;
+            place(dry, c0, end);
+        });
+        if (!__syncthreads_or(left < 0)) {
+            em.n = block_scan(dry.n, wsum, &total);
+            if (nspans <= kHeld) {
+                for (int q = 0; q < nspans; ++q) place(em, held0[q], held1[q]);
+            } else {
+                segments(INT_MAX, [&](int c0, int end) { place(em, c0, end); });
+            }
+            if (t == 0) counts[2 * blockIdx.x] = total > k.out_cap ? -1 : total;
+            return;
         }
+        if (s_down) {
+            // line locations out of order: the placement's search depends on the spans before
+            if (t == 0) {
+                LinePlacer lp{ll, f.lineoffset, f.lineoffset + f.linecount, f.lineoffset, (double)k.outlinelen, ll0,
+                              false, false, 0.0, 0.0, &em};
+                int prev = -1;
+                for (int w = w0; w < wend; ++w) {
+                    const unsigned m = words[w];
+                    if (!m) continue;
+                    if (rule.heads(32 * w + __ffs(m) - 1, prev))
+                        walk_segment(rule, words, marks, w, wend, INT_MAX, [&](int c0, int end) {
+                            const bool is_last = end >= top;
+                            const double c1 = rule.end(c0, end);
+                            lp.feed(start_of(c0, is_last), is_last ? c1 : c1 + 4.0);
+                        });
+                    prev = 32 * w + 31 - __clz(m);
+                }
+                lp.finish();
+                counts[2 * blockIdx.x] = em.over ? -1 : em.n;
+            }
+            return;
+        }
+        walk_windows(rule, words, marks, w0, wend, list, wsum);
+        // the spans that start in this thread's words, in order
+        auto spans = [&](Emitter& out) {
+            for (int w = wa; w < wb; ++w) {
+                for (unsigned m = marks[w]; m; m &= m - 1) {
+                    // every error up to the next span's start, and short of the reach, is this one's
+                    const int c0 = 32 * w + __ffs(m) - 1, far = rule.last_reached(c0);
+                    unsigned above = m & (m - 1), from_c0 = 0u - (m & (0u - m));
+                    int end = c0;
+                    for (int u = w; u < wend && 32 * u <= far; from_c0 = 0xffffffffu, above = ++u < wend ? marks[u] : 0u) {
+                        unsigned e = words[u] & from_c0;
+                        if (above) e &= (above & (0u - above)) - 1u;
+                        if (far - 32 * u < 31) e &= ~(0xfffffffeu << (far - 32 * u));
+                        if (e) end = 32 * u + 31 - __clz(e);
+                        if (above) break;
+                    }
+                    place(out, c0, end);
+                }
+            }
+        };
+        dry.n = 0;
+        spans(dry);
+        em.n = block_scan(dry.n, wsum, &total);
+        spans(em);
+        if (t == 0) counts[2 * blockIdx.x] = total > k.out_cap ? -1 : total;
     };
-    Emitter dry{nullptr, 0, 0, false};
-    place(dry);
-    const int at = block_scan(dry.n, wsum, &total);
-    em.n = at;
-    place(em);
-    if (t == 0) counts[2 * blockIdx.x] = total > k.out_cap ? -1 : total;
+    // (each form's pointers into one address space)
+    if (held) place_field(swords + kListWords - w0, swords + kListWords + sc.place_words - w0);
+    else place_field(gwords, sc.starts + f.word0);
 }
 
 size_t dropout_scratch(DropField* fields, int nfields, char* base, DropScratch* sc) {
@@ -617,6 +744,7 @@ size_t dropout_scratch(DropField* fields, int nfields, char* base, DropScratch* 
     q.bad = reinterpret_cast<int*>(take(nf * sizeof(int)));
     q.rf_hi = reinterpret_cast<float*>(take(nf * sizeof(float)));
     q.words = reinterpret_cast<unsigned*>(take(words * sizeof(unsigned)));
+    q.starts = reinterpret_cast<unsigned*>(take(words * sizeof(unsigned)));
     q.place_words = 0;
     if (sc) *sc = q;
     return (size_t)(p - base);
@@ -638,8 +766,8 @@ cudaError_t launch_dropouts(const DropField* fields, int nfields, long long max_
         dropout_merge_kernel<<<(n + 3) / 4, 128, 0, stream>>>(fields + lo, (int)n, q, rfstd ? rfstd + lo : nullptr);
         dropout_mask_kernel<<<dim3(mask_tiles, n), kMaskThreads, 0, stream>>>(fields + lo, k, q);
     }
-    // no more shared memory than the longest mask needs
-    const size_t bytes = (size_t)sc.place_words * sizeof(unsigned);
+    // no more shared memory than the longest mask and the list need
+    const size_t bytes = ((size_t)kListWords + 2 * sc.place_words) * sizeof(unsigned);
     static SmemAttr attr;
     const cudaError_t e = attr.ensure(dropout_place_kernel, bytes);
     if (e != cudaSuccess) return e;

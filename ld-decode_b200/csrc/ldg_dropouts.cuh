@@ -35,6 +35,7 @@ struct DropScratch {
     int* bad;
     float* rf_hi;       // the error limit of rfhpf (3 standard deviations)
     unsigned* words;
+    unsigned* starts;   // the spans' first error samples
     int place_words;    // mask words the placement's shared memory holds
 };
 

@@ -257,3 +257,92 @@ def test_long_mask_equals_oracle(cuda_ok):
         assert len(lines) > 20
         assert g == (list(lines), list(starts), list(ends))
     rf.close()
+
+
+def _pattern(kind, n, rng):
+    bad = np.zeros(n, bool)
+    if kind.startswith("every "):
+        bad[::int(kind[6:])] = True
+    elif kind.startswith("rate "):
+        bad = rng.random(n) < float(kind[5:])
+    else:  # runs and gaps around the rules' limits
+        gaps = [1, 19, 20, 21, 22, 37, 38, 60, 216, 217, 218, 219, 220, 221, 400, 501, 502]
+        at = 1500
+        while at < n - 3000:
+            ln = int(rng.choice([1, 1, 2, 20, 33, 282, 283, 480, 500, 501, 900]))
+            bad[at:at + ln] = True
+            at += ln + int(rng.choice(gaps))
+    return bad
+
+
+@pytest.mark.parametrize("kind", ["every 1", "every 2", "every 3", "every 20", "every 21", "every 22", "every 40",
+                                  "every 100", "every 218", "every 220", "every 480", "rate 0.01", "rate 0.1", "rate 0.5",
+                                  "limits"])
+@pytest.mark.parametrize("freq", [40.0, 28.636363636363637, 29.16666667, 100.0])
+def test_long_segments_equal_oracle(cuda_ok, kind, freq):
+    """Masks whose spans follow one another without a pause, so that one
+    segment holds the field's: walked by windows, and by one thread where the
+    span's cap is close to a whole number.  Whole fields, one too long for shared
+    memory, and one with its line locations out of order: the oracle's lists."""
+    import torch
+    from ldgpu import RFDecode
+    from ldgpu.dropouts import _field, run
+    rf = RFDecode(system="NTSC")
+    rf.freq = freq
+    rng = np.random.default_rng(len(kind))
+    lim = odrop.limits(rf.system, rf.DecoderParams["ire0"], rf.DecoderParams["hz_ire"], rf.SysParams["vsync_ire"])
+    descs, keep, want = [], [], []
+    for n, nlines, step in ((102_400 + 17, 40, 2542.2), (30_000, 11, 2542.2), (845_000, 240, 3520.7)):
+        if n > 800_000 and kind not in ("every 40", "rate 0.1"):
+            continue
+        ll = 1500.3 + step * np.arange(nlines)
+        if n == 30_000:
+            ll[6], ll[7] = np.floor(ll[7]) + 0.75, np.floor(ll[7]) + 0.25
+        demod = np.full(n, rf.iretohz(20), np.float32)
+        demod[_pattern(kind, n, rng)] = 2e6
+        d05 = np.full(n, rf.iretohz(20), np.float32)
+        hp = np.zeros(n, np.float32)
+        iserr, _ = odrop.mask(demod, d05, demod, hp, ll, 0, nlines - 3, True, 190, rf.system,
+                              int(rf.delays["video_rot"]), rf.freq_hz_half, lim)
+        want.append(odrop.detect(iserr, ll, 0, nlines - 3, freq, rf.SysParams["outlinelen"]))
+        t = [torch.from_numpy(v).cuda() for v in (demod, d05, demod, hp, ll)]
+        keep.append(t)
+        descs.append(_field(*(v.data_ptr() for v in t[:4]), n, t[4].data_ptr(), nlines, 0, nlines - 3, True, 190))
+    got = run(rf, descs, out_cap=1 << 16)
+    for i, (g, (lines, starts, ends)) in enumerate(zip(got, want)):
+        assert g == (list(lines), list(starts), list(ends)), i
+    rf.close()
+
+
+def test_noise_takes_no_longer_than_it_should(cuda_ok):
+    """A field of which every third sample is an error against one without
+    errors: 0.5 and 0.05 ms (216 ms by one thread's merge of its one segment)."""
+    import torch
+    from ldgpu import RFDecode
+    from ldgpu.dropouts import ERR_CAP, OUT_CAP, _field, dropout_params
+    import ctypes
+    rf = RFDecode(system="NTSC")
+    n, nlines = 263 * 2543 + 20_000, 273
+    ll = torch.from_numpy(1500.3 + 2542.2 * np.arange(nlines)).cuda()
+    flat, hp = torch.full((n,), float(rf.iretohz(20)), device="cuda"), torch.zeros(n, device="cuda")
+    drops = torch.empty(OUT_CAP * 3, dtype=torch.int32, device="cuda")
+    counts = torch.empty(2, dtype=torch.int32, device="cuda")
+    p, took = dropout_params(rf, ERR_CAP, OUT_CAP), []
+    for every in (0, 3):
+        x = flat.clone()
+        if every:
+            x[::every] = 2e6
+        d = (L.DropoutField * 1)(_field(x.data_ptr(), flat.data_ptr(), x.data_ptr(), hp.data_ptr(), n, ll.data_ptr(), nlines,
+                                        0, 262, True, 190))
+        times = []
+        for _ in range(7):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            L.check(rf._ctx._lib.ldg_dropouts(rf._ctx.handle, ctypes.byref(p), d, 1, drops.data_ptr(), counts.data_ptr(),
+                                              None, 1))
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        took.append(float(np.median(times)))
+    assert counts[0] > 1000 and took[1] < 60 * took[0], took
+    rf.close()
