@@ -35,6 +35,10 @@ namespace {
 constexpr int kThreads = 128;
 constexpr int kTile = 32 * kThreads;    // samples: one 32-bit word of sign flags per thread
 constexpr int kMaxChunks = 148 * 16;    // the resident CTAs
+// Crossings of a tile above which a warp writes them word by word, not each
+// thread its own word's: 80 M samples with a crossing every 4 take 153 us for 194,
+// white noise 180 for 537, a crossing every 8 the other way round 146 for 116.
+constexpr int kDense = kTile / 6;
 
 size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
@@ -176,7 +180,24 @@ __device__ __forceinline__ int write_tile(const int16_t* __restrict__ x, long lo
     long long k = end - total + ahead + inc - cnt;
     const int16_t* xt = x + t0 + 32 * t;
     const unsigned pos = (unsigned)(pos_offset + t0 + 32 * t);
-    if (In && end <= cap && (reinterpret_cast<uintptr_t>(edges) & 7) == 0) {
+    const bool whole = In && end <= cap && (reinterpret_cast<uintptr_t>(edges) & 7) == 0;
+    if (whole && total > kDense) {
+        // lane l takes sample l of the warp's words in turn, so that a store's lanes write side by side
+        uint2* out = reinterpret_cast<uint2*>(edges + (end - total + ahead));
+        const int16_t* xw = x + t0 + 1024 * warp + lane;
+        const unsigned pw = (unsigned)(pos_offset + t0 + 1024 * warp + lane);
+        const int at = inc - cnt;
+#pragma unroll 4
+        for (int s = 0; s < 32; ++s) {
+            const unsigned es = __shfl_sync(0xffffffffu, e, s);
+            const int o = __shfl_sync(0xffffffffu, at, s);
+            if ((es >> lane) & 1u)
+                out[o + __popc(es & ((1u << lane) - 1u))] =
+                    make_uint2(pw + 32 * s, (unsigned)(uint16_t)xw[32 * s - 1] | ((unsigned)(uint16_t)xw[32 * s] << 16));
+        }
+        return total;
+    }
+    if (whole) {
         uint2* out = reinterpret_cast<uint2*>(edges + k);
         while (e) {
             const int c = __ffs(e) - 1;

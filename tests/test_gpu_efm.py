@@ -130,3 +130,66 @@ def test_pll_from_gpu_edges_of_demodulated_efm(cuda_ok):
         total += len(ta)
     assert total > 1000 and a.state() == b.state()
     rf.close()
+
+
+@pytest.mark.parametrize("every", [1, 2, 3, 5, 6, 7, "noise", "mixed"])
+def test_dense_edges(cuda_ok, every):
+    """Tiles with more crossings than a thread writes for itself, among tiles
+    with fewer, from any alignment of the samples; and room for some of them."""
+    import ctypes
+
+    import torch
+    from ldgpu import lib as L
+    from ldgpu.efm import efm_edges
+    n = 3 * 4096 + 77
+    rng = np.random.default_rng(1)
+    if every == "noise":
+        x = rng.integers(-3000, 3000, n + 9)
+    elif every == "mixed":
+        x = np.where(np.arange(n + 9) // 4096 % 2, (-1) ** np.arange(n + 9), 1) * rng.integers(1, 99, n + 9)
+    else:
+        x = (-1) ** (np.arange(n + 9) // every) * rng.integers(1, 99, n + 9)
+    x = x.astype(np.int16)
+    for off in (0, 1, 5, 8):
+        t = torch.from_numpy(x).cuda()[off:off + n]
+        want = efm_crossings(x[off:off + n])
+        assert efm_edges(t).tobytes() == want.tobytes()
+    # a cap within a dense tile, a buffer that starts between 8-byte boundaries
+    lib, cap = L.load(), len(want) * 2 // 3
+    for shift, room in ((0, cap), (4, len(want)), (4, cap)):
+        buf = torch.full((8 * len(want) + 32,), 85, dtype=torch.uint8, device="cuda")
+        count = torch.zeros(1, dtype=torch.int64, device="cuda")
+        scratch = torch.empty(lib.ldg_efm_edges_scratch_bytes(n), dtype=torch.uint8, device="cuda")
+        L.check(lib.ldg_efm_edges(t.data_ptr(), n, 0, 0, ctypes.c_void_p(buf.data_ptr() + shift), room, count.data_ptr(),
+                                  scratch.data_ptr(), 1))
+        got = buf.cpu().numpy().tobytes()
+        assert int(count.item()) == len(want)
+        assert got[shift:shift + 8 * room] == want[:room].tobytes()
+        assert got[:shift] == b"U" * shift and set(got[shift + 8 * room:]) == {85}
+
+
+def test_noise_takes_no_longer_than_a_pass_and_its_edges(cuda_ok):
+    """20 M samples of alternating sign against samples of one sign: the 8
+    bytes of every crossing (160 MB) beside the 40 MB of samples, and not
+    scattered stores (76 against 28 us; 280 by each thread its own word's)."""
+    import torch
+    from ldgpu import lib as L
+    lib, n = L.load(), 20_000_000
+    edges = torch.empty(8 * n + 64, dtype=torch.uint8, device="cuda")
+    count = torch.zeros(1, dtype=torch.int64, device="cuda")
+    scratch = torch.empty(lib.ldg_efm_edges_scratch_bytes(n), dtype=torch.uint8, device="cuda")
+    took = []
+    for noisy in (False, True):
+        x = torch.full((n,), 5, dtype=torch.int16, device="cuda")
+        if noisy:
+            x[::2] = -5
+        times = []
+        for _ in range(15):
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            L.check(lib.ldg_efm_edges(x.data_ptr(), n, 0, 0, edges.data_ptr(), n, count.data_ptr(), scratch.data_ptr(), 1))
+            b.record()
+            b.synchronize()
+            times.append(a.elapsed_time(b))
+        took.append(float(np.median(times)))
+    assert int(count.item()) == n and took[1] < 6 * took[0], took
