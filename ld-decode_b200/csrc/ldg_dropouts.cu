@@ -116,64 +116,24 @@ struct Emitter {
     }
 };
 
-// Spans to TBC lines (core.py:2910-2960), fed one span at a time in order.
-struct LinePlacer {
-    const double* ll;
-    int line, end_line, lineoffset;
-    double outlinelen;
-    double ll0;
-    bool placing;          // past the reference's initial skip of spans before line `lineoffset`
-    bool have_pending;
-    double p0, p1;
-    Emitter* em;
-
-    __device__ void place(double c0, double c1) {
-        while (line < end_line) {
-            const double a = ll[line], b = ll[line + 1];
-            if (c0 >= a && c0 <= b) {
-                const double span = b - a;
-                const long long start = (long long)(((c0 - a) / span) * outlinelen);
-                const long long end = (long long)rint(((c1 - a) / span) * outlinelen);
-                const int first = line + 1 - lineoffset;
-                const long long ol = (long long)outlinelen;
-                if (end > ol) {
-                    const long long k = end / ol;
-                    em->put(first - 1, start, ol);
-                    for (long long j = 0; j < k - 1; ++j) em->put((int)(first + j + 1) - 1, 0, ol);
-                    em->put((int)(first + k) - 1, 0, end % ol);
-                } else {
-                    em->put(first - 1, start, end);
-                }
-                return;
-            }
-            ++line;
-        }
+// A span [c0, c1) that starts in line `line` (of line locations a, b at its ends)
+// as TBC line ranges (core.py:2910-2960).
+__device__ __forceinline__ void emit_span(Emitter& em, int line, int lineoffset, double a, double b, double c0, double c1,
+                                          double outlinelen) {
+    const double span = b - a;
+    const long long start = (long long)(((c0 - a) / span) * outlinelen);
+    const long long end = (long long)rint(((c1 - a) / span) * outlinelen);
+    const int first = line + 1 - lineoffset;
+    const long long ol = (long long)outlinelen;
+    if (end > ol) {
+        const long long k = end / ol;
+        em.put(first - 1, start, ol);
+        for (long long j = 0; j < k - 1; ++j) em.put((int)(first + j + 1) - 1, 0, ol);
+        em.put((int)(first + k) - 1, 0, end % ol);
+    } else {
+        em.put(first - 1, start, end);
     }
-    __device__ void feed(double s0, double s1) {
-        if (!placing) {
-            if (!have_pending) {
-                p0 = s0;
-                p1 = s1;
-                have_pending = true;
-                return;
-            }
-            if (p0 < ll0) {  // a later span exists: the reference pops on
-                p0 = s0;
-                p1 = s1;
-                return;
-            }
-            placing = true;
-            place(p0, p1);
-        }
-        place(s0, s1);
-    }
-    __device__ void finish() {
-        if (!placing && have_pending) {
-            placing = true;
-            place(p0, p1);
-        }
-    }
-};
+}
 
 // Exclusive scan of v over the CTA; *total its sum.
 __device__ int block_scan(int v, int* wsum, int* total) {
@@ -625,20 +585,28 @@ __global__ void __launch_bounds__(kPlaceThreads) dropout_place_kernel(const Drop
             return;
         }
         Emitter em{drops + (size_t)blockIdx.x * k.out_cap * 3, k.out_cap, 0, false}, dry{nullptr, 0, 0, false};
-        auto place = [&](Emitter& out, int c0, int end) {
+        const int line0 = f.lineoffset, line1 = f.lineoffset + f.linecount;
+        // the line of a span: the first one it starts in, -1 for none or a span that is skipped
+        auto skipped = [&](double s0, bool is_last) { return s0 < ll0 && !is_last; };  // a later span exists
+        auto line_of = [&](int c0, int end) {
             const bool is_last = end >= top;
-            const double s0 = start_of(c0, is_last), c1 = rule.end(c0, end);
-            if (s0 < ll0 && !is_last) return;  // skipped while a later span exists
-            // the line of a span: the first one it starts in
-            int x = f.lineoffset, y = f.lineoffset + f.linecount;  // first line with s0 <= its end
+            const double s0 = start_of(c0, is_last);
+            if (skipped(s0, is_last)) return -1;
+            int x = line0, y = line1;  // first line with s0 <= its end
             while (x < y) {
                 const int mid = (x + y) >> 1;
                 if (ll[mid + 1] >= s0) y = mid; else x = mid + 1;
             }
-            if (x == f.lineoffset + f.linecount || s0 < ll[x]) return;
-            LinePlacer lp{ll, x, x + 1, f.lineoffset, (double)k.outlinelen, ll0, true, false, 0.0, 0.0, &out};
-            lp.place(s0, is_last ? c1 : c1 + 4.0);
+            return x < line1 && s0 >= ll[x] ? x : -1;
         };
+        auto place_in = [&](Emitter& out, int c0, int end, int line) {
+            if (line < 0) return;
+            const bool is_last = end >= top;
+            const double c1 = rule.end(c0, end);
+            emit_span(out, line, line0, ll[line], ll[line + 1], start_of(c0, is_last), is_last ? c1 : c1 + 4.0,
+                      (double)k.outlinelen);
+        };
+        auto place = [&](Emitter& out, int c0, int end) { place_in(out, c0, end, line_of(c0, end)); };
         // the spans of the segments that start in this thread's words, in order
         auto segments = [&](int steps, auto&& span) {
             int prev = before;
@@ -669,31 +637,14 @@ __global__ void __launch_bounds__(kPlaceThreads) dropout_place_kernel(const Drop
             if (t == 0) counts[2 * blockIdx.x] = total > k.out_cap ? -1 : total;
             return;
         }
-        if (s_down) {
-            // line locations out of order: the placement's search depends on the spans before
-            if (t == 0) {
-                LinePlacer lp{ll, f.lineoffset, f.lineoffset + f.linecount, f.lineoffset, (double)k.outlinelen, ll0,
-                              false, false, 0.0, 0.0, &em};
-                int prev = -1;
-                for (int w = w0; w < wend; ++w) {
-                    const unsigned m = words[w];
-                    if (!m) continue;
-                    if (rule.heads(32 * w + __ffs(m) - 1, prev))
-                        walk_segment(rule, words, marks, w, wend, INT_MAX, [&](int c0, int end) {
-                            const bool is_last = end >= top;
-                            const double c1 = rule.end(c0, end);
-                            lp.feed(start_of(c0, is_last), is_last ? c1 : c1 + 4.0);
-                        });
-                    prev = 32 * w + 31 - __clz(m);
-                }
-                lp.finish();
-                counts[2 * blockIdx.x] = em.over ? -1 : em.n;
+        const bool marked = rule.plain;
+        if (marked) walk_windows(rule, words, marks, w0, wend, list, wsum);
+        // the spans that start in this thread's words (or in the segments that do), in order
+        auto spans = [&](auto&& body) {
+            if (!marked) {
+                segments(INT_MAX, body);
+                return;
             }
-            return;
-        }
-        walk_windows(rule, words, marks, w0, wend, list, wsum);
-        // the spans that start in this thread's words, in order
-        auto spans = [&](Emitter& out) {
             for (int w = wa; w < wb; ++w) {
                 for (unsigned m = marks[w]; m; m &= m - 1) {
                     // every error up to the next span's start, and short of the reach, is this one's
@@ -707,15 +658,53 @@ __global__ void __launch_bounds__(kPlaceThreads) dropout_place_kernel(const Drop
                         if (e) end = 32 * u + 31 - __clz(e);
                         if (above) break;
                     }
-                    place(out, c0, end);
+                    body(c0, end);
                 }
             }
         };
-        dry.n = 0;
-        spans(dry);
-        em.n = block_scan(dry.n, wsum, &total);
-        spans(em);
-        if (t == 0) counts[2 * blockIdx.x] = total > k.out_cap ? -1 : total;
+        // a span per thread at a time; with line locations out of order a span's line depends on the one of
+        // the span before, and one thread finds the lines
+        nspans = 0;
+        spans([&](int, int) { ++nspans; });
+        const int base = block_scan(nspans, wsum, &total);
+        int written = 0, line = line0;
+        for (int batch = 0; batch < total; batch += kPlaceThreads) {
+            if (base < batch + kPlaceThreads && base + nspans > batch) {
+                int i = base - batch;
+                spans([&](int c0, int end) {
+                    if (i >= 0 && i < kPlaceThreads) list[i] = make_int2(c0, end);
+                    ++i;
+                });
+            }
+            __syncthreads();
+            const int n = min(total - batch, kPlaceThreads);
+            int* lines = reinterpret_cast<int*>(list + kPlaceThreads);
+            if (s_down && t == 0) {
+                for (int i = 0; i < n; ++i) {
+                    const int2 q = list[i];
+                    const bool is_last = q.y >= top;
+                    const double s0 = start_of(q.x, is_last);
+                    lines[i] = -1;
+                    if (skipped(s0, is_last)) continue;
+                    while (line < line1 && !(s0 >= ll[line] && s0 <= ll[line + 1])) ++line;
+                    if (line < line1) lines[i] = line;
+                }
+            }
+            if (s_down) __syncthreads();
+            int c0 = 0, end = 0, at = -1;
+            if (t < n) {
+                c0 = list[t].x;
+                end = list[t].y;
+                at = s_down ? lines[t] : line_of(c0, end);
+            }
+            dry.n = 0;
+            place_in(dry, c0, end, at);
+            int made;
+            em.n = written + block_scan(dry.n, wsum, &made);
+            place_in(em, c0, end, at);
+            written += made;
+        }
+        if (t == 0) counts[2 * blockIdx.x] = written > k.out_cap ? -1 : written;
     };
     // (each form's pointers into one address space)
     if (held) place_field(swords + kListWords - w0, swords + kListWords + sc.place_words - w0);
