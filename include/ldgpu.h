@@ -241,8 +241,10 @@ int ldg_get_demod_variant(ldg_ctx* ctx, int32_t* variant);
 
 /* ldg_demod_blocks' schedule (no counterpart in the reference): each CTA
  * demodulates `blocks_per_cta` consecutive blocks (1..64) in one scratch
- * slot; 0 (the default) takes 2 for batches of at least 16 blocks per SM
- * and 1 below.  Outputs do not depend on it. */
+ * slot; 0 (the default) takes 2 for batches of at least 16 blocks per SM, 1
+ * below, and puts a cluster of four or two CTAs on each block of a batch of
+ * which as many clusters are resident at once (33 and 74 blocks on a B200);
+ * a set value takes no clusters.  Outputs do not depend on it. */
 int ldg_set_demod_schedule(ldg_ctx* ctx, int32_t blocks_per_cta);
 
 /* Device scratch the demodulator uses for a batch of `nblocks` blocks
@@ -412,7 +414,7 @@ typedef struct {
     int32_t system;          /* LDG_NTSC / LDG_PAL */
     int32_t video_rot;       /* rf.delays["video_rot"] (> 0) */
     int32_t outlinelen;      /* SysParams outlinelen */
-    int32_t err_cap;         /* error samples kept per field */
+    int32_t err_cap;         /* most error samples of a field (counts -1 above) */
     int32_t out_cap;         /* dropouts kept per field */
     int32_t pad;
     double freq_mhz;         /* rf.freq */
@@ -421,7 +423,7 @@ typedef struct {
     double vsync_ire;        /* SysParams */
 } ldg_dropout_params;
 
-/* Field.dropout_detect for nfields fields in one launch: the per-sample
+/* Field.dropout_detect for nfields fields in four launches: the per-sample
  * error mask (dropout_detect_demod, core.py:2829-2887; the rfhpf standard
  * deviation in FP64 over the field read), the merge of the error samples
  * into spans (build_errlist, 2889-2908) and the spans as TBC line ranges

@@ -500,8 +500,10 @@ __global__ void __launch_bounds__(kMaskThreads) dropout_mask_kernel(const DropFi
 // them and counts their dropouts, which it writes after a scan (walking again
 // when there are more than it keeps).  Noise (a carrier lost for lines on end) is
 // one segment of thousands of spans; there the whole field is walked by windows,
-// which mark the spans' starts for all threads to place.  Bound: a thread's chain of
-// instructions.
+// which mark the spans' starts for all threads to place, and so is a field whose
+// line locations turn back, where a span's line hangs on the span before: one
+// thread finds the lines and all place (one NTSC field, every 40th sample: 4.9 ms, 9.7 when
+// that thread placed them too).  Bound: a thread's chain of instructions.
 __global__ void __launch_bounds__(kPlaceThreads) dropout_place_kernel(const DropField* fields, const DropConsts k,
                                                                       const DropScratch sc, int* drops, int* counts) {
     extern __shared__ unsigned swords[];  // the list of walk_windows, 2 * place_words words

@@ -56,7 +56,7 @@ __global__ void __launch_bounds__(kThreads) lds_unpack_kernel(const uint8_t* __r
         reinterpret_cast<uint4*>(words)[v] = q;
     }
     __syncthreads();
-    const int lead = (int)(bit0 - 8 * at0);  // 0 .. 135
+    const int lead = (int)(bit0 - 8 * at0);  // 0 .. 127
 #pragma unroll
     for (int r = 0; r < kRounds; ++r) {
         const int i = r * kThreads + threadIdx.x;

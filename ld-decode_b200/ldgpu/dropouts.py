@@ -1,6 +1,6 @@
 """Dropout detection on the GPU (ldg_dropouts): Field.dropout_detect
 (lddecode/core.py:2829-2983) for one field or every located field of a
-capture in one launch.
+capture in one call.
 
 Results are the reference's: per field the lists (fieldLine, startx, endx)
 that LDdecode writes as the field's dropOuts (core.py:4535-4542).  A field

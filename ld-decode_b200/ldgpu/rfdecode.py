@@ -178,7 +178,8 @@ class RFDecode(RFParams):
     @property
     def blocks_per_cta(self):
         """Consecutive blocks a demodulator CTA takes (ldg_set_demod_schedule;
-        0: the library's choice, 2 for large batches, else 1)."""
+        0: the library's choice, 2 for large batches, several CTAs per block
+        for small ones, else 1)."""
         return getattr(self, "_blocks_per_cta", 0)
 
     @blocks_per_cta.setter
